@@ -3,7 +3,8 @@
 Every kernel reads keys and values from the pages; the tokens of the step were written there by
 the fused norm/rotary/cache kernel just before.
 
-* float32, or a shape the tensor-core kernels refuse: the CUDA-core kernel in 32-bit arithmetic.
+* float32, heads of 64 or 128 features: a tiled kernel in 32-bit arithmetic; otherwise, or a shape the
+  tensor-core kernels refuse: the CUDA-core kernel with a block a token and query head.
 * bfloat16, every segment a single token: a decode kernel.  Head sizes 64 and 128 with
   power-of-two pages, few pairs and contexts that are not long: a thread-block cluster a
   (token, kv head) pair, which cuts the pair's tiles among its blocks and merges through
@@ -254,6 +255,37 @@ def latent_wide_ok(dtype: torch.dtype, width: int, value_dim: int) -> bool:
     return dtype == torch.bfloat16 and bool(_lib.core()._dll.mrun_latent_attention_wide_ok(_c_int(width), _c_int(value_dim)))
 
 
+F32_TILE_ROWS = 64       # token rows x group heads of a tile of the 32-bit attention
+F32_TILE_GROUP = 16      # query heads a kv head that it takes
+
+
+def f32_tiles_ok(q: torch.Tensor, q_stride: int, head_dim: int, value_dim: int, ratio: int) -> bool:
+    """Whether the tiled 32-bit kernel takes this shape: heads of 64 or 128 features, rows on 16 bytes,
+    groups of up to 16 heads.  The kernel with a block a token and head reads the keys again for every row (B200,
+    32 heads over 8 of 128: prompts of 207 and 310 tokens 1,183 us against 103; four single tokens at contexts of 75
+    to 300, 44 against 30); wider groups stay with it, prompts and single tokens alike, since a block a token
+    and kv head leaves single tokens of theirs too few blocks (40 heads over 2: 78 us against 139)."""
+    return (q.dtype == torch.float32 and head_dim == value_dim and head_dim in (64, 128) and ratio <= F32_TILE_GROUP
+            and q_stride % 4 == 0 and q.data_ptr() % 16 == 0)
+
+
+def _paged_attention_f32(q, q_stride: int, out, cache, group, ctx, heads: int, scale: float, window: int) -> torch.Tensor:
+    def launch(first, count, tiles: int, tile_tokens: int):
+        ops.paged_attention_f32(q, q_stride, out, cache.k, cache.v, group.block_tables, ctx.token_slot, ctx.positions, first, count,
+                                tiles, tile_tokens, heads, scale, window)
+    if ctx.all_decode:
+        launch(None, None, ctx.num_tokens, 1)
+        return out
+    if ctx.num_tokens > ctx.real_tokens:
+        out[ctx.real_tokens:].zero_()
+    tokens = F32_TILE_ROWS // (heads // cache.k.shape[1])
+    for per_tile, longer_than, up_to in ((tokens, 1, 1 << 30), (1, 0, 1)):        # prompt portions; single tokens beside them
+        first, count, n = prefill_tiles(ctx, per_tile, longer_than, up_to)
+        if n:
+            launch(first, count, n, per_tile)
+    return out
+
+
 def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, group, ctx,
                     heads: int, scale: float, window: int, raw=None, value_dim: int = 0,
                     sink: Optional[torch.Tensor] = None, form: Optional[ScoreForm] = None) -> torch.Tensor:
@@ -293,6 +325,8 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
                          _c_long(pages * page_size), _c_float(scale), _c_int(splits), _ptr(part_o), _ptr(part_ml),
                          _stream())
         return out
+    if sink is None and form is None and f32_tiles_ok(q, q_stride, head_dim, v_dim, ratio):
+        return _paged_attention_f32(q, q_stride, out, cache, group, ctx, heads, scale, window)
     if not supports_tensor_cores(q.dtype, head_dim, ratio, v_dim):
         return ops.paged_attention_generic(q, q_stride, out, cache.k, cache.v, group.block_tables,
                                            ctx.token_slot, ctx.positions, heads, scale, window, sink=sink, form=form)

@@ -184,7 +184,7 @@ def build_host() -> str:
 
 
 CORE_SOURCES = ("common.cu", "elementwise.cu", "layernorm.cu", "latent.cu", "routed.cu", "streams.cu", "recurrent.cu", "recurrent_walk.cu", "selective_scan.cu", "attention_diff.cu", "gemm_f32.cu", "gemm_skinny.cu", "gemm_tc5.cu",
-                "attention_generic.cu", "attention_latent.cu", "sampling.cu")
+                "attention_generic.cu", "attention_f32.cu", "attention_latent.cu", "sampling.cu")
 
 
 def build_core() -> str:

@@ -381,6 +381,40 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
     return out
 
 
+def paged_attention_f32(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                        block_tables: torch.Tensor, token_slot: torch.Tensor, positions: torch.Tensor, first: Optional[torch.Tensor],
+                        count: Optional[torch.Tensor], tiles: int, tile_tokens: int, heads: int, scale: float,
+                        window: int = 0) -> torch.Tensor:
+    """32-bit attention over the pages for heads of 64 and 128 features (keys and values alike) in tiles of
+    at most ``tile_tokens`` consecutive tokens of a request: tile i holds ``count[i]`` tokens from row
+    ``first[i]`` on; None: every token a tile.  Rows that no tile names are left as they are."""
+    _check(q, "q", torch.float32, dense=False); _check(out, "out", torch.float32)
+    _check(k_cache, "k_cache", torch.float32); _check(v_cache, "v_cache", torch.float32)
+    _check(block_tables, "block_tables", torch.int32); _check(token_slot, "token_slot", torch.int32)
+    _check(positions, "positions", torch.int32)
+    pages, kv_heads, page_size, head_dim = k_cache.shape
+    tokens = positions.numel()
+    if v_cache.shape != k_cache.shape:
+        raise KernelError(f"paged_attention_f32: key pages {tuple(k_cache.shape)}, value pages {tuple(v_cache.shape)}")
+    if out.shape != (tokens, heads * head_dim) or token_slot.numel() != tokens:
+        raise KernelError(f"paged_attention_f32: out {tuple(out.shape)} / token_slot {token_slot.numel()} "
+                          f"do not match {tokens} tokens of {heads}x{head_dim}")
+    if block_tables.dim() != 2:
+        raise KernelError("paged_attention_f32: block_tables must be [slots, max_blocks]")
+    for name, t in (("first", first), ("count", count)):
+        if t is not None:
+            _check(t, name, torch.int32)
+            if t.numel() != tiles:
+                raise KernelError(f"paged_attention_f32: {name} has {t.numel()} entries for {tiles} tiles")
+    if first is None and tiles != tokens:
+        raise KernelError(f"paged_attention_f32: {tiles} tiles of single tokens for {tokens} tokens")
+    _lib.core().call("mrun_paged_attention_f32", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(k_cache), _ptr(v_cache),
+                     _ptr(block_tables), _c_int(block_tables.shape[1]), _ptr(token_slot), _ptr(positions), _ptr(first), _ptr(count),
+                     _c_int(tiles), _c_int(tile_tokens), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page_size),
+                     _c_long(pages * kv_heads * page_size), _c_float(scale), _c_int(window), _stream())
+    return out
+
+
 GATE_FUNCTIONS = {"silu": 1, "gelu_tanh": 2}      # codes of the C ABI (MRUN_GATE_*); 0 = no gated epilogue
 
 

@@ -1,11 +1,13 @@
-"""The 32-bit products at the edges of their tiles: against 64 bits, and bit for bit the same whichever
-kernel or tile takes a row."""
+"""The 32-bit products and the tiled 32-bit attention at the edges of their tiles: against 64 bits, and bit for bit
+the same whichever kernel or tile takes a row."""
 from __future__ import annotations
 
 import math
 
 import pytest
 import torch
+
+from test_attention_gpu import Case
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -41,3 +43,44 @@ def test_batched_products(m):
     for b in range(6):
         assert torch.equal(out[:, b, :40], ops.gemm_f32_nt(x[:, b].contiguous(), w[b].contiguous()))
     assert (out[:, :, 40:] == 7.0).all()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(8, 8, 64, 32), (32, 8, 128, 16), (32, 2, 64, 16), (16, 1, 128, 4),
+                                                               (16, 1, 64, 16), (6, 2, 128, 1), (8, 2, 128, 24), (9, 3, 64, 8)])
+@pytest.mark.parametrize("window", [0, 37, 64])
+def test_tiled_attention_against_plain(heads, kv_heads, head_dim, page_size, window):
+    segments = [(0, 70), (129, 1), (63, 2), (300, 1), (15, 33), (0, 1), (64, 64)]
+    scale = head_dim ** -0.5
+    case = Case(segments, heads, kv_heads, head_dim, page_size, torch.float32, seed=head_dim + window, window=window)
+    want = case.reference(scale)
+    got = case.run(scale)
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()
+    # the sums' order differs from the kernel with a block a token and head, nothing else does
+    assert (got - case.run(scale, force_generic=True)).abs().max() <= 4e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 4, 64), (8, 2, 128), (16, 1, 128), (32, 2, 64)])
+@pytest.mark.parametrize("window", [0, 50, -48])
+def test_tiled_attention_is_the_same_in_bits_for_every_cutting(heads, kv_heads, head_dim, window):
+    """A request's last tokens alone and in portions of any size, under a window and under chunks."""
+    scale, total = head_dim ** -0.5, 150
+    whole = Case([(0, total)], heads, kv_heads, head_dim, 16, torch.float32, seed=3, window=window)
+    want = whole.run(scale)
+    for start, n in ((149, 1), (64, 1), (128, 22), (63, 3), (100, 17), (1, 70)):
+        part = Case([(start, n)], heads, kv_heads, head_dim, 16, torch.float32, seed=3, window=window)
+        part.kd, part.vd, part.table = whole.kd, whole.vd, whole.table
+        part.group.block_tables, part.group.max_blocks = whole.group.block_tables, whole.group.max_blocks
+        part.ctx.token_slot = whole.ctx.token_slot[start:start + n].contiguous()
+        part.qd = whole.qd[start:start + n].contiguous()
+        assert torch.equal(part.run(scale), want[start:start + n]), (start, n)
+
+
+def test_what_a_row_does_not_see_does_not_enter_its_sums():
+    """Later keys and values of a tile that are infinite or no numbers leave the earlier rows alone."""
+    case = Case([(0, 40)], 4, 2, 64, 16, torch.float32, seed=9)
+    want = case.run(0.125)
+    page, at = case.seg_pages[0][30 // 16], 30 % 16
+    case.kd[page, :, at] = float("nan")
+    case.vd[page, :, at] = float("inf")
+    got = case.run(0.125)
+    assert torch.equal(got[:30], want[:30]) and not torch.isfinite(got[30:]).all()
