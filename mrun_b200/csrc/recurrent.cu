@@ -5,7 +5,8 @@
 // the flat batch, state slot seg_slot[s]); a segment of zero rows is padding.  Every kernel reads
 // the state its request left, walks the segment's tokens in order and leaves the state for the
 // next step, so a token's result does not depend on how the request was cut into steps or on the
-// requests beside it.  States and all arithmetic of the recurrences are 32-bit.
+// requests beside it (recurrent_chunk.cu takes long bfloat16 segments of some scans in chunks instead,
+// whose sums are ordered by the chunks).  States and all arithmetic of the recurrences are 32-bit.
 //
 // Kernels:
 //   causal_conv     y_t = sum_j w[:, j] x_(t - taps + 1 + j) per channel (the last tap meets the

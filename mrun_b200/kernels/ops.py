@@ -1372,6 +1372,43 @@ def _strided_rows(t: torch.Tensor, name: str) -> int:
     return t.stride(0)
 
 
+CHUNK = 64                # tokens a chunk of the chunked scans
+# The longest segment from which on they are worth their three kernels (B200, 16 heads of 128, decay / gated scan, us:
+# 128 tokens 47 / 48 in chunks and 47 / 48 walked, 160 tokens 52 / 48 and 55 / 56, 2,048 tokens 131 / 146 and 526 / 566).
+CHUNK_MIN_TOKENS = 128
+
+
+def _chunks(ctx, tokens: int) -> int:
+    """Chunks of the step's segments where the chunked scans take the step: a segment of at least
+    CHUNK_MIN_TOKENS, and short segments, each a chunk of its own, that pad the chunks by no more than a quarter of
+    the rows and one chunk.  0 otherwise."""
+    if ctx.max_q_len < CHUNK_MIN_TOKENS or len(ctx.segments) != ctx.num_segments:
+        return 0
+    n = ctx.shared.get("scan_chunks")
+    if n is None:
+        n = ctx.shared["scan_chunks"] = sum(-(-seg.q_len // CHUNK) for seg in ctx.segments)
+    return n if 4 * CHUNK * n <= 5 * tokens + 4 * CHUNK else 0
+
+
+def _chunked_scan(q, k, v, ld: int, decay, silu_inputs: bool, a, bias, tau: float, state, ctx, out, heads: int, dim: int,
+                  vdim: int) -> bool:
+    """Runs a decay or gated scan chunk by chunk where that form takes it."""
+    chunks = _chunks(ctx, q.shape[0])
+    if not chunks:
+        return False
+    size = _lib.core().function("mrun_chunked_scan_floats")
+    size.restype = _c_long
+    floats = size(_ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(dtype_code(q.dtype)), _ptr(a), _ptr(bias), _ptr(state), _ptr(out),
+                  _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim))
+    if not floats:
+        return False
+    scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
+    _lib.core().call("mrun_chunked_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _ptr(decay), _c_int(1 if silu_inputs else 0),
+                     _ptr(a), _ptr(bias), _c_float(tau), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start),
+                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    return True
+
+
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, state: torch.Tensor, ctx,
                heads: int, dim: int, vdim: int, silu_inputs: bool) -> torch.Tensor:
     """Per head S_t = decay_h S_(t-1) + k_t v_t^T, o_t = S_t^T q_t over each request's tokens, from
@@ -1386,6 +1423,8 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
             or state.shape[1:] != (heads, dim, vdim) or decay.numel() != heads:
         raise KernelError("decay_scan: sizes do not match")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    if _chunked_scan(q, k, v, ld, decay, silu_inputs, None, None, 1.0, state, ctx, out, heads, dim, vdim):
+        return out
     scratch = torch.empty(tokens * (2 * heads * dim + heads * vdim), dtype=torch.float32, device=q.device)
     _lib.core().call("mrun_decay_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype), _ptr(decay),
                      _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
@@ -1437,6 +1476,8 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
             or a.shape != (tokens, heads * dim) or bias.numel() != heads * dim or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("gated_scan: sizes do not match")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    if _chunked_scan(q, k, v, ld, None, False, a, bias, tau, state, ctx, out, heads, dim, vdim):
+        return out
     scratch = torch.empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32, device=q.device)
     _lib.core().call("mrun_gated_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype), _ptr(a), _ptr(bias),
                      _c_float(tau), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),

@@ -43,7 +43,7 @@ class DecayAttention:
 
     def activation_elements(self) -> int:
         s = self.spec
-        return 2 * s.heads * s.dim + 5 * s.heads * s.vdim
+        return s.heads * (7 * s.dim + 7 * s.vdim)        # the scan's scratch among them
 
     def cache_need(self):
         s = self.spec

@@ -1,0 +1,133 @@
+"""The chunked scans against the recurrence token by token in 64 bits, at the edges of chunks and runs, and against
+the walk they take over from."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def context(lengths, slots):
+    at = [0]
+    for n in lengths:
+        at.append(at[-1] + n)
+    order = [(5 * i + 2) % slots for i in range(len(lengths))]
+    assert len(set(order)) == len(order)
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    return SimpleNamespace(segments=[SimpleNamespace(q_len=n) for n in lengths], num_segments=len(lengths), max_q_len=max(lengths),
+                           shared={}, seg_q_start=dev(at), seg_slot=dev(order))
+
+
+def exact(q, k, v, g, ctx, state, beta=None):
+    """q, k, g: float64 [tokens, heads, dim], v: [tokens, heads, vdim]; (outputs, states)."""
+    new, out, at = state.double().clone(), torch.empty_like(v), ctx.seg_q_start.tolist()
+    for s, slot in enumerate(ctx.seg_slot.tolist()):
+        for t in range(at[s], at[s + 1]):
+            new[slot] *= g[t][:, :, None]
+            u = v[t]
+            if beta is not None:
+                u = beta[t][:, None] * (u - (new[slot] * k[t][:, :, None]).sum(1))
+            new[slot] += k[t][:, :, None] * u[:, None, :]
+            out[t] = (new[slot] * q[t][:, :, None]).sum(1)
+    return out.flatten(1), new
+
+
+LENGTHS = [[64], [63, 1, 65], [128], [129, 16, 17, 15], [1, 200, 33], [300]]
+
+
+def check(run, want, monkeypatch, chunks_taken):
+    """``run()`` -> (outputs, states) by the chunks and by the walk; both within 32-bit sums of ``want``: up to 192
+    terms a sum and a decay of a few roundings a token, 2^-24 each."""
+    from mrun_b200.kernels import ops
+    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens: sum(-(-seg.q_len // ops.CHUNK) for seg in ctx.segments))
+    taken = []
+    inner = ops._chunked_scan
+    monkeypatch.setattr(ops, "_chunked_scan", lambda *a, **k: taken.append(inner(*a, **k)) or taken[-1])
+    results = [run()]
+    assert taken == [chunks_taken]
+    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens: 0)
+    results.append(run())
+    for got in results:
+        for x, y in zip(got, want):
+            assert float((x.double() - y).abs().max() / y.abs().max()) <= 2e-5
+            assert float((x.double() - y).norm() / y.norm()) <= 5e-6
+
+
+@pytest.mark.parametrize("heads, dim, vdim", [(3, 128, 128), (2, 64, 64), (1, 64, 128), (2, 128, 64)])
+@pytest.mark.parametrize("lengths", LENGTHS, ids=str)
+@pytest.mark.parametrize("silu", [False, True])
+def test_decay_scan_in_chunks(heads, dim, vdim, lengths, silu, monkeypatch):
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(sum(lengths) + dim)
+    ctx, tokens = context(lengths, 7), sum(lengths)
+    y = torch.randn(tokens, heads * (2 * dim + vdim) + 4, generator=gen, device=DEV).bfloat16()
+    q, k, v = y[:, :heads * dim], y[:, heads * dim:2 * heads * dim], y[:, 2 * heads * dim:2 * heads * dim + heads * vdim]
+    decay = torch.tensor([0.999, 0.05, 0.8][:heads], device=DEV)
+    start = torch.randn(7, heads, dim, vdim, generator=gen, device=DEV)
+    fn = torch.nn.functional.silu if silu else (lambda t: t)
+    wide = [fn(t.double()).unflatten(1, (heads, -1)) for t in (q, k, v)]
+    want = exact(*wide, decay.double()[None, :, None].expand(tokens, heads, dim), ctx, start)
+
+    def run():
+        state = start.clone()
+        return ops.decay_scan(q, k, v, decay, state, ctx, heads, dim, vdim, silu), state
+    check(run, want, monkeypatch, True)
+
+
+@pytest.mark.parametrize("heads, dim, vdim", [(3, 128, 128), (2, 64, 64), (1, 64, 128), (2, 128, 64)])
+@pytest.mark.parametrize("lengths", LENGTHS, ids=str)
+@pytest.mark.parametrize("centre, spread", [(2.0, 1.5), (9.0, 1.0), (-300.0, 100.0), (0.0, 60.0)])
+def test_gated_scan_in_chunks(heads, dim, vdim, lengths, centre, spread, monkeypatch):
+    """Decays near one, decays that forget a token within a step (their products underflow), and both side by side."""
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(sum(lengths) + dim)
+    ctx, tokens = context(lengths, 7), sum(lengths)
+    y = torch.randn(tokens, heads * (2 * dim + vdim) + 4, generator=gen, device=DEV).bfloat16()
+    q, k, v = y[:, :heads * dim], y[:, heads * dim:2 * heads * dim], y[:, 2 * heads * dim:2 * heads * dim + heads * vdim]
+    a = torch.randn(tokens, heads * dim, generator=gen, device=DEV)
+    bias = centre + spread * torch.randn(heads * dim, generator=gen, device=DEV)
+    start = torch.randn(7, heads, dim, vdim, generator=gen, device=DEV)
+    split = lambda t: t.double().unflatten(1, (heads, -1))
+    g = torch.exp(torch.nn.functional.logsigmoid((a + bias).double()) / 8.0).unflatten(1, (heads, dim))
+    want = exact(split(q) * dim ** -0.5, split(k), split(v), g, ctx, start)
+
+    def run():
+        state = start.clone()
+        return ops.gated_scan(q, k, v, a, bias, 8.0, state, ctx, heads, dim, vdim), state
+    check(run, want, monkeypatch, True)
+
+
+def test_which_steps_are_scanned_in_chunks():
+    """Long segments, and short ones beside them as long as they pad little; never a captured step."""
+    from mrun_b200.kernels import ops
+
+    def chunks(lengths):
+        return ops._chunks(SimpleNamespace(segments=[SimpleNamespace(q_len=n) for n in lengths], shared={}, num_segments=len(lengths),
+                                           max_q_len=max(lengths)), sum(lengths))
+    assert chunks([ops.CHUNK_MIN_TOKENS - 1]) == 0
+    assert chunks([ops.CHUNK_MIN_TOKENS]) == -(-ops.CHUNK_MIN_TOKENS // ops.CHUNK)
+    assert chunks([640, 640, 1, 1]) == 22
+    assert chunks([256] + [1] * 20) == 0
+    assert ops._chunks(SimpleNamespace(segments=[], shared={}, num_segments=4, max_q_len=500), 4) == 0
+
+
+def test_rows_without_a_chunked_form_are_walked(monkeypatch):
+    """32-bit rows, other sizes and rows off their 8 bytes go to the walk as before."""
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    ctx = context([150], 7)
+    for dtype, dim, off in ((torch.float32, 64, 0), (torch.bfloat16, 48, 0), (torch.bfloat16, 64, 1)):
+        y = torch.randn(150, 3 * dim + 4, generator=gen, device=DEV).to(dtype)
+        q, k, v = (y[:, off + i * dim:off + (i + 1) * dim] for i in range(3))
+        decay, start = torch.tensor([0.9], device=DEV), torch.zeros(7, 1, dim, dim, device=DEV)
+        want = exact(*(t.double()[:, None] for t in (q, k, v)), torch.full((150, 1, dim), 0.9, device=DEV).double(), ctx, start)
+
+        def run():
+            state = start.clone()
+            return ops.decay_scan(q, k, v, decay, state, ctx, 1, dim, dim, False), state
+        with monkeypatch.context() as m:
+            check(run, want, m, False)
