@@ -1,7 +1,8 @@
 // Paged grouped-query attention for prompt portions on the fifth-generation tensor cores
 // (tcgen05, accumulators in tensor memory), compiled for one head size that is a multiple of 64
 // and at most 128: -DMRUN_HEAD_DIM=<64 | 128> (values of another of these sizes: -DMRUN_VALUE_DIM;
-// worked-on scores and gated outputs, attention_score.cuh: -DMRUN_SCORED=1).
+// worked-on scores and gated outputs, attention_score.cuh: -DMRUN_SCORED=1).  Keys may have 192 features
+// where the values have 64 or 128 and the scores are plain: Q and two stages of K and V then take 209 KB.
 //
 // One thread block per (tile of query tokens, kv head).  The tile's 128 rows are (token, query
 // head of the kv head's group) pairs, so a key/value tile read once serves the whole group.  Keys
@@ -57,7 +58,7 @@
 #define MRUN_SCORED 0
 #endif
 
-#if MRUN_HEAD_DIM % 64 == 0 && MRUN_HEAD_DIM <= 128 && MRUN_VALUE_DIM % 64 == 0 && MRUN_VALUE_DIM <= 128
+#if MRUN_HEAD_DIM % 64 == 0 && MRUN_HEAD_DIM <= (MRUN_SCORED ? 128 : 192) && MRUN_VALUE_DIM % 64 == 0 && MRUN_VALUE_DIM <= 128
 #define MRUN_ATTN_TC5 1
 #else
 #define MRUN_ATTN_TC5 0
@@ -487,7 +488,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 
 #endif  // MRUN_ATTN_TC5
 
-// 1 when this library holds the tcgen05 prefill kernel (head sizes 64 and 128).
+// 1 when this library holds the tcgen05 prefill kernel (head sizes 64 and 128, and keys of 192).
 MRUN_API int mrun_attn_prefill_tc5_available() { return MRUN_ATTN_TC5; }
 
 // Rows per tile of the tcgen05 kernel: a tile holds at most 128 / (heads / kv_heads) tokens.
@@ -545,6 +546,6 @@ MRUN_API int mrun_attn_prefill_tc5(const void* q, long q_stride, void* out, cons
     }
     return 0;
 #else
-    return mrun_set_error("attn_prefill_tc5: not built for head_dim=%d (head sizes 64 and 128 only)", MRUN_HEAD_DIM);
+    return mrun_set_error("attn_prefill_tc5: not built for head_dim=%d (head sizes 64 and 128, keys of 192 with smaller values)", MRUN_HEAD_DIM);
 #endif
 }

@@ -5,6 +5,7 @@
 //   latent_prepare    the down-projections' rows -> normed query latent, and the token's cache row
 //                     [normed key/value latent | rotated shared key part | zeros]
 //   latent_query      the rotated part of every query head into the attention's query rows
+//   latent_rotate     the same in place, for queries that meet keys made from the latents
 //   post_norm_add     stream += scale * rmsnorm(branch) * w_post, then rmsnorm(stream) * w_next
 //   route_top_k       router logits -> a dense row of expert weights (zero where not chosen)
 //   relu2_scaled      relu(u)^2 times the expert weight of the column's expert
@@ -71,6 +72,27 @@ latent_prepare_kernel(const TA* __restrict__ down, long ld, const float* __restr
     }
     for (int i = rot_dims + tid; i < rot_dim; i += blockDim.x) dst[kv_rank + i] = kr[i];
     for (int i = kv_rank + rot_dim + tid; i < width; i += blockDim.x) dst[i] = from_float<TA>(0.f);
+}
+
+// ------------------------------------------------------------------------------------------
+// Rotates the first rot_dims features of every head's rotated part in place: q[t, h] = [plain part (dim) | rotated
+// part (rot_dim)].  A thread owns a pair of features, so nothing is read after it was written.
+// ------------------------------------------------------------------------------------------
+template <typename TA>
+__global__ void __launch_bounds__(256)
+latent_rotate_kernel(TA* __restrict__ q, long ldq, const float2* __restrict__ rot, int rot_dims, int interleaved, int heads, int dim,
+                     int rot_dim) {
+    const int t = blockIdx.x, pairs = rot_dims / 2;
+    for (int item = threadIdx.x; item < heads * pairs; item += blockDim.x) {
+        const int h = item / pairs, i = item - h * pairs;
+        TA* part = q + (size_t)t * ldq + (size_t)h * (dim + rot_dim) + dim;
+        TA* first = part + (interleaved ? 2 * i : i);
+        TA* second = interleaved ? first + 1 : first + pairs;
+        const float2 cs = rot[(size_t)t * pairs + i];
+        const float x = to_float(*first), y = to_float(*second);
+        *first = from_float<TA>(x * cs.x - y * cs.y);
+        *second = from_float<TA>(y * cs.x + x * cs.y);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -369,6 +391,24 @@ MRUN_API int mrun_latent_prepare(const void* down, int act_dtype, long ld, const
     return 0;
 }
 
+// q: row t at q + t * ldq, [heads, dim + rot_dim]; rot: float32 [tokens, rot_dims / 2, 2].
+MRUN_API int mrun_latent_rotate(void* q, long ldq, int act_dtype, const float* rot, int rot_dims, int interleaved, int tokens, int heads,
+                                int dim, int rot_dim, cudaStream_t stream) {
+    MRUN_REQUIRE(tokens >= 0 && heads > 0 && dim >= 0 && rot_dims > 0 && rot_dims % 2 == 0 && rot_dims <= rot_dim && rot != nullptr &&
+                     ldq >= (long)heads * (dim + rot_dim),
+                 "latent_rotate: bad sizes heads=%d dim=%d rot_dim=%d rot_dims=%d ldq=%ld", heads, dim, rot_dim, rot_dims, ldq);
+    if (tokens == 0) return 0;
+    if (act_dtype == MRUN_F32)
+        latent_rotate_kernel<float><<<tokens, 256, 0, stream>>>((float*)q, ldq, (const float2*)rot, rot_dims, interleaved, heads, dim, rot_dim);
+    else if (act_dtype == MRUN_BF16)
+        latent_rotate_kernel<__nv_bfloat16><<<tokens, 256, 0, stream>>>((__nv_bfloat16*)q, ldq, (const float2*)rot, rot_dims, interleaved,
+                                                                        heads, dim, rot_dim);
+    else
+        return mrun_set_error("latent_rotate: unknown dtype code %d", act_dtype);
+    MRUN_CHECK_LAUNCH("latent_rotate");
+    return 0;
+}
+
 MRUN_API int mrun_latent_query(const void* q, long ldq, int act_dtype, const float* rot, int rot_dims, int interleaved,
                                void* q_att, int tokens, int heads, int dim, int rot_dim, int kv_rank, int width,
                                cudaStream_t stream) {
@@ -398,13 +438,15 @@ MRUN_API int mrun_latent_query(const void* q, long ldq, int act_dtype, const flo
 // The latents of whole contexts, laid side by side: out[segment, j, :kv_rank] = the cached latent of the
 // segment's token j for j < seg_kv_len[segment], and zeros from there up to the next multiple of 128
 // rows (attention tiles read whole; keys that do not exist must not be patterns that are no numbers).
+// The rotated key part behind the latent, which the heads share, goes to every head's key likewise:
+// keys[segment, h, j, dim:] (rows of dim + rot_dim features; rot_dim = 0: there is none).
 // grid: rows x segments.
 // ------------------------------------------------------------------------------------------
 template <typename TA>
 __global__ void __launch_bounds__(64)
 latent_rows_kernel(const TA* __restrict__ cache, const int* __restrict__ block_tables, int max_blocks,
                    const int* __restrict__ seg_slot, const int* __restrict__ seg_kv_len, TA* __restrict__ out, int rows,
-                   int page_size, int kv_rank, int width, int wide) {
+                   int page_size, int kv_rank, int width, int wide, TA* __restrict__ keys, int heads, int dim, int rot_dim) {
     const int j = blockIdx.x, seg = blockIdx.y, len = seg_kv_len[seg];
     if (j >= ((len + 127) & ~127)) return;
     TA* dst = out + ((size_t)seg * rows + j) * kv_rank;
@@ -414,28 +456,43 @@ latent_rows_kernel(const TA* __restrict__ cache, const int* __restrict__ block_t
         constexpr int N = 16 / sizeof(TA);
         for (int c = threadIdx.x; c < kv_rank / N; c += 64)
             reinterpret_cast<uint4*>(dst)[c] = page < 0 ? make_uint4(0, 0, 0, 0) : reinterpret_cast<const uint4*>(src)[c];
+        const int pieces = rot_dim / N;
+        for (int e = threadIdx.x; e < heads * pieces; e += 64) {
+            const int h = e / pieces, c = e % pieces;
+            reinterpret_cast<uint4*>(keys + (((size_t)seg * heads + h) * rows + j) * (dim + rot_dim) + dim)[c] =
+                page < 0 ? make_uint4(0, 0, 0, 0) : reinterpret_cast<const uint4*>(src + kv_rank)[c];
+        }
     } else {
         for (int c = threadIdx.x; c < kv_rank; c += 64) dst[c] = page < 0 ? from_float<TA>(0.f) : src[c];
+        for (int e = threadIdx.x; e < heads * rot_dim; e += 64) {
+            const int h = e / rot_dim, c = e % rot_dim;
+            keys[(((size_t)seg * heads + h) * rows + j) * (dim + rot_dim) + dim + c] = page < 0 ? from_float<TA>(0.f) : src[kv_rank + c];
+        }
     }
 }
 
-// out: [segments, rows, kv_rank]; rows: at least every segment's length rounded up to a multiple of 128.
+// out: [segments, rows, kv_rank]; rows: at least every segment's length rounded up to a multiple of 128.  keys:
+// null with rot_dim = 0, else [segments, heads, rows, dim + rot_dim], of which the last rot_dim features are filled.
 MRUN_API int mrun_latent_rows(const void* cache, int act_dtype, const int* block_tables, int max_blocks, const int* seg_slot,
                               const int* seg_kv_len, void* out, int segments, int rows, int page_size, int kv_rank, int width,
-                              cudaStream_t stream) {
+                              void* keys, int heads, int dim, int rot_dim, cudaStream_t stream) {
     MRUN_REQUIRE(segments >= 0 && segments <= 65535 && rows > 0 && rows % 128 == 0 && page_size > 0 && max_blocks > 0 && kv_rank > 0 &&
-                 width >= kv_rank, "latent_rows: bad sizes segments=%d rows=%d kv_rank=%d width=%d", segments, rows, kv_rank, width);
+                 rot_dim >= 0 && width >= kv_rank + rot_dim,
+                 "latent_rows: bad sizes segments=%d rows=%d kv_rank=%d rot_dim=%d width=%d", segments, rows, kv_rank, rot_dim, width);
+    MRUN_REQUIRE(rot_dim == 0 || (keys != nullptr && heads > 0 && dim >= 0), "latent_rows: no keys for the rotated part");
     if (segments == 0) return 0;
     const size_t unit = act_dtype == MRUN_F32 ? 4 : 2;
-    const int wide = kv_rank * unit % 16 == 0 && width * unit % 16 == 0 && (((uintptr_t)cache | (uintptr_t)out) & 15) == 0;
+    const int wide = kv_rank * unit % 16 == 0 && width * unit % 16 == 0 && dim * unit % 16 == 0 && rot_dim * unit % 16 == 0 &&
+                     (((uintptr_t)cache | (uintptr_t)out | (uintptr_t)keys) & 15) == 0;
     const dim3 grid(rows, segments);
     if (act_dtype == MRUN_F32)
         latent_rows_kernel<float><<<grid, 64, 0, stream>>>((const float*)cache, block_tables, max_blocks, seg_slot, seg_kv_len,
-                                                           (float*)out, rows, page_size, kv_rank, width, wide);
+                                                           (float*)out, rows, page_size, kv_rank, width, wide, (float*)keys, heads, dim,
+                                                           rot_dim);
     else if (act_dtype == MRUN_BF16)
         latent_rows_kernel<__nv_bfloat16><<<grid, 64, 0, stream>>>((const __nv_bfloat16*)cache, block_tables, max_blocks, seg_slot,
                                                                    seg_kv_len, (__nv_bfloat16*)out, rows, page_size, kv_rank, width,
-                                                                   wide);
+                                                                   wide, (__nv_bfloat16*)keys, heads, dim, rot_dim);
     else
         return mrun_set_error("latent_rows: unknown dtype code %d", act_dtype);
     MRUN_CHECK_LAUNCH("latent_rows");

@@ -1051,20 +1051,40 @@ def latent_prepare(down: torch.Tensor, q_weight: Optional[torch.Tensor], kv_weig
 
 
 def latent_rows(cache: torch.Tensor, block_tables: torch.Tensor, seg_slot: torch.Tensor, seg_kv_len: torch.Tensor, rows: int,
-                kv_rank: int) -> torch.Tensor:
+                kv_rank: int, keys: Optional[torch.Tensor] = None, rot_dim: int = 0) -> torch.Tensor:
     """[segments, rows, kv_rank]: the cached latents (the first ``kv_rank`` features of ``cache``'s rows, [pages,
     1, page_size, width]) of every segment's whole context, zeros from its length up to the next
-    multiple of 128 and nothing beyond.  ``rows``: a multiple of 128 that holds every context."""
+    multiple of 128 and nothing beyond.  ``rows``: a multiple of 128 that holds every context.  With ``rot_dim``
+    the features behind the latent go to the last ``rot_dim`` features of every head's row of ``keys`` (dense
+    [segments, heads, rows, dim + rot_dim]) likewise."""
     _check(cache, "cache"); _check(block_tables, "block_tables", torch.int32)
     _check(seg_slot, "seg_slot", torch.int32); _check(seg_kv_len, "seg_kv_len", torch.int32)
     segments = seg_slot.numel()
-    if cache.dim() != 4 or cache.shape[1] != 1 or seg_kv_len.numel() != segments or cache.shape[3] < kv_rank:
+    if cache.dim() != 4 or cache.shape[1] != 1 or seg_kv_len.numel() != segments or cache.shape[3] < kv_rank + rot_dim:
         raise KernelError(f"latent_rows: cache {tuple(cache.shape)}, {segments} segments, {seg_kv_len.numel()} lengths")
+    heads = dim = 0
+    if rot_dim:
+        _check(keys, "keys", cache.dtype)
+        if keys.dim() != 4 or keys.shape[0] != segments or keys.shape[2] != rows or keys.shape[3] < rot_dim:
+            raise KernelError(f"latent_rows: keys {tuple(keys.shape)} for {segments} segments of {rows} rows")
+        heads, dim = keys.shape[1], keys.shape[3] - rot_dim
     out = torch.empty((segments, rows, kv_rank), dtype=cache.dtype, device=cache.device)
     _lib.core().call("mrun_latent_rows", _ptr(cache), dtype_code(cache.dtype), _ptr(block_tables), _c_int(block_tables.shape[1]),
                      _ptr(seg_slot), _ptr(seg_kv_len), _ptr(out), _c_int(segments), _c_int(rows), _c_int(cache.shape[2]),
-                     _c_int(kv_rank), _c_int(cache.shape[3]), _stream())
+                     _c_int(kv_rank), _c_int(cache.shape[3]), _ptr(keys if rot_dim else None), _c_int(heads), _c_int(dim),
+                     _c_int(rot_dim), _stream())
     return out
+
+
+def latent_rotate(q: torch.Tensor, rot: torch.Tensor, rot_dims: int, pairing: str, heads: int, dim: int, rot_dim: int) -> None:
+    """In place on ``q`` [tokens, heads * (dim + rot_dim)] (rows may be strided): rotates the first ``rot_dims`` features
+    behind every head's ``dim`` plain ones."""
+    ldq = _strided_rows(q, "q"); _check(rot, "rot", torch.float32)
+    tokens = q.shape[0]
+    if q.shape[1] != heads * (dim + rot_dim) or rot.shape != (tokens, rot_dims // 2, 2):
+        raise KernelError(f"latent_rotate: q {tuple(q.shape)}, rot {tuple(rot.shape)}")
+    _lib.core().call("mrun_latent_rotate", _ptr(q), _c_long(ldq), dtype_code(q.dtype), _ptr(rot), _c_int(rot_dims),
+                     _c_int(PAIRINGS[pairing]), _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(rot_dim), _stream())
 
 
 def latent_query(q: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: int, pairing: str, q_att: torch.Tensor,

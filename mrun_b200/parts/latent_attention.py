@@ -22,10 +22,13 @@ per head, whose sigmoid multiplies the heads behind W_h.  A layer without positi
 caches the latent alone.  ``window`` reaches the
 attention kernels as it does for grouped-query attention.
 
-**Steps with prompt portions** of a layer without positions and without a window, where the heads' plain keys
-and values are 64 or 128 features, make the keys and values after all (``_expanded``): the scores of a
-portion against its own context cost (dim + vdim) a key and head that way against 2 kv_rank, and the tcgen05
-kernel takes the shape.  The contexts' latents are gathered out of the pages, each segment's keys and
+**Steps with prompt portions** of a layer without a window whose heads' keys (plain and rotated part together:
+64, 128 or 192 features) and values (64 or 128) the tcgen05 kernel takes make the keys and values after all
+(``_expanded``): the scores of a portion against its own context cost (dim + rot_dim + vdim) a key and head that
+way against 2 kv_rank + rot_dim, and rows wider than 128 features have no tcgen05 kernel (B200, two portions
+of 760 and 1,140 tokens behind 700 and 350, 16 heads of 128 + 64, a latent of 512: the kernel for wide rows takes
+688 of the mixer's 788 us; with keys and values made the mixer takes 222).  The contexts' latents are gathered
+out of the pages, the rotated part they share goes beside every head's plain key, each segment's keys and
 values become one large page of scratch, and the paged kernels run over those.  Only while the contexts
 together are not much longer than the step (``EXPAND_ROWS`` times its rows), so that a long context is not
 projected up again for every portion of it; other steps, decode steps and the 32-bit path stay with the
@@ -116,8 +119,12 @@ class LatentAttention:
         self.graph_safe = not (supports_tensor_cores(runtime.precision.act, self.width, s.heads) and s.heads > 16
                                and (s.window is not None or not latent_wide_ok(runtime.precision.act, self.width, s.kv_rank)))
 
-        self.expandable = (runtime.precision.act == torch.bfloat16 and s.rot_dim == 0 and not s.q_rank and s.window is None
-                           and s.dim in (64, 128) and s.vdim in (64, 128))
+        # Whether prompt steps may make the heads' keys and values from the latents (``_expanded``): key and value sizes
+        # that the tcgen05 kernel takes, and, with a rotated part or a query latent, cache rows that it does not
+        # take itself (on rows of 64 and 128 features it runs over the latents at the same cost).
+        self.expandable = (runtime.precision.act == torch.bfloat16 and s.window is None and s.vdim in (64, 128)
+                           and s.dim + s.rot_dim in (64, 128, 192) and s.dim % 8 == 0 and s.rot_dim % 8 == 0
+                           and (self.width > 128 or (s.rot_dim == 0 and not s.q_rank and s.dim in (64, 128))))
 
     def _scratch_rows(self, ctx) -> int:
         """Rows of the scratch pages of a step whose keys and values are made, 0 for a step that keeps the latent."""
@@ -129,15 +136,18 @@ class LatentAttention:
         return rows if rows * len(ctx.segments) <= EXPAND_ROWS * max(128, ctx.num_tokens) else 0
 
     def _expanded(self, q, ctx, cache, group, rows: int) -> torch.Tensor:
-        """The heads' outputs over keys and values made from the contexts' latents: [tokens, heads * vdim]."""
+        """The heads' outputs over keys and values made from the contexts' latents: [tokens, heads * vdim].  ``q``
+        is rotated in place."""
         s, n = self.spec, len(ctx.segments)
-        latents = ops.latent_rows(cache.k, group.block_tables, ctx.seg_slot[:n], ctx.seg_kv_len[:n], rows, s.kv_rank)
-        k = torch.empty((n, s.heads, rows, s.dim), dtype=q.dtype, device=q.device)
+        k = torch.empty((n, s.heads, rows, s.dim + s.rot_dim), dtype=q.dtype, device=q.device)
+        latents = ops.latent_rows(cache.k, group.block_tables, ctx.seg_slot[:n], ctx.seg_kv_len[:n], rows, s.kv_rank, k, s.rot_dim)
+        if self.rot_dims:
+            ops.latent_rotate(q, self.position.rotation(ctx), self.rot_dims, self.pairing, s.heads, s.dim, s.rot_dim)
         v = torch.empty((n, s.heads, rows, s.vdim), dtype=q.dtype, device=q.device)
         for i, seg in enumerate(ctx.segments):
             used = -(-(seg.pos_start + seg.q_len) // 128) * 128
             c = latents[i, :used].expand(s.heads, used, s.kv_rank)
-            torch.bmm(c, self.w_uk_t, out=k[i, :, :used])
+            torch.bmm(c, self.w_uk_t, out=k[i, :, :used, :s.dim])
             torch.bmm(c, self.w_uv.transpose(1, 2), out=v[i, :, :used])
         table = ctx.shared.get("segment_pages")
         if table is None:           # state slot -> its segment's page
@@ -154,7 +164,7 @@ class LatentAttention:
     def activation_elements(self) -> int:
         s = self.spec
         latent = s.q_rank + s.kv_rank + s.rot_dim + s.heads * (s.dim + s.rot_dim + 2 * self.width + s.vdim)
-        return latent + (EXPAND_ROWS * (s.kv_rank + s.heads * (s.dim + s.vdim)) if self.expandable else 0)
+        return latent + (EXPAND_ROWS * (s.kv_rank + s.heads * (s.dim + s.rot_dim + s.vdim)) if self.expandable else 0)
 
     def forward(self, x, ctx, cache, defer_output: bool = False):
         s, width = self.spec, self.width
