@@ -1396,13 +1396,15 @@ CHUNK = 64                # tokens a chunk of the chunked scans
 # The longest segment from which on they are worth their three kernels (B200, 16 heads of 128, decay / gated scan, us:
 # 128 tokens 47 / 48 in chunks and 47 / 48 walked, 160 tokens 52 / 48 and 55 / 56, 2,048 tokens 131 / 146 and 526 / 566).
 CHUNK_MIN_TOKENS = 128
+# The same for the delta scan (200 tokens 70 in chunks, 74 walked; 128 tokens 62 and 54; 2,048 tokens 266 and 647).
+DELTA_CHUNK_MIN_TOKENS = 192
 
 
-def _chunks(ctx, tokens: int) -> int:
+def _chunks(ctx, tokens: int, least: int) -> int:
     """Chunks of the step's segments where the chunked scans take the step: a segment of at least
-    CHUNK_MIN_TOKENS, and short segments, each a chunk of its own, that pad the chunks by no more than a quarter of
+    ``least`` tokens, and short segments, each a chunk of its own, that pad the chunks by no more than a quarter of
     the rows and one chunk.  0 otherwise."""
-    if ctx.max_q_len < CHUNK_MIN_TOKENS or len(ctx.segments) != ctx.num_segments:
+    if ctx.max_q_len < least or len(ctx.segments) != ctx.num_segments:
         return 0
     n = ctx.shared.get("scan_chunks")
     if n is None:
@@ -1410,22 +1412,39 @@ def _chunks(ctx, tokens: int) -> int:
     return n if 4 * CHUNK * n <= 5 * tokens + 4 * CHUNK else 0
 
 
+def _chunk_scratch(ctx, delta: bool, q, k, v, ld: int, a, bias, state, out, heads: int, dim: int, vdim: int):
+    """(scratch, chunks) of a scan that runs chunk by chunk, or None where it is walked."""
+    chunks = _chunks(ctx, q.shape[0], DELTA_CHUNK_MIN_TOKENS if delta else CHUNK_MIN_TOKENS)
+    if not chunks:
+        return None
+    size = _lib.core().function("mrun_chunked_scan_floats")
+    size.restype = _c_long
+    floats = size(_c_int(1 if delta else 0), _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(dtype_code(q.dtype)), _ptr(a), _ptr(bias),
+                  _ptr(state), _ptr(out), _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim))
+    return (torch.empty(floats, dtype=torch.float32, device=q.device), chunks) if floats else None
+
+
 def _chunked_scan(q, k, v, ld: int, decay, silu_inputs: bool, a, bias, tau: float, state, ctx, out, heads: int, dim: int,
                   vdim: int) -> bool:
     """Runs a decay or gated scan chunk by chunk where that form takes it."""
-    chunks = _chunks(ctx, q.shape[0])
-    if not chunks:
+    found = _chunk_scratch(ctx, False, q, k, v, ld, a, bias, state, out, heads, dim, vdim)
+    if found is None:
         return False
-    size = _lib.core().function("mrun_chunked_scan_floats")
-    size.restype = _c_long
-    floats = size(_ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(dtype_code(q.dtype)), _ptr(a), _ptr(bias), _ptr(state), _ptr(out),
-                  _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim))
-    if not floats:
-        return False
-    scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
     _lib.core().call("mrun_chunked_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _ptr(decay), _c_int(1 if silu_inputs else 0),
-                     _ptr(a), _ptr(bias), _c_float(tau), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start),
-                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+                     _ptr(a), _ptr(bias), _c_float(tau), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
+                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(found[1]), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    return True
+
+
+def _chunked_delta_scan(q, k, v, ld: int, a, b, ldb: int, a_log, dt_bias, state, ctx, out, heads: int, kv_heads: int, dim: int,
+                        vdim: int) -> bool:
+    """Runs a delta scan chunk by chunk where that form takes it."""
+    found = _chunk_scratch(ctx, True, q, k, v, ld, a, dt_bias, state, out, heads, dim, vdim)
+    if found is None:
+        return False
+    _lib.core().call("mrun_chunked_delta_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(heads // kv_heads), _ptr(a), _ptr(b),
+                     _c_long(ldb), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
+                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(found[1]), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
     return True
 
 
@@ -1472,6 +1491,8 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
             or a_log.numel() != heads or dt_bias.numel() != heads * dim or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("delta_scan: sizes do not match")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    if _chunked_delta_scan(q, k, v, ld, a, b, ldb, a_log, dt_bias, state, ctx, out, heads, kv_heads, dim, vdim):
+        return out
     scratch = torch.empty(tokens * (2 * kv_heads * dim + heads * (vdim + dim + 1)), dtype=torch.float32, device=q.device)
     _lib.core().call("mrun_delta_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype),
                      _c_int(heads // kv_heads), _ptr(a), _ptr(b), _c_long(ldb), _ptr(a_log), _ptr(dt_bias), _ptr(state),

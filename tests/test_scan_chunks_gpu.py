@@ -43,13 +43,13 @@ def check(run, want, monkeypatch, chunks_taken):
     """``run()`` -> (outputs, states) by the chunks and by the walk; both within 32-bit sums of ``want``: up to 192
     terms a sum and a decay of a few roundings a token, 2^-24 each."""
     from mrun_b200.kernels import ops
-    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens: sum(-(-seg.q_len // ops.CHUNK) for seg in ctx.segments))
+    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens, least: sum(-(-seg.q_len // ops.CHUNK) for seg in ctx.segments))
     taken = []
-    inner = ops._chunked_scan
-    monkeypatch.setattr(ops, "_chunked_scan", lambda *a, **k: taken.append(inner(*a, **k)) or taken[-1])
+    for name in ("_chunked_scan", "_chunked_delta_scan"):
+        monkeypatch.setattr(ops, name, lambda *a, inner=getattr(ops, name): taken.append(inner(*a)) or taken[-1])
     results = [run()]
     assert taken == [chunks_taken]
-    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens: 0)
+    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens, least: 0)
     results.append(run())
     for got in results:
         for x, y in zip(got, want):
@@ -101,18 +101,48 @@ def test_gated_scan_in_chunks(heads, dim, vdim, lengths, centre, spread, monkeyp
     check(run, want, monkeypatch, True)
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(3, 3, 128, 128), (4, 2, 64, 64), (2, 1, 64, 128), (2, 2, 128, 64)])
+@pytest.mark.parametrize("lengths", LENGTHS, ids=str)
+@pytest.mark.parametrize("centre, spread, alike", [(-3.0, 2.0, 0.0), (-9.0, 1.0, 0.0), (-9.0, 1.0, 1.0), (0.0, 40.0, 0.5)])
+def test_delta_scan_in_chunks(heads, kv_heads, dim, vdim, lengths, centre, spread, alike, monkeypatch):
+    """Keys apart and (``alike``) nearly the same key again and again, which couples a chunk's writes the most."""
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(sum(lengths) + dim)
+    ctx, tokens = context(lengths, 7), sum(lengths)
+    y = torch.randn(tokens, 2 * kv_heads * dim + heads * vdim + 4, generator=gen, device=DEV)
+    y[:, kv_heads * dim:2 * kv_heads * dim] += 4 * alike * torch.randn(kv_heads * dim, generator=gen, device=DEV)
+    y = y.bfloat16()
+    q, k = y[:, :kv_heads * dim], y[:, kv_heads * dim:2 * kv_heads * dim]
+    v = y[:, 2 * kv_heads * dim:2 * kv_heads * dim + heads * vdim]
+    a = torch.randn(tokens, heads * dim, generator=gen, device=DEV)
+    b = torch.randn(tokens, heads + 3, generator=gen, device=DEV).bfloat16()[:, :heads]
+    a_log = torch.rand(heads, generator=gen, device=DEV) * 3 - 3
+    dt_bias = centre + spread * torch.randn(heads * dim, generator=gen, device=DEV)
+    start = torch.randn(7, heads, dim, vdim, generator=gen, device=DEV)
+    unit = lambda t: (lambda x: x / torch.sqrt((x ** 2).sum(-1, keepdim=True) + 1e-6))(t.double().unflatten(1, (kv_heads, dim)))
+    both = lambda t: t.repeat_interleave(heads // kv_heads, dim=1)
+    g = torch.exp(-torch.exp(a_log.double())[None, :, None] * torch.nn.functional.softplus((a + dt_bias).double()).unflatten(1, (heads, dim)))
+    want = exact(both(unit(q)) * dim ** -0.5, both(unit(k)), v.double().unflatten(1, (heads, vdim)), g, ctx, start,
+                 torch.sigmoid(b.double()))
+
+    def run():
+        state = start.clone()
+        return ops.delta_scan(q, k, v, a, b, a_log, dt_bias, state, ctx, heads, kv_heads, dim, vdim), state
+    check(run, want, monkeypatch, True)
+
+
 def test_which_steps_are_scanned_in_chunks():
     """Long segments, and short ones beside them as long as they pad little; never a captured step."""
     from mrun_b200.kernels import ops
 
     def chunks(lengths):
         return ops._chunks(SimpleNamespace(segments=[SimpleNamespace(q_len=n) for n in lengths], shared={}, num_segments=len(lengths),
-                                           max_q_len=max(lengths)), sum(lengths))
+                                           max_q_len=max(lengths)), sum(lengths), ops.CHUNK_MIN_TOKENS)
     assert chunks([ops.CHUNK_MIN_TOKENS - 1]) == 0
     assert chunks([ops.CHUNK_MIN_TOKENS]) == -(-ops.CHUNK_MIN_TOKENS // ops.CHUNK)
     assert chunks([640, 640, 1, 1]) == 22
     assert chunks([256] + [1] * 20) == 0
-    assert ops._chunks(SimpleNamespace(segments=[], shared={}, num_segments=4, max_q_len=500), 4) == 0
+    assert ops._chunks(SimpleNamespace(segments=[], shared={}, num_segments=4, max_q_len=500), 4, 1) == 0
 
 
 def test_rows_without_a_chunked_form_are_walked(monkeypatch):
