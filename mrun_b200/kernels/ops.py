@@ -25,7 +25,9 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def _stream() -> ctypes.c_void_p:
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device.  Asked for by its raw handle: a Stream object took 29 % of an
+    uncaptured step's host time (a mixer's decode step of five kernels on B200: 119 us a pass, 96 without)."""
+    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
