@@ -477,6 +477,51 @@ gated_norm_kernel(const float* __restrict__ o, const float* __restrict__ w, int 
     }
 }
 
+// The same eight features at a time in 16-byte pieces, read once and kept in registers: LANES lanes a (token,
+// group) of up to 32 * LANES features (a multiple of 8, fewer than 1,024).  Bound by the exponential and the division
+// of every gate: 2,048 tokens x 32 heads of 128, 67 MB, 27.7 us against 35.3 an element a lane.  (A block a group of
+// 2,048 features this way takes 19.2 us against 18.1 for the kernel below, so wide groups stay there.)
+template <typename TA, int LANES>
+__global__ void __launch_bounds__(128)
+gated_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_len, const TA* __restrict__ gate, long ldg, float eps,
+                      TA* __restrict__ out, long ldo, float scale, long pairs, int groups, int n, int gate_silu) {
+    constexpr int EACH = 128 / LANES;     // pairs a block
+    const long pair = (long)blockIdx.x * EACH + threadIdx.x / LANES;
+    const int lane = threadIdx.x % LANES, pieces = n >> 3;
+    const bool in = pair < pairs;         // the others keep their warp company
+    const long t = in ? pair / groups : 0;
+    const int c0 = in ? (int)(pair - t * groups) * n : 0;
+    const float* row = o + (t * groups) * n + c0;
+    const TA* grow = gate + t * ldg + c0;
+    float y[4][8], gv[4][8];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (in && lane + i * LANES < pieces) {
+            Vec8<float>::load(row + (lane + i * LANES) * 8, y[i]);
+            Vec8<TA>::load(grow + (lane + i * LANES) * 8, gv[i]);
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (in && lane + i * LANES < pieces)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ss = fmaf(y[i][e], y[i][e], ss);
+#pragma unroll
+    for (int d = LANES / 2; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    const float inv = scale / sqrtf(ss / (float)n + eps);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (in && lane + i * LANES < pieces) {
+            const int c = c0 + (lane + i * LANES) * 8;
+            float wv[8];
+            Vec8<float>::load(w + (w_len == n ? c - c0 : c), wv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                y[i][e] = y[i][e] * inv * wv[e] * ((gate_silu ? gv[i][e] : 1.f) / (1.f + expf(-gv[i][e])));
+            Vec8<TA>::store(out + t * ldo + c, y[i]);
+        }
+}
+
 // A block a (token, group), for groups of many features.  The sums differ from the warp kernel's in
 // their order; which of the two runs depends on the group's size only.
 template <typename TA>
@@ -498,6 +543,19 @@ gated_norm_block_kernel(const float* __restrict__ o, const float* __restrict__ w
         const float gv = to_float(gate[t * ldg + c]);
         out[t * ldo + c] = from_float<TA>(row[i] * inv * w[c % w_len] * ((gate_silu ? gv : 1.f) / (1.f + expf(-gv))));
     }
+}
+
+// Groups of 64 and 128 features are a piece a lane.
+template <typename TA>
+void launch_gated_norm_vec(const float* o, const float* w, int w_len, const void* gate, long ldg, float eps, void* out, long ldo, float scale,
+                           long pairs, int groups, int n, int gate_silu, cudaStream_t stream) {
+#define MRUN_GATED_NORM(LANES)                                                                                                   \
+    gated_norm_vec_kernel<TA, LANES><<<(unsigned)((pairs + 128 / LANES - 1) / (128 / LANES)), 128, 0, stream>>>(                     \
+        o, w, w_len, (const TA*)gate, ldg, eps, (TA*)out, ldo, scale, pairs, groups, n, gate_silu)
+    if (n <= 64) MRUN_GATED_NORM(8);
+    else if (n <= 128) MRUN_GATED_NORM(16);
+    else MRUN_GATED_NORM(32);
+#undef MRUN_GATED_NORM
 }
 
 // ------------------------------------------------------------------------------------------
@@ -915,6 +973,16 @@ MRUN_API int mrun_gated_norm(const float* o, const float* w, int w_len, const vo
     if (tokens == 0) return 0;
     const long pairs = (long)tokens * groups;
     const unsigned blocks = (unsigned)((pairs + 3) / 4);
+    const size_t unit = act_dtype == MRUN_F32 ? 4 : 2;
+    if (n % 8 == 0 && n < 1024 && (w_len == n || w_len == groups * n) && ldg * unit % 16 == 0 && ldo * unit % 16 == 0 &&
+        (((uintptr_t)o | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15) == 0 && (act_dtype == MRUN_F32 || act_dtype == MRUN_BF16)) {
+        if (act_dtype == MRUN_F32)
+            launch_gated_norm_vec<float>(o, w, w_len, gate, ldg, eps, out, ldo, scale, pairs, groups, n, gate_silu, stream);
+        else
+            launch_gated_norm_vec<__nv_bfloat16>(o, w, w_len, gate, ldg, eps, out, ldo, scale, pairs, groups, n, gate_silu, stream);
+        MRUN_CHECK_LAUNCH("gated_norm");
+        return 0;
+    }
     if (n >= 1024) {            // a block a pair
         if (act_dtype == MRUN_F32)
             gated_norm_block_kernel<float><<<(unsigned)pairs, 256, 0, stream>>>(o, w, w_len, (const float*)gate, ldg, eps,

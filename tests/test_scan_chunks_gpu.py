@@ -161,3 +161,23 @@ def test_rows_without_a_chunked_form_are_walked(monkeypatch):
             return ops.decay_scan(q, k, v, decay, state, ctx, 1, dim, dim, False), state
         with monkeypatch.context() as m:
             check(run, want, m, False)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("groups, n", [(3, 8), (5, 64), (2, 72), (7, 128), (3, 136), (2, 1016), (1, 1024), (2, 8192), (1, 8200)])
+@pytest.mark.parametrize("shared", [False, True])
+def test_gated_norm_in_pieces(dtype, groups, n, shared):
+    """Group sizes on both sides of every number of threads, weights a group or a row long, strided gates and outputs."""
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    for tokens in (1, 13):
+        o, gate, weight = rand(tokens, groups * n), rand(tokens, groups * n + 8).to(dtype)[:, 8:], rand(n if shared else groups * n)
+        out = torch.full((tokens, groups * n + 16), 7.0, dtype=dtype, device=DEV)
+        ops.gated_norm(o, weight, gate, 1e-5, groups, dtype, gate_function="silu", out=out[:, :groups * n], scale=0.5)
+        x = o.double().view(tokens, groups, n)
+        want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * weight.double().view(1, -1, n)
+        want = 0.5 * want.flatten(1) * torch.nn.functional.silu(gate.double())
+        # a few roundings of 2^-24 behind a sum of n squares; bfloat16 rounds the result to 8 bits
+        assert ((out[:, :groups * n].double() - want).abs() <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * want.abs() + 1e-6).all()
+        assert (out[:, groups * n:] == 7.0).all()
