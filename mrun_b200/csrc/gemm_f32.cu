@@ -14,7 +14,7 @@
 //           long.  BM x BN outputs a block, TM x TN a thread as pairs of columns (packed fused multiply-adds,
 //           two a lane and instruction, which leaves issue slots for the loads), k slices of 16 brought
 //           k-major by asynchronous 4-byte copies, so no operand needs an alignment of its own.  517 rows, K =
-//           4,096: N = 24,576 2,275 us (64 x 64 tiles of one slice at a time: 3,676), 46 TFLOP/s of 74; N = 6,144
+//           4,096: N = 24,576 2,241 us (64 x 64 tiles of one slice at a time: 3,676), 46 TFLOP/s of 74; N = 6,144
 //           594 us (1,132).  Thread tiles of 8 x 16, which read less, leave too few warps: 2,865 us.
 #include "common.cuh"
 
@@ -154,15 +154,29 @@ gemm_f32_tile_kernel(const float* __restrict__ x, const float* __restrict__ w, f
     // copies: a thread keeps its k within the slice and walks over rows
     constexpr int PER = THREADS / TILE_K;
     const int ck = tid % TILE_K, row_of = tid / TILE_K, place = row_of ^ (ck & 8 ? 2 : 0);
+    // The FMAs share their issue slots with this arithmetic: a thread's rows by an addition each from its first, held on
+    // the last row there is, instead of a clamped index times the pitch (517 rows, K = 4,096, N = 24,576, B200:
+    // 2,306 -> 2,241 us; 100 rows, K = 12,288: 464 -> 433).
+    const float* x_first = x + (size_t)min(row0 + row_of, M - 1) * ldx;
+    const float* w_first = w + (size_t)min(col0 + row_of, N - 1) * K;
+    const long x_step = (long)PER * ldx, w_step = (long)PER * K;
+    const int x_rows = M - row0 - row_of, w_rows = N - col0 - row_of;      // of this thread's rows on
     auto fetch = [&](int step) {
         float* as = smem + (step % TILE_STAGES) * STAGE + ck * PM + place;
         float* bs = smem + (step % TILE_STAGES) * STAGE + TILE_K * PM + ck * PN + place;
         const int k = step * TILE_K + ck;
         const int bytes = k < K ? 4 : 0, at = k < K ? k : 0;
+        const float *x_at = x_first + at, *w_at = w_first + at;
 #pragma unroll
-        for (int r = 0; r < BM; r += PER) copy_4_or_zero(as + r, x + (size_t)min(row0 + r + row_of, M - 1) * ldx + at, bytes);
+        for (int r = 0; r < BM; r += PER) {
+            copy_4_or_zero(as + r, x_at, bytes);
+            x_at += r + PER < x_rows ? x_step : 0;
+        }
 #pragma unroll
-        for (int r = 0; r < BN; r += PER) copy_4_or_zero(bs + r, w + (size_t)min(col0 + r + row_of, N - 1) * K + at, bytes);
+        for (int r = 0; r < BN; r += PER) {
+            copy_4_or_zero(bs + r, w_at, bytes);
+            w_at += r + PER < w_rows ? w_step : 0;
+        }
     };
 #pragma unroll
     for (int s = 0; s < TILE_STAGES - 1; ++s) {
