@@ -17,9 +17,10 @@
 // Pairs of tokens within a run multiply their decays one after the other as the walk does.
 //
 // Bound by the FMA pipe, the shared-memory reads that feed it (thread tiles of 8 x 8) and, in prepare, by the
-// exponentials.  2,048 tokens, 16 heads of 128 x 128, walked / in chunks, us: decay 526 / 131 (prepare 64, carry
-// 15, finish 43), gated 566 / 146 (85, 15, 38); 32 heads 625 / 248 and 681 / 276, the carry then 56 since its 117
-// MB of scratch leave the L2 cache.
+// exponentials.  2,048 tokens, 16 heads of 128 x 128, walked / in chunks, us: decay 521 / 118 (prepare 64, carry
+// 13, finish 41), gated 561 / 133; 32 heads 621 / 229 and 677 / 258 (prepare 145, carry 53, finish 60: its 117
+// MB of scratch leave the L2 cache).  finish leaves out the values that come after a row's token, runs of them as a whole
+// (decay 44 -> 41, delta 36 -> 34).
 #include "common.cuh"
 
 using namespace mrun;
@@ -397,8 +398,29 @@ chunk_carry_kernel(const ChunkArgs w) {
     store4(st, s);
 }
 
-constexpr int SLICE = 16, STAGES = 3;        // k of a slice, slices in flight
+constexpr int SLICE = SUB, STAGES = 3;       // k of a slice, slices in flight
 template <int V> constexpr int finish_smem() { return STAGES * SLICE * (CHUNK + V) * (int)sizeof(float); }
+
+// Four rows of a thread's outputs over one slice of values; with SEEN, row i takes the values up to its own, the slice's
+// (row + i)-th.
+template <int V, bool SEEN>
+__device__ __forceinline__ void quad_rows(const float* as, const float* bs, int row, float2 (&x0)[4], float2 (&x1)[4], float2 (&x2)[4],
+                                          float2 (&x3)[4]) {
+#pragma unroll 4
+    for (int k = 0; k < SLICE; ++k) {
+        const float4 a = load4(as + k * CHUNK);
+        float2 b[4];
+        *reinterpret_cast<float4*>(b) = load4(bs + k * V);
+        *reinterpret_cast<float4*>(b + 2) = load4(bs + k * V + V / 2);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!SEEN || k <= row) x0[j] = __ffma2_rn(make_float2(a.x, a.x), b[j], x0[j]);
+            if (!SEEN || k <= row + 1) x1[j] = __ffma2_rn(make_float2(a.y, a.y), b[j], x1[j]);
+            if (!SEEN || k <= row + 2) x2[j] = __ffma2_rn(make_float2(a.z, a.z), b[j], x2[j]);
+            if (!SEEN || k <= row + 3) x3[j] = __ffma2_rn(make_float2(a.w, a.w), b[j], x3[j]);
+        }
+    }
+}
 
 template <int MODE, int D, int V>
 __global__ void __launch_bounds__(V, 512 / V)
@@ -458,8 +480,22 @@ chunk_finish_kernel(const ChunkArgs w) {
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* as = smem + (step % STAGES) * SLICE * (CHUNK + V);
         const float* bs = as + SLICE * CHUNK;
+        if (step < STATE_STEPS) {
 #pragma unroll
-        for (int k = 0; k < SLICE; ++k) outer8<CHUNK, V>(as + k * CHUNK + ty * 4, bs + k * V + tx * 4, acc);
+            for (int k = 0; k < SLICE; ++k) outer8<CHUNK, V>(as + k * CHUNK + ty * 4, bs + k * V + tx * 4, acc);
+            continue;
+        }
+        // A value enters the sums of its own token and of later ones only (zero times an infinity is no number): a
+        // slice is one run's values, a warp's quads of rows lie in one run of the chunk's first half and one of its second.
+        const int run = step - STATE_STEPS;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int ahead = half * (SUBS / 2) + ty / 4 - run;           // the rows' run before (negative), at or after the values'
+            const float* a = as + half * (CHUNK / 2) + ty * 4;
+            if (ahead > 0) quad_rows<V, false>(a, bs + tx * 4, 0, acc[half * 4], acc[half * 4 + 1], acc[half * 4 + 2], acc[half * 4 + 3]);
+            if (ahead == 0)
+                quad_rows<V, true>(a, bs + tx * 4, ty % 4 * 4, acc[half * 4], acc[half * 4 + 1], acc[half * 4 + 2], acc[half * 4 + 3]);
+        }
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -479,8 +515,8 @@ chunk_finish_kernel(const ChunkArgs w) {
 // columns a thread; the carry is a chain of two products a chunk, U = U0 - W S and S' = G S + k^T U, for a slice of
 // value columns a block; finish is the same.  The carry is bound by the shared-memory reads of its two products and,
 // with one block a multiprocessor, by their latency (3.9 us a chunk).  16 heads of 128 x 128, walked / in chunks, us:
-// 2,048 tokens 647 / 266 (prepare 99, carry 124, finish 36), segments of 396, 592 and 789 tokens 351 / 249 (97, 108,
-// 36; the segments in the order they come instead of the longest first, and reads that met banks twice: 174).
+// 2,048 tokens 642 / 257 (prepare 99, carry 124, finish 34), segments of 396, 592 and 789 tokens 346 / 239 (96, 108,
+// 34; the segments in the order they come instead of the longest first, and reads that met banks twice: 174).
 // ------------------------------------------------------------------------------------------
 constexpr int PAIR_FLOATS = SUBS * (SUBS + 1) / 2 * SUB * SUB;     // L below and on its diagonal blocks, [block][j][i]
 __host__ __device__ constexpr int pair_block(int run_i, int run_j) { return (run_i * (run_i + 1) / 2 + run_j) * SUB * SUB; }

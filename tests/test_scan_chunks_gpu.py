@@ -131,6 +131,41 @@ def test_delta_scan_in_chunks(heads, kv_heads, dim, vdim, lengths, centre, sprea
     check(run, want, monkeypatch, True)
 
 
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (64, 64)])
+@pytest.mark.parametrize("kind", ["decay", "gated", "delta"])
+def test_earlier_tokens_do_not_meet_later_values_that_are_no_numbers(kind, dim, vdim, monkeypatch):
+    """A key or a value that is infinite or no number spoils its own token and later ones of its request, as in the walk; the
+    tokens before it keep their bits."""
+    from mrun_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(dim)
+    heads, ctx, tokens = 2, context([150, 70], 7), 220
+    y = torch.randn(tokens, heads * (2 * dim + vdim), generator=gen, device=DEV).bfloat16()
+    a, bias = torch.randn(tokens, heads * dim, generator=gen, device=DEV), torch.full((heads * dim,), 2.0, device=DEV)
+    b = torch.randn(tokens, heads, generator=gen, device=DEV).bfloat16()
+    rate = torch.full((heads,), -2.0, device=DEV)
+    monkeypatch.setattr(ops, "_chunks", lambda ctx, tokens, least: sum(-(-seg.q_len // ops.CHUNK) for seg in ctx.segments))
+
+    def run(y):
+        q, k, v = y[:, :heads * dim], y[:, heads * dim:2 * heads * dim], y[:, 2 * heads * dim:]
+        state = torch.ones(7, heads, dim, vdim, device=DEV)
+        if kind == "decay":
+            return ops.decay_scan(q, k, v, torch.full((heads,), 0.9, device=DEV), state, ctx, heads, dim, vdim, True)
+        if kind == "gated":
+            return ops.gated_scan(q, k, v, a, bias, 8.0, state, ctx, heads, dim, vdim)
+        return ops.delta_scan(q, k, v, a, b, rate, bias, state, ctx, heads, heads, dim, vdim)
+    want = run(y)
+    assert torch.isfinite(want).all()
+    keys, values = slice(heads * dim, 2 * heads * dim), slice(2 * heads * dim, None)
+    for at in (0, 1, 37, 63, 64, 79, 149):         # the chunk's and the runs' edges, both halves of a chunk
+        for what in (float("inf"), float("nan")):
+            for spoilt in (keys, values):
+                rows = y.clone()
+                rows[at, spoilt] = what
+                got = run(rows)
+                assert torch.equal(got[:at], want[:at]) and torch.equal(got[150:], want[150:]), (at, what, spoilt)
+                assert not torch.isfinite(got[at]).any()
+
+
 def test_which_steps_are_scanned_in_chunks():
     """Long segments, and short ones beside them as long as they pad little; never a captured step."""
     from mrun_b200.kernels import ops
