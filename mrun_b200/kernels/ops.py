@@ -1396,27 +1396,68 @@ def _strided_rows(t: torch.Tensor, name: str) -> int:
 
 CHUNK = 64                # tokens a chunk of the chunked scans
 # The longest segment from which on they are worth their three kernels (B200, 16 heads of 128, decay / gated scan, us:
-# 128 tokens 47 / 48 in chunks and 47 / 48 walked, 160 tokens 52 / 48 and 55 / 56, 2,048 tokens 131 / 146 and 526 / 566).
+# 128 tokens 39 / 41 in chunks and 41 / 42 walked, 192 tokens 40 / 42 and 56 / 59, 2,048 tokens 118 / 133 and 521 / 561).
 CHUNK_MIN_TOKENS = 128
-# The same for the delta scan (200 tokens 70 in chunks, 74 walked; 128 tokens 62 and 54; 2,048 tokens 266 and 647).
+# The same for the delta scan (192 tokens 59 in chunks, 67 walked; 128 tokens 56 and 48; 2,048 tokens 257 and 642).
 DELTA_CHUNK_MIN_TOKENS = 192
+_NEVER = 1 << 30
+
+
+def _chunk_count(ctx) -> int:
+    """Chunks of the step's segments, 0 where the step's segments are not known on the host."""
+    if len(ctx.segments) != ctx.num_segments:
+        return 0
+    n = ctx.shared.get("scan_chunks")
+    if n is None:
+        n = ctx.shared["scan_chunks"] = sum(-(-seg.q_len // CHUNK) for seg in ctx.segments)
+    return n
+
+
+def _chunk_least(ctx, tokens: int, delta: bool, heads: int, dim: int, vdim: int) -> int:
+    """Tokens that the step's longest segment has at least where the chunked scans take the step, _NEVER where
+    the walk is the faster one whatever its length.
+
+    A walk takes as long as its longest segment while its blocks fit the device, and longer in proportion once heads
+    and segments side by side fill it; the chunks take a time in proportion to (chunk, head) pairs and, in a delta
+    scan, a step a chunk of the longest segment.  ``side``: rows of chunks times heads over the longest segment, how many
+    chains lie side by side.  On B200, us in chunks / walked (the lines below lie where the two meet):
+
+    * heads of 128 x 128: chunks from the thresholds on; at 128 tokens and (chunk, head) pairs for less than half of the
+      device the decay and gated scans lose by up to 7 % (4 heads, one segment 40 / 37, sixteen segments 44 / 62);
+    * decay and gated, 64 x 64: a walk has a quarter of the work and the chunks' padding counts: 16 segments of 160
+      tokens, a sixth of the chunks' rows empty, 64 heads 311 / 288 and 4 heads 38 / 45; of 128 tokens, 64 heads 212 / 237;
+    * delta, 64 x 64: 8 segments of 192 tokens, 32 heads 154 / 121, 64 heads 285 / 218, but one segment of 192 and 64
+      heads 54 / 69, two of 1,024 375 / 391; 64 x 128: segments of 200, 40 and 300, 64 heads 189 / 171; 128 x 64 loses
+      where rows are padded (three segments of 300 and three short ones, 32 heads 178 / 162) and not without
+      (8 segments of 192 tokens, 32 heads 256 / 261)."""
+    least, longest = DELTA_CHUNK_MIN_TOKENS if delta else CHUNK_MIN_TOKENS, ctx.max_q_len
+    n = _chunk_count(ctx) if longest >= least else 0
+    if not n:
+        return least
+    rows = CHUNK * n
+    side, padded, small = heads * rows / longest, 10 * rows > 11 * tokens, dim * vdim < 128 * 64
+    if dim * vdim >= 128 * 128:
+        return least if delta or heads * n >= 64 else 160
+    if not delta:
+        return _NEVER if small and padded and side > 280 else least
+    if dim >= 128 and not padded:
+        return least
+    return least if side * longest <= (200 if small else 160) * (longest - 111) else _NEVER
 
 
 def _chunks(ctx, tokens: int, least: int) -> int:
     """Chunks of the step's segments where the chunked scans take the step: a segment of at least
     ``least`` tokens, and short segments, each a chunk of its own, that pad the chunks by no more than a quarter of
-    the rows and one chunk.  0 otherwise."""
-    if ctx.max_q_len < least or len(ctx.segments) != ctx.num_segments:
-        return 0
-    n = ctx.shared.get("scan_chunks")
-    if n is None:
-        n = ctx.shared["scan_chunks"] = sum(-(-seg.q_len // CHUNK) for seg in ctx.segments)
+    the rows and one chunk (which bounds the scratch; steps beyond it are walked as a whole, although chunks
+    would still be the faster form for most: a decay scan of 16 heads of 128 over a segment of 1,024 tokens
+    takes 138 us in chunks and 297 walked beside 16 single tokens).  0 otherwise."""
+    n = 0 if ctx.max_q_len < least else _chunk_count(ctx)
     return n if 4 * CHUNK * n <= 5 * tokens + 4 * CHUNK else 0
 
 
 def _chunk_scratch(ctx, delta: bool, q, k, v, ld: int, a, bias, state, out, heads: int, dim: int, vdim: int):
     """(scratch, chunks) of a scan that runs chunk by chunk, or None where it is walked."""
-    chunks = _chunks(ctx, q.shape[0], DELTA_CHUNK_MIN_TOKENS if delta else CHUNK_MIN_TOKENS)
+    chunks = _chunks(ctx, q.shape[0], _chunk_least(ctx, q.shape[0], delta, heads, dim, vdim))
     if not chunks:
         return None
     size = _lib.core().function("mrun_chunked_scan_floats")
