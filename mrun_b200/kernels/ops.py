@@ -1455,6 +1455,15 @@ def _chunks(ctx, tokens: int, least: int) -> int:
     return n if 4 * CHUNK * n <= 5 * tokens + 4 * CHUNK else 0
 
 
+def chunk_scratch_elements(dim: int, vdim: int, delta: bool) -> int:
+    """16-bit elements a token and head of the chunked scans' scratch at most, with the padding that :func:`_chunks`
+    admits (its one chunk beside that left to the engine's fixed allowance); 0 for sizes that are walked."""
+    if dim not in (64, 128) or vdim not in (64, 128):
+        return 0
+    floats = (dim + CHUNK) * CHUNK + dim * vdim + dim + (CHUNK * (2 * dim + vdim) if delta else 0)      # of a chunk
+    return -(-5 * 2 * floats // (4 * CHUNK))
+
+
 def _chunk_scratch(ctx, delta: bool, q, k, v, ld: int, a, bias, state, out, heads: int, dim: int, vdim: int):
     """(scratch, chunks) of a scan that runs chunk by chunk, or None where it is walked."""
     chunks = _chunks(ctx, q.shape[0], _chunk_least(ctx, q.shape[0], delta, heads, dim, vdim))

@@ -59,8 +59,8 @@ class ChannelDelta:
 
     def activation_elements(self) -> int:
         s = self.spec
-        # the chunked scan's scratch among them: per head two states, two rows of keys and one of values a chunk
-        return 2 * self.channels + s.heads * (1 + 12 * s.dim + 9 * s.vdim) + s.decay_rank + s.gate_rank
+        scratch = ops.chunk_scratch_elements(s.dim, s.vdim, True)
+        return 2 * self.channels + s.heads * (1 + 2 * s.dim + 3 * s.vdim + scratch) + s.decay_rank + s.gate_rank
 
     def cache_need(self):
         s = self.spec

@@ -43,7 +43,7 @@ class DecayAttention:
 
     def activation_elements(self) -> int:
         s = self.spec
-        return s.heads * (7 * s.dim + 7 * s.vdim)        # the scan's scratch among them
+        return s.heads * (2 * s.dim + 5 * s.vdim + ops.chunk_scratch_elements(s.dim, s.vdim, False))
 
     def cache_need(self):
         s = self.spec

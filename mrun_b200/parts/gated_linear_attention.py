@@ -49,7 +49,7 @@ class GatedLinearAttention:
 
     def activation_elements(self) -> int:
         s = self.spec
-        return s.heads * (8 * s.dim + 7 * s.vdim) + s.rank        # the scan's scratch among them
+        return s.heads * (5 * s.dim + 5 * s.vdim + ops.chunk_scratch_elements(s.dim, s.vdim, False)) + s.rank
 
     def cache_need(self):
         s = self.spec

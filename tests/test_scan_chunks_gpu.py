@@ -216,3 +216,55 @@ def test_gated_norm_in_pieces(dtype, groups, n, shared):
         # a few roundings of 2^-24 behind a sum of n squares; bfloat16 rounds the result to 8 bits
         assert ((out[:, :groups * n].double() - want).abs() <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * want.abs() + 1e-6).all()
         assert (out[:, groups * n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("kind", ["decay", "gated", "delta"])
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (64, 128), (128, 64), (64, 64)])
+def test_a_mixer_holds_no_more_than_it_declares(kind, dim, vdim):
+    """Beside its inputs and outputs, over a step whose segments pad the chunks nearly as much as a chunked step may."""
+    from mrun_b200.config import spec as specs
+    from mrun_b200.engine import StepEntry
+    from mrun_b200.engine.batch import HostStaging, build_context
+    from mrun_b200.cache import CacheManager
+    from mrun_b200.kernels import ops
+    from mrun_b200.parts import MIXERS, Precision, Runtime
+    hidden, heads, lengths = 256, 16, [641] * 3 + [1] * 4
+    spec = {"decay": lambda: specs.DecayAttentionSpec(hidden=hidden, heads=heads, dim=dim, vdim=vdim, eps=1e-5, decay=(0.9,) * heads),
+            "gated": lambda: specs.GatedLinearAttentionSpec(hidden=hidden, heads=heads, dim=dim, vdim=vdim, tau=8.0, rank=16, eps=1e-5),
+            "delta": lambda: specs.ChannelDeltaSpec(hidden=hidden, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, conv=4, decay_rank=16,
+                                                    gate_rank=16, eps=1e-5)}[kind]()
+    rt = Runtime(torch.device(DEV), Precision.of("bfloat16"), 16)
+    gen = torch.Generator().manual_seed(1)
+    weights = {t.name[2:]: 0.1 * torch.randn(t.shape, generator=gen) for t in MIXERS.tensor_specs(spec, "m")}
+    part = MIXERS.build(spec, weights, rt)
+    manager = CacheManager([part.cache_need()], [None], 16, 200, len(lengths), device=torch.device(DEV), dtype=torch.bfloat16)
+    requests = [manager.admit(i) for i in range(len(lengths))]
+    manager.plan_append(list(zip(requests, lengths)))
+    ctx = build_context([StepEntry(r, [0] * n) for r, n in zip(requests, lengths)], manager, HostStaging(torch.device(DEV)))
+    tokens = sum(lengths)
+    assert ops._chunks(ctx, tokens, ops._chunk_least(ctx, tokens, kind == "delta", heads, dim, vdim))
+    x = torch.randn(tokens, hidden, device=DEV).bfloat16()
+    part.forward(x, ctx, manager.entries[0])                     # the vendor library's workspace
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    part.forward(x, ctx, manager.entries[0])
+    held = torch.cuda.max_memory_allocated() - before
+    chunk = heads * ops.chunk_scratch_elements(dim, vdim, kind == "delta") * ops.CHUNK * 2         # the one chunk beside the quarter
+    assert held <= 2 * tokens * (part.activation_elements() + hidden) + chunk
+
+
+def test_declared_scratch_is_the_kernels():
+    """The estimate's floats of a chunk are those that the kernels ask for."""
+    from mrun_b200.kernels import ops
+    like = torch.empty(64, 128, device=DEV)
+    q = torch.empty(64, 128, device=DEV, dtype=torch.bfloat16)
+    for delta in (False, True):
+        for dim in (64, 128):
+            for vdim in (64, 128):
+                size = ops._lib.core().function("mrun_chunked_scan_floats")
+                size.restype = ops._c_long
+                floats = size(ops._c_int(delta), ops._ptr(q), ops._ptr(q), ops._ptr(q), ops._c_long(128), ops._c_int(ops.dtype_code(q.dtype)),
+                              ops._ptr(like), ops._ptr(like), ops._ptr(like), ops._ptr(like), ops._c_int(1), ops._c_int(1), ops._c_int(dim),
+                              ops._c_int(vdim))
+                assert ops.chunk_scratch_elements(dim, vdim, delta) == -(-5 * 2 * floats // (4 * ops.CHUNK))
