@@ -478,10 +478,13 @@ gated_norm_kernel(const float* __restrict__ o, const float* __restrict__ w, int 
 }
 
 // The same eight features at a time in 16-byte pieces, read once and kept in registers: LANES lanes a (token,
-// group) of up to 32 * LANES features (a multiple of 8, fewer than 1,024).  Bound by the exponential and the division
-// of every gate: 2,048 tokens x 32 heads of 128, 67 MB, 27.7 us against 35.3 an element a lane.  (A block a group of
-// 2,048 features this way takes 19.2 us against 18.1 for the kernel below, so wide groups stay there.)
-template <typename TA, int LANES>
+// group) of up to 8 * PIECES * LANES features (a multiple of 8, fewer than 1,024).  Bound by the exponential and the division
+// of every gate: 2,048 tokens x 32 heads of 128, 67 MB, 16.1 us against 35.3 an element a lane (27.7 with four pieces a lane
+// whatever the group, whose registers leave few warps).  (A block a group of 2,048 features this way takes 19.2 us against
+// 18.1 for the kernel below, so wide groups stay there.)  Few groups are bound by one trip to memory after the other, so where
+// a lane has one piece its weights are under way with the row: one token x 16 groups of 8 2.2 us, 2.6 before and 2.0 an
+// element a lane.
+template <typename TA, int LANES, int PIECES>
 __global__ void __launch_bounds__(128)
 gated_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_len, const TA* __restrict__ gate, long ldg, float eps,
                       TA* __restrict__ out, long ldo, float scale, long pairs, int groups, int n, int gate_silu) {
@@ -493,16 +496,18 @@ gated_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, 
     const int c0 = in ? (int)(pair - t * groups) * n : 0;
     const float* row = o + (t * groups) * n + c0;
     const TA* grow = gate + t * ldg + c0;
-    float y[4][8], gv[4][8];
+    const float* wrow = w + (w_len == n ? 0 : c0);
+    float y[PIECES][8], gv[PIECES][8], first[8];
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < PIECES; ++i)
         if (in && lane + i * LANES < pieces) {
             Vec8<float>::load(row + (lane + i * LANES) * 8, y[i]);
             Vec8<TA>::load(grow + (lane + i * LANES) * 8, gv[i]);
         }
+            if constexpr (PIECES == 1) Vec8<float>::load(wrow + lane * 8, first);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < PIECES; ++i)
         if (in && lane + i * LANES < pieces)
 #pragma unroll
             for (int e = 0; e < 8; ++e) ss = fmaf(y[i][e], y[i][e], ss);
@@ -510,11 +515,16 @@ gated_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, 
     for (int d = LANES / 2; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
     const float inv = scale / sqrtf(ss / (float)n + eps);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < PIECES; ++i)
         if (in && lane + i * LANES < pieces) {
             const int c = c0 + (lane + i * LANES) * 8;
             float wv[8];
-            Vec8<float>::load(w + (w_len == n ? c - c0 : c), wv);
+            if constexpr (PIECES == 1) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) wv[e] = first[e];
+            } else {
+                Vec8<float>::load(wrow + (lane + i * LANES) * 8, wv);
+            }
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 y[i][e] = y[i][e] * inv * wv[e] * ((gate_silu ? gv[i][e] : 1.f) / (1.f + expf(-gv[i][e])));
@@ -545,16 +555,16 @@ gated_norm_block_kernel(const float* __restrict__ o, const float* __restrict__ w
     }
 }
 
-// Groups of 64 and 128 features are a piece a lane.
 template <typename TA>
 void launch_gated_norm_vec(const float* o, const float* w, int w_len, const void* gate, long ldg, float eps, void* out, long ldo, float scale,
                            long pairs, int groups, int n, int gate_silu, cudaStream_t stream) {
-#define MRUN_GATED_NORM(LANES)                                                                                                   \
-    gated_norm_vec_kernel<TA, LANES><<<(unsigned)((pairs + 128 / LANES - 1) / (128 / LANES)), 128, 0, stream>>>(                     \
+#define MRUN_GATED_NORM(LANES, PIECES)                                                                                           \
+    gated_norm_vec_kernel<TA, LANES, PIECES><<<(unsigned)((pairs + 128 / LANES - 1) / (128 / LANES)), 128, 0, stream>>>(             \
         o, w, w_len, (const TA*)gate, ldg, eps, (TA*)out, ldo, scale, pairs, groups, n, gate_silu)
-    if (n <= 64) MRUN_GATED_NORM(8);
-    else if (n <= 128) MRUN_GATED_NORM(16);
-    else MRUN_GATED_NORM(32);
+    if (n <= 64) MRUN_GATED_NORM(8, 1);
+    else if (n <= 128) MRUN_GATED_NORM(16, 1);
+    else if (n <= 256) MRUN_GATED_NORM(32, 1);
+    else MRUN_GATED_NORM(32, 4);
 #undef MRUN_GATED_NORM
 }
 
