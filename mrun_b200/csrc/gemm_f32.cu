@@ -286,6 +286,7 @@ int launch_product(const float* x, const float* w, float* y, int batch, int M, i
     float least = 0.f;
     for (int i = 0; i < 3; ++i) {
         const TileCost& c = TILE_COSTS[i];
+        if (i > 0 && (M + c.bm - 1) / c.bm > 65535) continue;         // more rows of tiles than a grid has
         const long tiles = (long)((M + c.bm - 1) / c.bm) * ((N + c.bn - 1) / c.bn) * batch;
         const float cost = fmaxf(c.alone, c.each * (float)((tiles + sms - 1) / sms));
         if (i == 0 || cost < least) { best = i; least = cost; }

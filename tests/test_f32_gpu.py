@@ -34,6 +34,15 @@ def test_products_of_every_row_count_agree_in_bits(n, k):
         assert torch.equal(ops.gemm_f32_nt(wide[:m, 3:], w), ops.gemm_f32_nt(wide[:m, 3:].contiguous(), w)), m
 
 
+def test_products_of_more_rows_than_small_tiles_reach():
+    """Few columns would choose tiles of 32 rows, of which a grid holds 65,535."""
+    from mrun_b200.kernels import ops
+    m = 65535 * 32 + 5
+    x, w = torch.randn(m, 4, generator=torch.Generator(device=DEV).manual_seed(6), device=DEV), rows(8, 4, 7)
+    got, want = ops.gemm_f32_nt(x, w), x.double() @ w.double().T
+    assert (got.double() - want).abs().max() <= 2.0 ** -24 * 4 * (x.double().abs() @ w.double().abs().T).max()
+
+
 @pytest.mark.parametrize("m", [1, 5, 16, 40])
 def test_batched_products(m):
     from mrun_b200.kernels import ops
