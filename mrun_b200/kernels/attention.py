@@ -259,14 +259,15 @@ F32_TILE_ROWS = 64       # token rows x group heads of a tile of the 32-bit atte
 F32_TILE_GROUP = 16      # query heads a kv head that it takes
 
 
-def f32_tiles_ok(q: torch.Tensor, q_stride: int, head_dim: int, value_dim: int, ratio: int) -> bool:
+def f32_tiles_ok(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, ratio: int) -> bool:
     """Whether the tiled 32-bit kernel takes this shape: heads of 64 or 128 features, rows on 16 bytes,
     groups of up to 16 heads.  The kernel with a block a token and head reads the keys again for every row (B200,
     32 heads over 8 of 128: prompts of 207 and 310 tokens 1,183 us against 103; four single tokens at contexts of 75
     to 300, 44 against 30); wider groups stay with it, prompts and single tokens alike, since a block a token
     and kv head leaves single tokens of theirs too few blocks (40 heads over 2: 78 us against 139)."""
-    return (q.dtype == torch.float32 and head_dim == value_dim and head_dim in (64, 128) and ratio <= F32_TILE_GROUP
-            and q_stride % 4 == 0 and q.data_ptr() % 16 == 0)
+    head_dim = cache.k.shape[3]
+    return (q.dtype == torch.float32 and head_dim == cache.v.shape[3] and head_dim in (64, 128) and ratio <= F32_TILE_GROUP
+            and q_stride % 4 == 0 and not any(t.data_ptr() % 16 for t in (q, out, cache.k, cache.v)))
 
 
 def _paged_attention_f32(q, q_stride: int, out, cache, group, ctx, heads: int, scale: float, window: int) -> torch.Tensor:
@@ -325,7 +326,7 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
                          _c_long(pages * page_size), _c_float(scale), _c_int(splits), _ptr(part_o), _ptr(part_ml),
                          _stream())
         return out
-    if sink is None and form is None and f32_tiles_ok(q, q_stride, head_dim, v_dim, ratio):
+    if sink is None and form is None and f32_tiles_ok(q, q_stride, out, cache, ratio):
         return _paged_attention_f32(q, q_stride, out, cache, group, ctx, heads, scale, window)
     if not supports_tensor_cores(q.dtype, head_dim, ratio, v_dim):
         return ops.paged_attention_generic(q, q_stride, out, cache.k, cache.v, group.block_tables,

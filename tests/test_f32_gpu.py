@@ -93,3 +93,22 @@ def test_what_a_row_does_not_see_does_not_enter_its_sums():
     case.vd[page, :, at] = float("inf")
     got = case.run(0.125)
     assert torch.equal(got[:30], want[:30]) and not torch.isfinite(got[30:]).all()
+
+
+def test_tiled_attention_leaves_unaligned_outputs_to_the_general_kernel():
+    """Outputs, keys or values that do not start on 16 bytes are taken as before."""
+    from mrun_b200.kernels.attention import paged_attention
+    case = Case([(0, 20), (30, 1)], 4, 2, 64, 16, torch.float32, seed=10)
+    want = case.run(0.125)
+    shifted = lambda t: torch.empty(t.numel() + 1, device=DEV)[1:].view(t.shape).copy_(t)
+    for which in range(3):
+        cache, out = Case.Cache(), torch.empty(case.tokens, 4 * 64, device=DEV)
+        cache.k, cache.v = case.kd, case.vd
+        if which == 0:
+            out = shifted(out)
+        elif which == 1:
+            cache.k = shifted(case.kd)
+        else:
+            cache.v = shifted(case.vd)
+        paged_attention(case.qd, case.qd.stride(0), out, cache, case.group, case.ctx, 4, 0.125, 0)
+        assert (out.cpu() - want).abs().max() <= 4e-6 * want.abs().max()
