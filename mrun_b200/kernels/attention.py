@@ -182,8 +182,8 @@ def prefill_tiles(ctx, tokens_per_tile: int, longer_than: int = 0, up_to: int = 
         found.sort(key=lambda tile: -tile[0])
         first, count = [tile[1] for tile in found], [tile[2] for tile in found]
         n = len(first)
-        both = ctx.upload(np.asarray(first + count, dtype=np.int32))
-        tiles = ctx.shared[key] = (both[:n], both[n:], n)
+        both = ctx.upload(np.asarray(first + count, dtype=np.int32)) if n else None
+        tiles = ctx.shared[key] = (both[:n], both[n:], n) if n else (None, None, 0)
     return tiles
 
 

@@ -31,7 +31,8 @@ of 760 and 1,140 tokens behind 700 and 350, 16 heads of 128 + 64, a latent of 51
 out of the pages, the rotated part they share goes beside every head's plain key, each segment's keys and
 values become one large page of scratch, and the paged kernels run over those.  Only while the contexts
 together are not much longer than the step (``EXPAND_ROWS`` times its rows), so that a long context is not
-projected up again for every portion of it; other steps, decode steps and the 32-bit path stay with the
+projected up again for every portion of it, and, with a rotated part or a query latent, only where the
+scores over the latents cost more (``_worth_making``); other steps, decode steps and the 32-bit path stay with the
 latent.
 
 Per step: one product for both down-projections (their weights stacked), one kernel that norms
@@ -125,15 +126,30 @@ class LatentAttention:
         self.expandable = (runtime.precision.act == torch.bfloat16 and s.window is None and s.vdim in (64, 128)
                            and s.dim + s.rot_dim in (64, 128, 192) and s.dim % 8 == 0 and s.rot_dim % 8 == 0
                            and (self.width > 128 or (s.rot_dim == 0 and not s.q_rank and s.dim in (64, 128))))
+        self.costly = bool(s.rot_dim or s.q_rank)
 
     def _scratch_rows(self, ctx) -> int:
         """Rows of the scratch pages of a step whose keys and values are made, 0 for a step that keeps the latent."""
         if not self.expandable or ctx.max_q_len == 1 or len(ctx.segments) > EXPAND_SEGMENTS:
             return 0
+        if self.costly and not self._worth_making(ctx):
+            return 0
         rows = 128
         while rows < ctx.max_kv_len:
             rows *= 2
         return rows if rows * len(ctx.segments) <= EXPAND_ROWS * max(128, ctx.num_tokens) else 0
+
+    def _worth_making(self, ctx) -> bool:
+        """Whether the step's scores over the latents cost more than keys and values made for them.  On B200, us a layer: the
+        kernel for wide rows takes 0.45 for 1,000 (token, key) pairs of 16 heads, the absorbed products 0.03 a token; made keys
+        and values cost the host two more products a segment and, once a step, two more uploads.  A layer's pass over a
+        planned step, made / latents: one request of 384 tokens 164 / 153, of 768 159 / 217, four of 128 316 / 188, four of
+        475 257 / 311.  A new step of a model of four such layers: one request of 512 tokens 1,576 / 1,372, of 768
+        1,608 / 1,469, of 1,024 1,631 / 1,910, two of 512 1,796 / 1,518, two of 768 1,847 / 2,242, four of 384
+        2,101 / 1,808, four of 500 2,124 / 2,323, eight of 250 2,583 / 1,957."""
+        groups = -(-self.spec.heads // 16)
+        pairs = sum(seg.q_len * (2 * seg.pos_start + seg.q_len + 1) // 2 for seg in ctx.segments)
+        return groups * (0.45e-3 * pairs + 0.03 * ctx.num_tokens) >= 100 + 31 * len(ctx.segments)
 
     def _expanded(self, q, ctx, cache, group, rows: int) -> torch.Tensor:
         """The heads' outputs over keys and values made from the contexts' latents: [tokens, heads * vdim].  ``q``
