@@ -5,7 +5,8 @@
 // side by side, RT rows a block, so the keys and values that it brings to shared memory serve all of
 // them (32 heads over 8 of 128, prompts of 207 and 310 tokens: 102 us; a block a token and head, which reads
 // the keys again for every row: 1,184).  Bound by the shared-memory reads that feed the FMA pipe, for
-// single tokens by the latency of one tile after the other (4.5 us a tile).
+// single tokens by the latency of one tile after the other (4.5 us a tile, so 590 us at a context of 8,000, whether
+// one request decodes or sixteen: a token and kv head's keys are not dealt to several blocks).
 //
 // Keys come in tiles of KT counted from position 0.  A thread owns RPT rows x 4 keys of the scores (keys tx,
 // tx + 16, ...) and the same rows x D / 16 columns of the output.  A score is one chain of fused
@@ -18,6 +19,8 @@
 // Math: s = scale * q·k, p = softmax(s), o = p·v; query head h reads kv head h / (heads/kv_heads)
 // (crates/mrun-engine/src/models/common.rs:129,199-205; causal alignment to the end of the keys,
 // crates/mrun-engine/src/tensor/nuvec.rs:866-872).
+#include <type_traits>
+
 #include "common.cuh"
 
 using namespace mrun;
@@ -117,24 +120,29 @@ attention_f32_kernel(const float* __restrict__ q, long q_stride, float* __restri
         for (int i = 0; i < RPT; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-        if (computes)
+        const int here = min(KT, last + 1 - tile);        // keys of the tile that there are
+        auto score = [&](auto columns) {
 #pragma unroll 4
-        for (int d = 0; d < D; d += 4) {
-            float4 a[RPT], b[4];
+            for (int d = 0; d < D; d += 4) {
+                float4 a[RPT], b[columns];
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * RPT + i) * PITCH + d);
+                for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty * RPT + i) * PITCH + d);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * PITCH + d);
+                for (int j = 0; j < columns; ++j) b[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * PITCH + d);
 #pragma unroll
-            for (int i = 0; i < RPT; ++i)
+                for (int i = 0; i < RPT; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
-                    s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
-                    s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
-                    s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
-                }
-        }
+                    for (int j = 0; j < columns; ++j) {
+                        s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+                        s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+                        s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+                        s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+                    }
+            }
+        };
+        // the first tokens of a request see a quarter of a tile
+        if (computes && here > 16) score(std::integral_constant<int, 4>());
+        else if (computes) score(std::integral_constant<int, 1>());
         __syncthreads();                  // the keys have been read, the next ones looked up
         if (tile + KT <= last) bring(k_cache, ks, PITCH, which ^ 1);
         copies_commit();
@@ -173,7 +181,7 @@ attention_f32_kernel(const float* __restrict__ q, long q_stride, float* __restri
         __syncthreads();
         if (computes)
 #pragma unroll 2
-        for (int j = 0; j < KT; j += 4) {
+        for (int j = 0; j < here; j += 4) {
             float p[RPT][4];
 #pragma unroll
             for (int i = 0; i < RPT; ++i)

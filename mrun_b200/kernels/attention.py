@@ -255,7 +255,7 @@ def latent_wide_ok(dtype: torch.dtype, width: int, value_dim: int) -> bool:
     return dtype == torch.bfloat16 and bool(_lib.core()._dll.mrun_latent_attention_wide_ok(_c_int(width), _c_int(value_dim)))
 
 
-F32_TILE_ROWS = 64       # token rows x group heads of a tile of the 32-bit attention
+F32_TILE_ROWS = (64, 16, 4)     # token rows x group heads of the tiles of the 32-bit attention
 F32_TILE_GROUP = 16      # query heads a kv head that it takes
 
 
@@ -270,6 +270,21 @@ def f32_tiles_ok(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, ratio
             and q_stride % 4 == 0 and not any(t.data_ptr() % 16 for t in (q, out, cache.k, cache.v)))
 
 
+def f32_tile_rows(ctx, ratio: int, kv_heads: int, sms: int) -> int:
+    """Rows (token x group head) of a tile of the 32-bit attention in a step with prompt portions: the fewest with which
+    the step's blocks are at most two a multiprocessor, since a block's time grows with its rows (a tile of 64 keys of
+    128 features takes 4.6 / 6.6 / 11.5 us at 4 / 16 / 64 rows) and the device's does not while blocks fit it.
+    A token's bits are the same whichever.  B200, us at 64 / 16 / 4 rows (blocks): 32 heads over 8 of 128 behind 2,000
+    tokens, 33 new ones 383 (24) / 203 (72) / 176 (264), 100 new ones 376 (56) / 343 (200) / 392 (800); 12 heads
+    over 4 of 64, 400 new ones 349 (80) / 311 (320) / 548 (1,600)."""
+    rows = F32_TILE_ROWS[0]
+    for fewer in F32_TILE_ROWS[1:]:
+        per_tile = fewer // ratio
+        if per_tile and kv_heads * sum(-(-seg.q_len // per_tile) for seg in ctx.segments) <= 2 * sms:
+            rows = fewer
+    return rows
+
+
 def _paged_attention_f32(q, q_stride: int, out, cache, group, ctx, heads: int, scale: float, window: int) -> torch.Tensor:
     def launch(first, count, tiles: int, tile_tokens: int):
         ops.paged_attention_f32(q, q_stride, out, cache.k, cache.v, group.block_tables, ctx.token_slot, ctx.positions, first, count,
@@ -279,8 +294,16 @@ def _paged_attention_f32(q, q_stride: int, out, cache, group, ctx, heads: int, s
         return out
     if ctx.num_tokens > ctx.real_tokens:
         out[ctx.real_tokens:].zero_()
-    tokens = F32_TILE_ROWS // (heads // cache.k.shape[1])
-    for per_tile, longer_than, up_to in ((tokens, 1, 1 << 30), (1, 0, 1)):        # prompt portions; single tokens beside them
+    kv_heads = cache.k.shape[1]
+    ratio = heads // kv_heads
+    rows = f32_tile_rows(ctx, ratio, kv_heads, ops.sm_count(q.device))
+    tokens = max(1, rows // ratio)
+    # Single tokens beside portions in small tiles go in the same launch (a portion of 5 behind 300 tokens beside single
+    # tokens at 100 and 200, 32 heads over 8 of 128: 25 us, two launches 47), unless its tiles are larger than the ones they
+    # would have alone and their contexts are what the step waits for.
+    longest = max((seg.pos_start + seg.q_len for seg in ctx.segments if seg.q_len > 1), default=0)
+    together = rows < F32_TILE_ROWS[0] and (rows == F32_TILE_ROWS[-1] or ratio > F32_TILE_ROWS[-1] or 2 * longest >= ctx.max_kv_len)
+    for per_tile, longer_than, up_to in [(tokens, 0, 1 << 30)] if together else [(tokens, 1, 1 << 30), (1, 0, 1)]:
         first, count, n = prefill_tiles(ctx, per_tile, longer_than, up_to)
         if n:
             launch(first, count, n, per_tile)

@@ -112,3 +112,22 @@ def test_tiled_attention_leaves_unaligned_outputs_to_the_general_kernel():
             cache.v = shifted(case.vd)
         paged_attention(case.qd, case.qd.stride(0), out, cache, case.group, case.ctx, 4, 0.125, 0)
         assert (out.cpu() - want).abs().max() <= 4e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(8, 8, 64, 32), (32, 8, 128, 16), (32, 2, 64, 16), (16, 1, 128, 4),
+                                                               (6, 2, 128, 1), (9, 3, 64, 8), (10, 2, 128, 16)])
+@pytest.mark.parametrize("window", [0, 37])
+def test_tiles_of_every_size_give_the_same_bits(heads, kv_heads, head_dim, page_size, window, monkeypatch):
+    """Portions and single tokens, contexts within and beyond the first quarter of a tile, in tiles of 64, 16 and 4 rows."""
+    from mrun_b200.kernels import attention
+    segments = [(0, 70), (129, 1), (63, 2), (300, 1), (15, 33), (0, 1), (0, 17), (9, 1), (64, 64)]
+    scale = head_dim ** -0.5
+    case = Case(segments, heads, kv_heads, head_dim, page_size, torch.float32, seed=head_dim + window, window=window)
+    want = case.reference(scale)
+    results = []
+    for rows in attention.F32_TILE_ROWS:
+        case.ctx.shared.clear()
+        monkeypatch.setattr(attention, "f32_tile_rows", lambda *a: rows)
+        results.append(case.run(scale))
+    assert (results[0] - want).abs().max() <= 2e-5 * want.abs().max()
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])

@@ -1,4 +1,5 @@
-"""Which steps the scans take in chunks and which they walk, on both sides of the lines between them."""
+"""Which steps the scans take in chunks and which they walk, and which tiles the 32-bit attention takes, on both sides of the
+lines between them."""
 from __future__ import annotations
 
 from types import SimpleNamespace
@@ -28,3 +29,11 @@ def test_a_step_is_walked_where_the_walk_is_the_faster_form(kind, dim, vdim, hea
     tokens = sum(lengths)
     least = ops._chunk_least(ctx, tokens, kind == "delta", heads, dim, vdim)
     assert bool(ops._chunks(ctx, tokens, least)) == chunked
+
+
+@pytest.mark.parametrize("ratio, kv_heads, portions, rows", [(4, 8, [2], 4), (4, 8, [17, 1, 1], 4), (4, 8, [33], 4), (4, 8, [100], 16),
+                                                             (4, 8, [207, 310], 64), (16, 1, [2], 16), (8, 1, [150], 16), (3, 4, [400], 64), (3, 4, [300], 16)])
+def test_tiles_of_the_32_bit_attention_follow_the_blocks_they_make(ratio, kv_heads, portions, rows):
+    from mrun_b200.kernels.attention import f32_tile_rows
+    ctx = SimpleNamespace(segments=[SimpleNamespace(q_len=n) for n in portions])
+    assert f32_tile_rows(ctx, ratio, kv_heads, 148) == rows
