@@ -41,18 +41,22 @@ def test_keys_and_values_made_from_latents(name, expand, monkeypatch):
 @pytest.mark.parametrize("pairing", ["interleaved", "half"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rotation_in_place(pairing, dtype):
-    """The same bits as the rotation into query rows, in strided rows, nothing else touched."""
+    """Within the roundings of one product sum of the rotation in 64 bits, in strided rows, nothing else touched."""
     from mrun_b200.kernels import ops
     heads, dim, rot_dim, rot_dims = 3, 10, 12, 8
     wide = torch.randn(9, heads * (dim + rot_dim) + 5, device=DEV).to(dtype)
     q = wide[:, :heads * (dim + rot_dim)]
     rot = torch.randn(9, rot_dims // 2, 2, device=DEV)
-    rows = torch.empty(9, heads, 4 + rot_dim, dtype=dtype, device=DEV)
-    ops.latent_query(q, rot, rot_dims, pairing, rows, heads, dim, rot_dim, 4)
-    want = wide.clone()
-    want[:, :heads * (dim + rot_dim)].unflatten(1, (heads, -1))[:, :, dim:] = rows[:, :, 4:]
+    part = q.double().unflatten(1, (heads, -1))[:, :, dim:dim + rot_dims]
+    lanes = (slice(0, None, 2), slice(1, None, 2)) if pairing == "interleaved" else (slice(0, rot_dims // 2), slice(rot_dims // 2, None))
+    x, y, c, s = part[:, :, lanes[0]], part[:, :, lanes[1]], rot[:, None, :, 0].double(), rot[:, None, :, 1].double()
+    before = wide.clone()
     ops.latent_rotate(q, rot, rot_dims, pairing, heads, dim, rot_dim)
-    assert (wide.float() - want.float()).abs().max() <= (1e-6 if dtype == torch.float32 else 0.04)     # one rounding apart at most
+    got = q.double().unflatten(1, (heads, -1))[:, :, dim:dim + rot_dims]
+    # two products and a sum in 32 bits (24 significant bits: 2^-24 of a value each), then the result in bfloat16 (8: 2^-8)
+    unit = 3 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    for lane, want, size in ((lanes[0], x * c - y * s, (x * c).abs() + (y * s).abs()), (lanes[1], y * c + x * s, (y * c).abs() + (x * s).abs())):
+        assert ((got[:, :, lane] - want).abs() <= unit * size).all()
     keep = torch.ones_like(wide, dtype=torch.bool)
     keep[:, :heads * (dim + rot_dim)].unflatten(1, (heads, -1))[:, :, dim:dim + rot_dims] = False
-    assert torch.equal(wide[keep], want[keep])
+    assert torch.equal(wide[keep], before[keep])

@@ -199,7 +199,7 @@ def test_rows_without_a_chunked_form_are_walked(monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("groups, n", [(3, 8), (5, 64), (2, 72), (7, 128), (3, 136), (2, 1016), (1, 1024), (2, 8192), (1, 8200)])
+@pytest.mark.parametrize("groups, n", [(3, 8), (5, 64), (2, 72), (7, 128), (3, 136), (2, 256), (5, 264), (2, 1016), (1, 1024), (2, 8192), (1, 8200)])
 @pytest.mark.parametrize("shared", [False, True])
 def test_gated_norm_in_pieces(dtype, groups, n, shared):
     """Group sizes on both sides of every number of threads, weights a group or a row long, strided gates and outputs."""
@@ -268,3 +268,36 @@ def test_declared_scratch_is_the_kernels():
                               ops._ptr(like), ops._ptr(like), ops._ptr(like), ops._ptr(like), ops._c_int(1), ops._c_int(1), ops._c_int(dim),
                               ops._c_int(vdim))
                 assert ops.chunk_scratch_elements(dim, vdim, delta) == -(-5 * 2 * floats // (4 * ops.CHUNK))
+
+
+@pytest.mark.parametrize("kind", ["decay", "gated", "delta"])
+def test_a_short_segment_beside_a_long_one(kind, record_property):
+    """A step is walked or goes in chunks as a whole, so a short segment's outputs and its state move beside a long one: in
+    the rounding of 32-bit sums only."""
+    from mrun_b200.kernels import ops
+    heads, dim, vdim, short = 16, 128, 128, 16
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    y = torch.randn(short + 512, heads * (2 * dim + vdim), generator=gen, device=DEV).bfloat16()
+    a, bias = torch.randn(short + 512, heads * dim, generator=gen, device=DEV), torch.full((heads * dim,), 1.0, device=DEV)
+    b = torch.randn(short + 512, heads, generator=gen, device=DEV).bfloat16()
+    rate, decay = torch.full((heads,), -2.0, device=DEV), torch.full((heads,), 0.95, device=DEV)
+    start = torch.randn(7, heads, dim, vdim, generator=gen, device=DEV)
+    results = []
+    for lengths in ([short], [short, 512]):
+        ctx, n = context(lengths, 7), sum(lengths)
+        least = ops._chunk_least(ctx, n, kind == "delta", heads, dim, vdim)
+        assert bool(ops._chunks(ctx, n, least)) == (len(lengths) == 2)
+        q, k, v = y[:n, :heads * dim], y[:n, heads * dim:2 * heads * dim], y[:n, 2 * heads * dim:]
+        state = start.clone()
+        if kind == "decay":
+            out = ops.decay_scan(q, k, v, decay, state, ctx, heads, dim, vdim, True)
+        elif kind == "gated":
+            out = ops.gated_scan(q, k, v, a[:n], bias, 8.0, state, ctx, heads, dim, vdim)
+        else:
+            out = ops.delta_scan(q, k, v, a[:n], b[:n], rate, bias, state, ctx, heads, heads, dim, vdim)
+        results.append((out[:short], state[ctx.seg_slot[0]]))
+    for name, alone, beside in zip(("outputs", "state"), *results):
+        moved = float((beside - alone).norm() / alone.norm())
+        record_property(f"{kind} {name}", moved)
+        print(f"{kind}: a short segment's {name} move by {moved:.2e} beside a long one")
+        assert moved <= 5e-6
