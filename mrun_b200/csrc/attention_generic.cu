@@ -1,6 +1,6 @@
 // Paged grouped-query attention on CUDA cores in 32-bit arithmetic, for any head size.
 //
-// This is the attention of the whole-model 32-bit path, and the kernel that takes the shapes the
+// This is the kernel of the 32-bit path for the shapes that attention_f32.cu does not take, and for the shapes the
 // tensor-core kernels refuse.  One block per (token, query head).  A token at position p of its
 // request sees keys lo..p, lo = 0, p - window + 1, or the start of p's chunk for a window of minus
 // the chunk's size (first_visible()), read from the request's pages; the keys of

@@ -5,8 +5,9 @@
 // the flat batch, state slot seg_slot[s]); a segment of zero rows is padding.  Every kernel reads
 // the state its request left, walks the segment's tokens in order and leaves the state for the
 // next step, so a token's result does not depend on how the request was cut into steps or on the
-// requests beside it (recurrent_chunk.cu takes long bfloat16 segments of some scans in chunks instead,
-// whose sums are ordered by the chunks).  States and all arithmetic of the recurrences are 32-bit.
+// requests beside it.  (recurrent_chunk.cu takes bfloat16 steps with long segments of some scans in chunks instead:
+// its sums are ordered by the chunks, and whether a step goes there is decided by all of its segments, so a result then
+// moves in rounding with the cut and with the requests beside it.)  States and all arithmetic of the recurrences are 32-bit.
 //
 // Kernels:
 //   causal_conv     y_t = sum_j w[:, j] x_(t - taps + 1 + j) per channel (the last tap meets the
@@ -504,8 +505,8 @@ gated_norm_vec_kernel(const float* __restrict__ o, const float* __restrict__ w, 
         if (in && lane + i * LANES < pieces) {
             Vec8<float>::load(row + (lane + i * LANES) * 8, y[i]);
             Vec8<TA>::load(grow + (lane + i * LANES) * 8, gv[i]);
-        }
             if constexpr (PIECES == 1) Vec8<float>::load(wrow + lane * 8, first);
+        }
 #pragma unroll
     for (int i = 0; i < PIECES; ++i)
         if (in && lane + i * LANES < pieces)

@@ -14,7 +14,7 @@ the fused norm/rotary/cache kernel just before.
   into a ring for those head and page sizes, else copied with cp.async.
 * bfloat16 otherwise: a step with prompt portions.  Its single-token segments (the decoding
   requests beside the prompts) go through the TMA decode kernel as a selection of the step's rows
-  where that kernel takes the shape; the rest as follows.  Head sizes 64 and 128: the tcgen05 kernel (128-row tiles
+  where that kernel takes the shape; the rest as follows.  Head sizes 64 and 128, and keys of 192: the tcgen05 kernel (128-row tiles
   of tokens x group heads, accumulators in tensor memory) for every segment with more rows than
   one tile of the older kernel; the mma.sync kernel (64-row tiles) for the rest of the step (the
   single decode tokens of a mixed step, short tails) and for the other head sizes.
@@ -275,8 +275,8 @@ def f32_tile_rows(ctx, ratio: int, kv_heads: int, sms: int) -> int:
     the step's blocks are at most two a multiprocessor, since a block's time grows with its rows (a tile of 64 keys of
     128 features takes 4.6 / 6.6 / 11.5 us at 4 / 16 / 64 rows) and the device's does not while blocks fit it.
     A token's bits are the same whichever.  B200, us at 64 / 16 / 4 rows (blocks): 32 heads over 8 of 128 behind 2,000
-    tokens, 33 new ones 383 (24) / 203 (72) / 176 (264), 100 new ones 376 (56) / 343 (200) / 392 (800); 12 heads
-    over 4 of 64, 400 new ones 349 (80) / 311 (320) / 548 (1,600)."""
+    tokens, 2 new ones 361 (8) / 201 (8) / 142 (16), 33 new ones 384 (24) / 205 (72) / 165 (264), 100 new ones
+    378 (56) / 343 (200) / 374 (800); 12 heads over 4 of 64, 400 new ones 348 (80) / 311 (320) / 563 (1,600)."""
     rows = F32_TILE_ROWS[0]
     for fewer in F32_TILE_ROWS[1:]:
         per_tile = fewer // ratio
@@ -441,7 +441,8 @@ _tc5_prefill = {}
 
 
 def prefill_uses_tcgen05(library, ratio: int, page_size: int) -> bool:
-    """Head sizes 64 and 128, pages of a power-of-two size (the kernel copies whole pages by TMA)."""
+    """Head sizes 64 and 128 and keys of 192 with such values, pages of a power-of-two size (the kernel copies
+    whole pages by TMA)."""
     if not TC5_PREFILL or ratio > 128 or page_size & (page_size - 1):
         return False
     have = _tc5_prefill.get(library.path)
