@@ -673,10 +673,12 @@ def linear_into_norm(pending: PendingLinear, resid: torch.Tensor, weight: torch.
 
 
 def gemm_f32_nt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x @ w.T in IEEE 32-bit with a fixed summation order.  x may have a row stride."""
+    """y = x @ w.T in 32-bit with a fixed summation order, whatever the number of rows.  x may have a row stride."""
     _check(x, "x", torch.float32, dense=False); _check(w, "w", torch.float32)
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.stride(1) != 1:
         raise KernelError(f"gemm_f32_nt: x {tuple(x.shape)} (strides {x.stride()}) vs w {tuple(w.shape)}")
+    if f32_tc_ok(w):
+        return gemm_f32_tc(x, w, out)
     m, k = x.shape
     n = w.shape[0]
     if out is None:
@@ -686,6 +688,48 @@ def gemm_f32_nt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
         raise KernelError(f"gemm_f32_nt: out is {tuple(out.shape)}, expected {(m, n)}")
     _lib.core().call("mrun_gemm_f32_nt", _ptr(x), _ptr(w), _ptr(out), _c_int(m), _c_int(n), _c_int(k),
                      _c_long(x.stride(0) if m > 1 else k), _c_long(n), _stream())
+    return out
+
+
+F32_TC_SCRATCH = 128 << 20       # bytes of a product's split rows at most: longer ones go in portions
+F32_TC_MIN_K = 2048
+F32_TC_MIN_N = 64
+
+
+def f32_tc_ok(w: torch.Tensor) -> bool:
+    """Whether 32-bit products with ``w`` go to the tensor cores.  Decided by w alone, so that a row's bits do not depend on
+    the rows beside it.  From K = 2,048 on they are faster for any number of rows (B200, us, this / the chain of
+    multiply-adds: 1 row of 2,048 x 2,048 10.5 / 10.8, 17 rows 12.7 / 41; 1 row of 128 x 4,096 10.3 / 19; 517 rows of 24,576 x 4,096
+    429 / 2,233) and closer to 64 bits (3.4e-7 / 1.1e-6 at K = 4,096); at K = 1,024 a few rows take longer (8.2 / 6.0), and at
+    K = 256 both are equally close (2.9e-7)."""
+    n, k = w.shape
+    return k >= F32_TC_MIN_K and n >= F32_TC_MIN_N and k % 4 == 0 and w.data_ptr() % 16 == 0
+
+
+def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, ranges: int = 0, tile: int = 0,
+                cluster: int = 0) -> torch.Tensor:
+    """:func:`gemm_f32_nt` on the tensor cores, every operand as the sum of three bfloat16 values (``csrc/gemm_f32_tc.cu``).
+    ``ranges`` of k, ``tile`` tokens a block, ``cluster`` blocks a tile; 0: chosen, the ranges by the sizes of ``w`` alone."""
+    _check(x, "x", torch.float32, dense=False); _check(w, "w", torch.float32)
+    if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.stride(1) != 1:
+        raise KernelError(f"gemm_f32_tc: x {tuple(x.shape)} (strides {x.stride()}) vs w {tuple(w.shape)}")
+    m, k = x.shape
+    n = w.shape[0]
+    if out is None:
+        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    _check(out, "out", torch.float32)
+    if out.shape != (m, n):
+        raise KernelError(f"gemm_f32_tc: out is {tuple(out.shape)}, expected {(m, n)}")
+    pitch = -(-k // 8) * 8
+    rows = max(1, min(m, F32_TC_SCRATCH // (6 * pitch)))
+    parts = torch.empty(3 * rows * pitch, dtype=torch.bfloat16, device=x.device)
+    status = status_word(x.device, "gemm_f32_tc", {1: "the copies of w", 2: "the copies of x", 3: "the conversion of w",
+                                                   4: "the MMA issuer", 5: "the sums"})
+    for at in range(0, m, rows):
+        part, to = x[at:at + rows], out[at:at + rows]
+        _lib.core().call("mrun_gemm_f32_tc", _ptr(part), _ptr(w), _ptr(to), _ptr(parts), _c_int(part.shape[0]), _c_int(n), _c_int(k),
+                         _c_long(x.stride(0) if m > 1 else k), _c_long(n), _c_int(ranges), _c_int(tile), _c_int(cluster), _ptr(status),
+                         _stream())
     return out
 
 
@@ -770,7 +814,7 @@ def tc5_check(device: Optional[torch.device] = None) -> None:
 
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x @ w.T (+ bias).  float32: this library's own IEEE kernel.  bfloat16 with at most 16
+    """y = x @ w.T (+ bias).  float32: this library's own kernels.  bfloat16 with at most 16
     rows (decode): this library's weight-streaming tensor-core kernel (``x`` may then be
     :class:`NormedRows`).  bfloat16 otherwise (prefill): the vendor GEMM library with 32-bit
     accumulation (the reference calls its array library's matmul for the same products and adds
