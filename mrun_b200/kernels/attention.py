@@ -44,7 +44,7 @@ def _decode_slots(library, tma_group: int = 0) -> int:
     slots = _slots.get((library.path, tma_group))
     if slots is None:
         if tma_group:
-            per_sm = max(1, int(library._dll.mrun_attn_decode_tma_occupancy(_c_int(tma_group))))
+            per_sm = max(1, int(library._dll.mrun_attn_decode_tma_occupancy(tma_group)))
         else:
             query = library._dll.mrun_attn_decode_occupancy
             query.restype = ctypes.c_int
@@ -153,10 +153,10 @@ def decode_plan(ctx, library, window: int, kv_heads: int, blocks: int, splits: i
         if positions is None:
             positions = ctx.positions
         n = positions.shape[0]
-        prefix = torch.empty(2 * (n + 1) + 1, dtype=torch.int32, device=positions.device)
-        assignment = torch.empty(blocks * 8, dtype=torch.int32, device=positions.device)
-        library.call("mrun_attn_decode_plan", _ptr(positions), _c_int(n), _c_int(window),
-                     _c_int(kv_heads), _c_int(blocks), _c_int(MIN_TILES), _c_int(splits), _ptr(prefix),
+        prefix = positions.new_empty(2 * (n + 1) + 1, dtype=torch.int32)
+        assignment = positions.new_empty(blocks * 8, dtype=torch.int32)
+        library.call("mrun_attn_decode_plan", _ptr(positions), n, window,
+                     kv_heads, blocks, MIN_TILES, splits, _ptr(prefix),
                      _ptr(assignment), _stream())
         plan = ctx.shared[key] = (prefix, assignment)
     return plan
@@ -252,7 +252,7 @@ LATENT_WIDE_MAX_SPLITS = 32     # the most blocks one token's keys are dealt to 
 def latent_wide_ok(dtype: torch.dtype, width: int, value_dim: int) -> bool:
     """Whether the tensor-core kernel for wide latent rows takes this shape (bfloat16, rows of a
     multiple of 16 features, at most 512 value columns)."""
-    return dtype == torch.bfloat16 and bool(_lib.core()._dll.mrun_latent_attention_wide_ok(_c_int(width), _c_int(value_dim)))
+    return dtype == torch.bfloat16 and bool(_lib.core()._dll.mrun_latent_attention_wide_ok(width, value_dim))
 
 
 F32_TILE_ROWS = (64, 16, 4)     # token rows x group heads of the tiles of the 32-bit attention
@@ -340,13 +340,13 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         splits = max(1, min(LATENT_WIDE_MAX_SPLITS, 2 * ops.sm_count(q.device) // blocks, -(-ctx.max_kv_len // 128)))
         part_o = part_ml = None
         if splits > 1:
-            cols = int(_lib.core()._dll.mrun_latent_attention_wide_piece_cols(_c_int(value_dim)))
-            part_o = torch.empty((blocks * splits, 16, cols), dtype=torch.float32, device=q.device)
-            part_ml = torch.empty((blocks * splits, 16, 2), dtype=torch.float32, device=q.device)
-        _lib.core().call("mrun_latent_attention_wide", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(cache.k),
-                         _ptr(group.block_tables), _c_int(group.max_blocks), _ptr(ctx.token_slot), _ptr(ctx.positions),
-                         _c_int(ctx.num_tokens), _c_int(heads), _c_int(head_dim), _c_int(value_dim), _c_int(page_size),
-                         _c_long(pages * page_size), _c_float(scale), _c_int(splits), _ptr(part_o), _ptr(part_ml),
+            cols = int(_lib.core()._dll.mrun_latent_attention_wide_piece_cols(value_dim))
+            part_o = q.new_empty((blocks * splits, 16, cols), dtype=torch.float32)
+            part_ml = q.new_empty((blocks * splits, 16, 2), dtype=torch.float32)
+        _lib.core().call("mrun_latent_attention_wide", _ptr(q), q_stride, _ptr(out), _ptr(cache.k),
+                         _ptr(group.block_tables), group.max_blocks, _ptr(ctx.token_slot), _ptr(ctx.positions),
+                         ctx.num_tokens, heads, head_dim, value_dim, page_size,
+                         pages * page_size, scale, splits, _ptr(part_o), _ptr(part_ml),
                          _stream())
         return out
     if sink is None and form is None and f32_tiles_ok(q, q_stride, out, cache, ratio):
@@ -356,36 +356,36 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
                                            ctx.token_slot, ctx.positions, heads, scale, window, sink=sink, form=form)
     library = _lib.attention(head_dim, v_dim, form is not None)
     tokens = ctx.num_tokens
-    common = (_ptr(cache.k), _ptr(cache.v), _ptr(group.block_tables), _c_int(group.max_blocks),
+    common = (_ptr(cache.k), _ptr(cache.v), _ptr(group.block_tables), group.max_blocks,
               _ptr(ctx.token_slot), _ptr(ctx.positions))
-    tail = (_c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page_size), _c_float(scale),
-            _c_int(window), _ptr(sink), _stream())
+    tail = (heads, kv_heads, head_dim, page_size, scale,
+            window, _ptr(sink), _stream())
     if ctx.all_decode and ratio <= 16:
         if tokens * kv_heads > COUNTER_CAPACITY:
             raise ValueError(f"a decode step of {tokens} tokens x {kv_heads} kv heads exceeds {COUNTER_CAPACITY} pairs")
-        fused = (_c_int(0), _ptr(None), _ptr(None), _c_float(0.0), _ptr(None), _c_int(0), _ptr(None))
+        fused = (0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None))
         if raw is not None:
             q_weight, k_weight, eps, rot, rotary_dim, slots = raw
-            fused = (_c_int(1), _ptr(q_weight), _ptr(k_weight), _c_float(eps), _ptr(rot), _c_int(rotary_dim),
+            fused = (1, _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot), rotary_dim,
                      _ptr(slots))
         cluster = decode_cluster(library, ratio, page_size, tokens, kv_heads, ctx.max_kv_len)
         if cluster:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_cluster", _ptr(q), _c_long(q_stride), _ptr(out), *common, _c_int(tokens),
-                         _c_int(cluster), *tail[:-1], *fused, _ptr(None), _c_long(pages), formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_decode_cluster", _ptr(q), q_stride, _ptr(out), *common, tokens,
+                         cluster, *tail[:-1], *fused, _ptr(None), pages, formed, _ptr(status), tail[-1])
             return out
         tma = decode_uses_tma(library, ratio, page_size)
         blocks, splits = decode_launch(tokens, kv_heads, decode_slots(library, ratio, page_size))
-        part_o = torch.empty((blocks, 2, 16, v_dim), dtype=torch.float32, device=q.device)
-        part_ml = torch.empty((blocks, 2, 16, 2), dtype=torch.float32, device=q.device)
+        part_o = q.new_empty((blocks, 2, 16, v_dim), dtype=torch.float32)
+        part_ml = q.new_empty((blocks, 2, 16, 2), dtype=torch.float32)
         prefix, assignment = decode_plan(ctx, library, window, kv_heads, blocks, splits)
         extra = (formed,)
         if tma:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            extra = (_ptr(None), _c_long(pages), formed, _ptr(status))
-        library.call("mrun_attn_decode_tma" if tma else "mrun_attn_decode", _ptr(q), _c_long(q_stride), _ptr(out),
-                     *common, _ptr(prefix), _ptr(assignment), _c_int(tokens), _ptr(part_o), _ptr(part_ml),
-                     _ptr(_split_counters(q.device)), _c_int(blocks), *tail[:-1], *fused, *extra, tail[-1])
+            extra = (_ptr(None), pages, formed, _ptr(status))
+        library.call("mrun_attn_decode_tma" if tma else "mrun_attn_decode", _ptr(q), q_stride, _ptr(out),
+                     *common, _ptr(prefix), _ptr(assignment), tokens, _ptr(part_o), _ptr(part_ml),
+                     _ptr(_split_counters(q.device)), blocks, *tail[:-1], *fused, *extra, tail[-1])
         return out
     if raw is not None:
         raise ValueError("raw q, k, v rows are taken by the decode kernel only")
@@ -399,24 +399,24 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         cluster = decode_cluster(library, ratio, page_size, n_single, kv_heads, ctx.max_kv_len) if n_single else 0
         if cluster:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_cluster", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(cache.k), _ptr(cache.v),
-                         _ptr(group.block_tables), _c_int(group.max_blocks), _ptr(row_slots), _ptr(row_positions),
-                         _c_int(n_single), _c_int(cluster), *tail[:-1],
-                         _c_int(0), _ptr(None), _ptr(None), _c_float(0.0), _ptr(None), _c_int(0), _ptr(None),
-                         _ptr(rows), _c_long(pages), formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_decode_cluster", _ptr(q), q_stride, _ptr(out), _ptr(cache.k), _ptr(cache.v),
+                         _ptr(group.block_tables), group.max_blocks, _ptr(row_slots), _ptr(row_positions),
+                         n_single, cluster, *tail[:-1],
+                         0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None),
+                         _ptr(rows), pages, formed, _ptr(status), tail[-1])
             shortest = 1
         elif n_single and n_single * kv_heads <= COUNTER_CAPACITY:
             blocks, splits = decode_launch(n_single, kv_heads, decode_slots(library, ratio, page_size))
-            part_o = torch.empty((blocks, 2, 16, v_dim), dtype=torch.float32, device=q.device)
-            part_ml = torch.empty((blocks, 2, 16, 2), dtype=torch.float32, device=q.device)
+            part_o = q.new_empty((blocks, 2, 16, v_dim), dtype=torch.float32)
+            part_ml = q.new_empty((blocks, 2, 16, 2), dtype=torch.float32)
             prefix, assignment = decode_plan(ctx, library, window, kv_heads, blocks, splits, positions=row_positions)
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_tma", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(cache.k), _ptr(cache.v),
-                         _ptr(group.block_tables), _c_int(group.max_blocks), _ptr(row_slots), _ptr(row_positions),
-                         _ptr(prefix), _ptr(assignment), _c_int(n_single), _ptr(part_o), _ptr(part_ml),
-                         _ptr(_split_counters(q.device)), _c_int(blocks), *tail[:-1],
-                         _c_int(0), _ptr(None), _ptr(None), _c_float(0.0), _ptr(None), _c_int(0), _ptr(None),
-                         _ptr(rows), _c_long(pages), formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_decode_tma", _ptr(q), q_stride, _ptr(out), _ptr(cache.k), _ptr(cache.v),
+                         _ptr(group.block_tables), group.max_blocks, _ptr(row_slots), _ptr(row_positions),
+                         _ptr(prefix), _ptr(assignment), n_single, _ptr(part_o), _ptr(part_ml),
+                         _ptr(_split_counters(q.device)), blocks, *tail[:-1],
+                         0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None),
+                         _ptr(rows), pages, formed, _ptr(status), tail[-1])
             shortest = 1
     short_up_to = 1 << 30
     if prefill_uses_tcgen05(library, ratio, page_size):
@@ -426,13 +426,13 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         if n_tiles:
             status = ops.status_word(q.device, "attn_prefill_tc5",
                                      {1: "a key/value loader", 2: "the MMA issuer", 3: "the softmax warps"})
-            library.call("mrun_attn_prefill_tc5", _ptr(q), _c_long(q_stride), _ptr(out), *common, _ptr(first),
-                         _ptr(count), _c_int(n_tiles), *tail[:-1], _c_long(pages), formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_prefill_tc5", _ptr(q), q_stride, _ptr(out), *common, _ptr(first),
+                         _ptr(count), n_tiles, *tail[:-1], pages, formed, _ptr(status), tail[-1])
     if short_up_to > shortest:
         first, count, n_tiles = prefill_tiles(ctx, 64 // ratio, longer_than=shortest, up_to=short_up_to)
         if n_tiles:
-            library.call("mrun_attn_prefill", _ptr(q), _c_long(q_stride), _ptr(out), *common, _ptr(first),
-                         _ptr(count), _c_int(n_tiles), *tail[:-1], formed, tail[-1])
+            library.call("mrun_attn_prefill", _ptr(q), q_stride, _ptr(out), *common, _ptr(first),
+                         _ptr(count), n_tiles, *tail[:-1], formed, tail[-1])
     return out
 
 

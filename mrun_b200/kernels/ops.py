@@ -13,7 +13,7 @@ from . import lib as _lib
 from .lib import KernelError
 
 F32, BF16 = 0, 1
-_c_void_p, _c_int, _c_long, _c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_long, ctypes.c_float
+_c_int, _c_long, _c_float = ctypes.c_int, ctypes.c_long, ctypes.c_float
 
 
 def dtype_code(dtype: torch.dtype) -> int:
@@ -24,14 +24,14 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise KernelError(f"dtype {dtype} has no kernel (float32 and bfloat16 do)")
 
 
-def _stream() -> ctypes.c_void_p:
+def _stream() -> int:
     """The current stream of the current device.  Asked for by its raw handle: a Stream object took 29 % of an
     uncaptured step's host time (a mixer's decode step of five kernels on B200: 119 us a pass, 96 without)."""
-    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return _c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
 
 
 def _check(t: torch.Tensor, name: str, dtype: Optional[torch.dtype] = None, dense: bool = True) -> None:
@@ -51,7 +51,7 @@ def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor) -> torch.Te
     if out.shape != (tokens, hidden):
         raise KernelError(f"embed: out is {tuple(out.shape)}, expected {(tokens, hidden)}")
     _lib.core().call("mrun_embed", _ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out),
-                     _c_int(tokens), _c_int(hidden), _c_int(vocab), _stream())
+                     tokens, hidden, vocab, _stream())
     return out
 
 
@@ -79,7 +79,7 @@ def add_rmsnorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: torc
         raise KernelError(f"add_rmsnorm: weight {tuple(weight.shape)}, out {tuple(out.shape)}, "
                           f"expected hidden {hidden}, rows {n_rows}")
     _lib.core().call("mrun_add_rmsnorm", _ptr(resid), _ptr(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
-                     _ptr(weight), _c_float(eps), _ptr(out), dtype_code(out.dtype), _ptr(rows), _c_int(n_rows), _c_int(hidden),
+                     _ptr(weight), eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden,
                      _ptr(extra), _ptr(share), _stream())
     return out
 
@@ -90,7 +90,7 @@ def add_scaled_rows(y: torch.Tensor, x: torch.Tensor, share: torch.Tensor) -> to
     if y.dim() != 2 or x.shape != y.shape or share.numel() != y.shape[0]:
         raise KernelError(f"add_scaled_rows: y {tuple(y.shape)}, x {tuple(x.shape)}, share {tuple(share.shape)}")
     _lib.core().call("mrun_add_scaled_rows", _ptr(y), dtype_code(y.dtype), _ptr(x), dtype_code(x.dtype), _ptr(share),
-                     _c_int(y.shape[0]), _c_int(y.shape[1]), _stream())
+                     y.shape[0], y.shape[1], _stream())
     return y
 
 
@@ -118,8 +118,8 @@ def add_layernorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: to
         raise KernelError(f"add_layernorm: weight {tuple(weight.shape)}, out {tuple(out.shape)}, "
                           f"expected hidden {hidden}, rows {n_rows}")
     _lib.core().call("mrun_add_layernorm", _ptr(resid), _ptr(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
-                     _ptr(weight), _ptr(bias), _c_float(eps), _ptr(out), dtype_code(out.dtype), _ptr(rows), _c_int(n_rows),
-                     _c_int(hidden), _stream())
+                     _ptr(weight), _ptr(bias), eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows,
+                     hidden, _stream())
     return out
 
 
@@ -153,9 +153,9 @@ def post_layernorm_add(stream: torch.Tensor, pending, next_weight: Optional[torc
             raise KernelError(f"post_layernorm_add: out {tuple(out.shape)}, expected {(n_rows, hidden)}")
     if rows is not None:
         _check(rows, "rows", torch.int32)
-    _lib.core().call("mrun_post_layernorm_add", _ptr(stream), _ptr(branch), _ptr(weight), _ptr(bias), _c_float(eps),
-                     _ptr(next_weight), _ptr(next_bias), _c_float(next_eps), _ptr(out), _c_int(code), _ptr(rows),
-                     _c_int(n_rows), _c_int(hidden), _stream())
+    _lib.core().call("mrun_post_layernorm_add", _ptr(stream), _ptr(branch), _ptr(weight), _ptr(bias), eps,
+                     _ptr(next_weight), _ptr(next_bias), next_eps, _ptr(out), code, _ptr(rows),
+                     n_rows, hidden, _stream())
     return out
 
 
@@ -169,8 +169,8 @@ def pair_norm_mean(a: torch.Tensor, b: torch.Tensor, weight_a: torch.Tensor, wei
     if b.shape != a.shape or weight_a.numel() != hidden or weight_b.numel() != hidden:
         raise KernelError(f"pair_norm_mean: a {tuple(a.shape)}, b {tuple(b.shape)}, weights {weight_a.numel()} / {weight_b.numel()}")
     out = torch.empty_like(a)
-    _lib.core().call("mrun_pair_norm_mean", _ptr(a), _ptr(b), _ptr(weight_a), _ptr(weight_b), _c_float(eps),
-                     _c_float(share), _ptr(out), _c_int(rows), _c_int(hidden), _stream())
+    _lib.core().call("mrun_pair_norm_mean", _ptr(a), _ptr(b), _ptr(weight_a), _ptr(weight_b), eps,
+                     share, _ptr(out), rows, hidden, _stream())
     return out
 
 
@@ -191,8 +191,8 @@ def pair_norm_add_layernorm(resid: torch.Tensor, pending, weight: torch.Tensor, 
         raise KernelError(f"pair_norm_add_layernorm: resid {tuple(resid.shape)}, a {tuple(pending.a.shape)}, "
                           f"b {tuple(pending.b.shape)}, out {tuple(out.shape)}")
     _lib.core().call("mrun_pair_norm_add_layernorm", _ptr(resid), _ptr(pending.a), _ptr(pending.b), _ptr(pending.weight_a),
-                     _ptr(pending.weight_b), _c_float(pending.eps), _c_float(pending.share), _ptr(weight), _c_float(eps),
-                     _ptr(out), dtype_code(out.dtype), _ptr(rows), _c_int(n_rows), _c_int(hidden), _stream())
+                     _ptr(pending.weight_b), pending.eps, pending.share, _ptr(weight), eps,
+                     _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream())
     return out
 
 
@@ -204,8 +204,8 @@ def rotary_table(positions: torch.Tensor, inv_freq: torch.Tensor, out: torch.Ten
     tokens, half = positions.numel(), inv_freq.numel()
     if out.shape != (tokens, half, 2):
         raise KernelError(f"rotary_table: out is {tuple(out.shape)}, expected {(tokens, half, 2)}")
-    _lib.core().call("mrun_rotary_table", _ptr(positions), _ptr(inv_freq), _ptr(out), _c_int(tokens),
-                     _c_int(half), ctypes.c_double(magnitude), _stream())
+    _lib.core().call("mrun_rotary_table", _ptr(positions), _ptr(inv_freq), _ptr(out), tokens,
+                     half, magnitude, _stream())
     return out
 
 
@@ -240,9 +240,9 @@ def qk_norm_rope_cache(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: i
                 raise KernelError(f"qk_norm_rope_cache: {name} is {tuple(c.shape)}, expected "
                                   f"[pages, {kv_heads}, {page_size}, {head_dim}]")
     _lib.core().call("mrun_qk_norm_rope_cache", _ptr(qkv), dtype_code(qkv.dtype), _ptr(q_weight),
-                     _ptr(k_weight), _c_float(eps), _ptr(rot), _c_int(rotary_dim if rot is not None else 0),
-                     _ptr(slots), _ptr(k_cache), _ptr(v_cache), _c_int(tokens), _c_int(heads),
-                     _c_int(kv_heads), _c_int(head_dim), _c_int(page_size), _stream())
+                     _ptr(k_weight), eps, _ptr(rot), rotary_dim if rot is not None else 0,
+                     _ptr(slots), _ptr(k_cache), _ptr(v_cache), tokens, heads,
+                     kv_heads, head_dim, page_size, _stream())
 
 
 def proj_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: int, kv_heads: int, dim: int,
@@ -275,11 +275,11 @@ def proj_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, he
     width = x.shape[1]
     if q_off + heads * dim > width or (k_off >= 0 and (k_off + kv_heads * dim > width or v_off + kv_heads * vdim > width)):
         raise KernelError("proj_norm_rope_cache: the heads do not fit the rows")
-    _lib.core().call("mrun_proj_norm_rope_cache", _ptr(x), _c_long(ld), _c_long(q_off), _c_long(k_off), _c_long(v_off),
-                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), _c_float(eps), _ptr(rot),
-                     _c_int(rotary_dim if rot is not None else 0), _c_int(PAIRINGS[pairing]),
-                     _ptr(slots if k_off >= 0 else None), _ptr(k_cache), _ptr(v_cache), _c_int(tokens), _c_int(heads),
-                     _c_int(kv_heads), _c_int(dim), _c_int(vdim), _c_int(page_size), _stream())
+    _lib.core().call("mrun_proj_norm_rope_cache", _ptr(x), ld, q_off, k_off, v_off,
+                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot),
+                     rotary_dim if rot is not None else 0, PAIRINGS[pairing],
+                     _ptr(slots if k_off >= 0 else None), _ptr(k_cache), _ptr(v_cache), tokens, heads,
+                     kv_heads, dim, vdim, page_size, _stream())
 
 
 def head_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: int, kv_heads: int, dim: int,
@@ -326,12 +326,12 @@ def head_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, he
     width = x.shape[1]
     if q_off + heads * dim > width or k_off + kv_heads * dim > width or (v_off >= 0 and v_off + kv_heads * vdim > width):
         raise KernelError("head_norm_rope_cache: the heads do not fit the rows")
-    _lib.core().call("mrun_head_norm_rope_cache", _ptr(x), _c_long(ld), _c_long(q_off), _c_long(k_off), _c_long(v_off),
-                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), _c_float(eps), _ptr(rot),
-                     _c_int(rotary_dim if rot is not None else 0), _c_int(PAIRINGS[pairing]), _ptr(slots), _ptr(k_cache),
-                     _ptr(v_cache), _c_int(tokens), _c_int(heads), _c_int(kv_heads), _c_int(dim), _c_int(vdim),
-                     _c_int(page_size), _ptr(bias), _ptr(first), _c_long(strides[1]), _c_float(share), _ptr(keep),
-                     _c_long(strides[0]), _stream())
+    _lib.core().call("mrun_head_norm_rope_cache", _ptr(x), ld, q_off, k_off, v_off,
+                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot),
+                     rotary_dim if rot is not None else 0, PAIRINGS[pairing], _ptr(slots), _ptr(k_cache),
+                     _ptr(v_cache), tokens, heads, kv_heads, dim, vdim,
+                     page_size, _ptr(bias), _ptr(first), strides[1], share, _ptr(keep),
+                     strides[0], _stream())
 
 
 def check_sink(sink: Optional[torch.Tensor], heads: int) -> None:
@@ -374,11 +374,11 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
         gate_stride = _strided_rows(gate, "gate")
         if gate.shape != (tokens, heads) or gate.dtype != q.dtype:
             raise KernelError(f"paged_attention: gate is {tuple(gate.shape)} {gate.dtype}, expected {(tokens, heads)} {q.dtype}")
-    _lib.core().call("mrun_paged_attention_generic", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(k_cache),
-                     _ptr(v_cache), dtype_code(q.dtype), _ptr(block_tables), _c_int(block_tables.shape[1]),
-                     _ptr(token_slot), _ptr(positions), _c_int(tokens), _c_int(heads), _c_int(kv_heads),
-                     _c_int(head_dim), _c_int(value_dim), _c_int(page_size), _c_long(pages * kv_heads * page_size),
-                     _c_float(scale), _c_int(window), _ptr(sink), _ptr(gate), _c_long(gate_stride),
+    _lib.core().call("mrun_paged_attention_generic", _ptr(q), q_stride, _ptr(out), _ptr(k_cache),
+                     _ptr(v_cache), dtype_code(q.dtype), _ptr(block_tables), block_tables.shape[1],
+                     _ptr(token_slot), _ptr(positions), tokens, heads, kv_heads,
+                     head_dim, value_dim, page_size, pages * kv_heads * page_size,
+                     scale, window, _ptr(sink), _ptr(gate), gate_stride,
                      ctypes.byref(form) if form is not None else _ptr(None), _stream())
     return out
 
@@ -410,10 +410,10 @@ def paged_attention_f32(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cac
                 raise KernelError(f"paged_attention_f32: {name} has {t.numel()} entries for {tiles} tiles")
     if first is None and tiles != tokens:
         raise KernelError(f"paged_attention_f32: {tiles} tiles of single tokens for {tokens} tokens")
-    _lib.core().call("mrun_paged_attention_f32", _ptr(q), _c_long(q_stride), _ptr(out), _ptr(k_cache), _ptr(v_cache),
-                     _ptr(block_tables), _c_int(block_tables.shape[1]), _ptr(token_slot), _ptr(positions), _ptr(first), _ptr(count),
-                     _c_int(tiles), _c_int(tile_tokens), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_int(page_size),
-                     _c_long(pages * kv_heads * page_size), _c_float(scale), _c_int(window), _stream())
+    _lib.core().call("mrun_paged_attention_f32", _ptr(q), q_stride, _ptr(out), _ptr(k_cache), _ptr(v_cache),
+                     _ptr(block_tables), block_tables.shape[1], _ptr(token_slot), _ptr(positions), _ptr(first), _ptr(count),
+                     tiles, tile_tokens, heads, kv_heads, head_dim, page_size,
+                     pages * kv_heads * page_size, scale, window, _stream())
     return out
 
 
@@ -435,8 +435,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False, 
     tokens, inter = out.shape
     if gate_up.shape != (tokens, 2 * inter):
         raise KernelError(f"swiglu: gate_up {tuple(gate_up.shape)} vs out {tuple(out.shape)}")
-    _lib.core().call("mrun_swiglu", _ptr(gate_up), _ptr(out), dtype_code(out.dtype), _c_int(tokens),
-                     _c_int(inter), _c_int(8 if interleaved else 0), _c_int(gate_code(activation)), _stream())
+    _lib.core().call("mrun_swiglu", _ptr(gate_up), _ptr(out), dtype_code(out.dtype), tokens,
+                     inter, 8 if interleaved else 0, gate_code(activation), _stream())
     return out
 
 
@@ -445,8 +445,8 @@ def add_bias(y: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
     _check(y, "y"); _check(bias, "bias", torch.float32)
     if y.dim() != 2 or bias.numel() != y.shape[1]:
         raise KernelError(f"add_bias: y {tuple(y.shape)} vs bias {tuple(bias.shape)}")
-    _lib.core().call("mrun_add_bias", _ptr(y), dtype_code(y.dtype), _ptr(bias), _c_int(y.shape[0]),
-                     _c_int(y.shape[1]), _stream())
+    _lib.core().call("mrun_add_bias", _ptr(y), dtype_code(y.dtype), _ptr(bias), y.shape[0],
+                     y.shape[1], _stream())
     return y
 
 
@@ -490,8 +490,8 @@ class NormedRows:
     def finish(self) -> torch.Tensor:
         tokens, width = self.xw.shape
         out = torch.empty_like(self.xw)
-        _lib.core().call("mrun_norm_finish", _ptr(self.xw), _ptr(self.sums), _c_float(self.eps), _ptr(out),
-                         _c_int(tokens), _c_int(width), _stream())
+        _lib.core().call("mrun_norm_finish", _ptr(self.xw), _ptr(self.sums), self.eps, _ptr(out),
+                         tokens, width, _stream())
         return out
 
 
@@ -602,8 +602,8 @@ PENDING = (PendingLinear, PendingPostNorm, PendingPairNorm, PendingPostLayerNorm
 def _normed(x):
     """(rows, totals pointer, eps) of a product's x, which may be :class:`NormedRows`."""
     if isinstance(x, NormedRows):
-        return x.xw, _ptr(x.sums), _c_float(x.eps)
-    return x, _ptr(None), _c_float(0.0)
+        return x.xw, _ptr(x.sums), x.eps
+    return x, _ptr(None), 0.0
 
 
 def gemm_skinny(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
@@ -620,11 +620,11 @@ def gemm_skinny(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
     n = w.shape[0]
     if w.shape[1] != k:
         raise KernelError(f"gemm_skinny: x {tuple(x.shape)} vs w {tuple(w.shape)}")
-    out = torch.empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype, device=x.device)
+    out = x.new_empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype)
     _lib.core().call("mrun_gemm_skinny", _ptr(x), _ptr(w), _ptr(out), dtype_code(out_dtype),
-                     _c_int(gate_code(activation) if swiglu_rows else 0), _c_int(m), _c_int(n), _c_int(k),
-                     _c_long(x.stride(0) if m > 1 else max(k, x.stride(0))), _c_long(out.shape[1]),
-                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), _c_int(rows), _ptr(None), _c_long(0), _ptr(None),
+                     gate_code(activation) if swiglu_rows else 0, m, n, k,
+                     x.stride(0) if m > 1 else max(k, x.stride(0)), out.shape[1],
+                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), rows, _ptr(None), 0, _ptr(None),
                      _stream())
     return out
 
@@ -660,15 +660,15 @@ def linear_into_norm(pending: PendingLinear, resid: torch.Tensor, weight: torch.
             raise KernelError(f"linear_into_norm: extra {tuple(extra.shape)} {extra.dtype}, share {tuple(share.shape)}")
         if not skinny:          # the tcgen05 product's epilogue has no such rows
             add_scaled_rows(resid, extra.contiguous(), share)
-    xw = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+    xw = x.new_empty((m, n), dtype=torch.bfloat16)
     out_sums = RowSums.take(x.device, m)
-    head = (_ptr(x), _ptr(w), _ptr(None), dtype_code(torch.bfloat16), _c_int(0), _c_int(m), _c_int(n), _c_int(k),
-            _c_long(x.stride(0) if m > 1 else max(k, x.stride(0))), _c_long(n), in_sums, in_eps, _ptr(resid),
+    head = (_ptr(x), _ptr(w), _ptr(None), dtype_code(torch.bfloat16), 0, m, n, k,
+            x.stride(0) if m > 1 else max(k, x.stride(0)), n, in_sums, in_eps, _ptr(resid),
             _ptr(weight), _ptr(xw), _ptr(out_sums))
     if skinny:
-        _lib.core().call("mrun_gemm_skinny", *head, _c_int(rows), _ptr(extra), _c_long(ld_extra), _ptr(share), _stream())
+        _lib.core().call("mrun_gemm_skinny", *head, rows, _ptr(extra), ld_extra, _ptr(share), _stream())
     else:
-        _lib.core().call("mrun_gemm_tc5", *head, _c_int(0), _ptr(_tc5_status(x.device)), _stream())
+        _lib.core().call("mrun_gemm_tc5", *head, 0, _ptr(_tc5_status(x.device)), _stream())
     return NormedRows(xw, out_sums, eps)
 
 
@@ -682,12 +682,12 @@ def gemm_f32_nt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     m, k = x.shape
     n = w.shape[0]
     if out is None:
-        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+        out = x.new_empty((m, n), dtype=torch.float32)
     _check(out, "out", torch.float32)
     if out.shape != (m, n):
         raise KernelError(f"gemm_f32_nt: out is {tuple(out.shape)}, expected {(m, n)}")
-    _lib.core().call("mrun_gemm_f32_nt", _ptr(x), _ptr(w), _ptr(out), _c_int(m), _c_int(n), _c_int(k),
-                     _c_long(x.stride(0) if m > 1 else k), _c_long(n), _stream())
+    _lib.core().call("mrun_gemm_f32_nt", _ptr(x), _ptr(w), _ptr(out), m, n, k,
+                     x.stride(0) if m > 1 else k, n, _stream())
     return out
 
 
@@ -716,19 +716,19 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     m, k = x.shape
     n = w.shape[0]
     if out is None:
-        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+        out = x.new_empty((m, n), dtype=torch.float32)
     _check(out, "out", torch.float32)
     if out.shape != (m, n):
         raise KernelError(f"gemm_f32_tc: out is {tuple(out.shape)}, expected {(m, n)}")
     pitch = -(-k // 8) * 8
     rows = max(1, min(m, F32_TC_SCRATCH // (6 * pitch)))
-    parts = torch.empty(3 * rows * pitch, dtype=torch.bfloat16, device=x.device)
+    parts = x.new_empty(3 * rows * pitch, dtype=torch.bfloat16)
     status = status_word(x.device, "gemm_f32_tc", {1: "the copies of w", 2: "the copies of x", 3: "the conversion of w",
                                                    4: "the MMA issuer", 5: "the sums"})
     for at in range(0, m, rows):
         part, to = x[at:at + rows], out[at:at + rows]
-        _lib.core().call("mrun_gemm_f32_tc", _ptr(part), _ptr(w), _ptr(to), _ptr(parts), _c_int(part.shape[0]), _c_int(n), _c_int(k),
-                         _c_long(x.stride(0) if m > 1 else k), _c_long(n), _c_int(ranges), _c_int(tile), _c_int(cluster), _ptr(status),
+        _lib.core().call("mrun_gemm_f32_tc", _ptr(part), _ptr(w), _ptr(to), _ptr(parts), part.shape[0], n, k,
+                         x.stride(0) if m > 1 else k, n, ranges, tile, cluster, _ptr(status),
                          _stream())
     return out
 
@@ -779,11 +779,11 @@ def gemm_tc5(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, swiglu
     n = w.shape[0]
     if w.shape[1] != k:
         raise KernelError(f"gemm_tc5: x {tuple(x.shape)} vs w {tuple(w.shape)}")
-    out = torch.empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype, device=x.device)
+    out = x.new_empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype)
     _lib.core().call("mrun_gemm_tc5", _ptr(x), _ptr(w), _ptr(out), dtype_code(out_dtype),
-                     _c_int(gate_code(activation) if swiglu_rows else 0), _c_int(m), _c_int(n), _c_int(k),
-                     _c_long(x.stride(0) if m > 1 else max(k, x.stride(0))), _c_long(out.shape[1]),
-                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), _c_int(split),
+                     gate_code(activation) if swiglu_rows else 0, m, n, k,
+                     x.stride(0) if m > 1 else max(k, x.stride(0)), out.shape[1],
+                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), split,
                      _ptr(_tc5_status(x.device)), _stream())
     return out
 
@@ -845,9 +845,9 @@ ACTIVATIONS = {"relu2": 1, "tanh": 2}      # codes of the C ABI (MRUN_ACT_*): fu
 def plain_act(x: torch.Tensor, activation: str, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """act(x) element by element in 32-bit."""
     _check(x, "x")
-    out = torch.empty(x.shape, dtype=out_dtype or x.dtype, device=x.device)
-    _lib.core().call("mrun_plain_act", _ptr(x), _c_int(dtype_code(x.dtype)), _ptr(out), _c_int(dtype_code(out.dtype)),
-                     _c_long(x.numel()), _c_int(ACTIVATIONS[activation]), _stream())
+    out = x.new_empty(x.shape, dtype=out_dtype or x.dtype)
+    _lib.core().call("mrun_plain_act", _ptr(x), dtype_code(x.dtype), _ptr(out), dtype_code(out.dtype),
+                     x.numel(), ACTIVATIONS[activation], _stream())
     return out
 
 
@@ -871,7 +871,7 @@ def linears_batched(x: torch.Tensor, w: torch.Tensor, activation: Optional[str] 
     rows, batch, k = x.shape
     n = w.shape[1]
     if out is None:
-        out = torch.empty((rows, batch, n), dtype=x.dtype, device=x.device)
+        out = x.new_empty((rows, batch, n))
     if not (x.dtype == torch.bfloat16 and rows <= SKINNY_ROWS and k % 32 == 0 and x.stride(0) % 8 == 0
             and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0):
         if activation is not None:
@@ -889,10 +889,10 @@ def linears_batched(x: torch.Tensor, w: torch.Tensor, activation: Optional[str] 
         if gate.shape != (rows, batch) or gate.dtype != x.dtype:
             raise KernelError(f"linears_batched: gate {tuple(gate.shape)} {gate.dtype}")
     _lib.core().call("mrun_gemm_skinny_batched", _ptr(x), _ptr(w), _ptr(out), dtype_code(out.dtype),
-                     _c_int(ACTIVATIONS[activation] if activation else 0), _c_int(batch), _c_int(rows), _c_int(n), _c_int(k),
-                     _c_long(x.stride(0) if rows > 1 else max(k, x.stride(0))), _c_long(out.stride(0) if rows > 1 else max(n, out.stride(0))),
-                     _c_long(x.stride(1) if batch > 1 else 0), _c_long(out.stride(1) if batch > 1 else n), _ptr(None), _ptr(None), _c_long(0),
-                     _c_int(0), _c_int(0), _c_float(0.0), _ptr(gate), _c_long(ld_gate), _ptr(None), _c_float(0.0), _stream())
+                     ACTIVATIONS[activation] if activation else 0, batch, rows, n, k,
+                     x.stride(0) if rows > 1 else max(k, x.stride(0)), out.stride(0) if rows > 1 else max(n, out.stride(0)),
+                     x.stride(1) if batch > 1 else 0, out.stride(1) if batch > 1 else n, _ptr(None), _ptr(None), 0,
+                     0, 0, 0.0, _ptr(gate), ld_gate, _ptr(None), 0.0, _stream())
     return out
 
 
@@ -917,12 +917,12 @@ def linear_blended(x, w: torch.Tensor, bias: Optional[torch.Tensor] = None, blen
         ld_rows, columns = _strided_rows(rows, "blend"), rows.shape[1]
         if rows.shape[0] != m or rows.dtype != torch.bfloat16:
             raise KernelError(f"linear_blended: blend {tuple(rows.shape)} {rows.dtype}")
-    out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+    out = x.new_empty((m, n), dtype=torch.bfloat16)
     _lib.core().call("mrun_gemm_skinny_batched", _ptr(x), _ptr(w), _ptr(out), dtype_code(out.dtype),
-                     _c_int(ACTIVATIONS[activation] if activation else 0), _c_int(1),
-                     _c_int(m), _c_int(n), _c_int(k), _c_long(x.stride(0) if m > 1 else max(k, x.stride(0))), _c_long(n), _c_long(0),
-                     _c_long(n), _ptr(bias), _ptr(rows), _c_long(ld_rows), _c_int(column), _c_int(columns), _c_float(share), _ptr(None),
-                     _c_long(0), sums, eps, _stream())
+                     ACTIVATIONS[activation] if activation else 0, 1,
+                     m, n, k, x.stride(0) if m > 1 else max(k, x.stride(0)), n, 0,
+                     n, _ptr(bias), _ptr(rows), ld_rows, column, columns, share, _ptr(None),
+                     0, sums, eps, _stream())
     return out
 
 
@@ -968,7 +968,7 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.
                 raise KernelError(f"sample: {name} has {t.numel()} entries for {rows} rows")
     if out.numel() < rows:
         raise KernelError(f"sample: out has {out.numel()} entries for {rows} rows")
-    _lib.core().call("mrun_sample", _ptr(logits), _c_int(rows), _c_int(vocab), _ptr(temperature), _ptr(top_p),
+    _lib.core().call("mrun_sample", _ptr(logits), rows, vocab, _ptr(temperature), _ptr(top_p),
                      _ptr(top_k), _ptr(min_p), _ptr(keys), _ptr(out), _stream())
     return out
 
@@ -979,9 +979,9 @@ def top_logprobs(logits: torch.Tensor, n: int):
     _check(logits, "logits", torch.float32)
     rows, vocab = logits.shape
     n = max(1, min(int(n), vocab))
-    ids = torch.empty((rows, n), dtype=torch.int32, device=logits.device)
-    values = torch.empty((rows, n), dtype=torch.float32, device=logits.device)
-    _lib.core().call("mrun_top_logprobs", _ptr(logits), _c_int(rows), _c_int(vocab), _c_int(n), _ptr(ids),
+    ids = logits.new_empty((rows, n), dtype=torch.int32)
+    values = logits.new_empty((rows, n), dtype=torch.float32)
+    _lib.core().call("mrun_top_logprobs", _ptr(logits), rows, vocab, n, _ptr(ids),
                      _ptr(values), _stream())
     return ids, values
 
@@ -994,8 +994,8 @@ def apply_token_mask(logits: torch.Tensor, rows: torch.Tensor, words: torch.Tens
     masks = rows.numel()
     if words.dim() != 2 or words.shape[0] != masks or mask_vocab.numel() != masks:
         raise KernelError(f"apply_token_mask: {masks} rows, words {tuple(words.shape)}, {mask_vocab.numel()} vocabularies")
-    _lib.core().call("mrun_apply_token_mask", _ptr(logits), _c_int(logits.shape[1]), _ptr(rows), _ptr(words),
-                     _c_int(words.shape[1]), _ptr(mask_vocab), _c_int(masks), _stream())
+    _lib.core().call("mrun_apply_token_mask", _ptr(logits), logits.shape[1], _ptr(rows), _ptr(words),
+                     words.shape[1], _ptr(mask_vocab), masks, _stream())
 
 
 def repetition_penalty(logits: torch.Tensor, recent: torch.Tensor, penalty: torch.Tensor) -> None:
@@ -1005,8 +1005,8 @@ def repetition_penalty(logits: torch.Tensor, recent: torch.Tensor, penalty: torc
     rows, vocab = logits.shape
     if recent.dim() != 2 or recent.shape[0] != rows or penalty.numel() < rows:
         raise KernelError(f"repetition_penalty: recent {tuple(recent.shape)}, penalty {penalty.numel()}, rows {rows}")
-    _lib.core().call("mrun_repetition_penalty", _ptr(logits), _c_int(rows), _c_int(vocab), _ptr(recent),
-                     _c_int(recent.shape[1]), _ptr(penalty), _stream())
+    _lib.core().call("mrun_repetition_penalty", _ptr(logits), rows, vocab, _ptr(recent),
+                     recent.shape[1], _ptr(penalty), _stream())
 
 
 def scatter_i32(dst: torch.Tensor, index: torch.Tensor, value: torch.Tensor) -> None:
@@ -1014,8 +1014,8 @@ def scatter_i32(dst: torch.Tensor, index: torch.Tensor, value: torch.Tensor) -> 
     _check(dst, "dst", torch.int32); _check(index, "index", torch.int32); _check(value, "value", torch.int32)
     if index.numel() != value.numel():
         raise KernelError("scatter_i32: index and value differ in length")
-    _lib.core().call("mrun_scatter_i32", _ptr(dst), _ptr(index), _ptr(value), _c_int(index.numel()),
-                     _c_long(dst.numel()), _stream())
+    _lib.core().call("mrun_scatter_i32", _ptr(dst), _ptr(index), _ptr(value), index.numel(),
+                     dst.numel(), _stream())
 
 
 def select_tokens(ids: torch.Tensor, previous: torch.Tensor, source: torch.Tensor) -> None:
@@ -1023,8 +1023,8 @@ def select_tokens(ids: torch.Tensor, previous: torch.Tensor, source: torch.Tenso
     _check(ids, "ids", torch.int32); _check(previous, "previous", torch.int32); _check(source, "source", torch.int32)
     if source.numel() != ids.numel():
         raise KernelError("select_tokens: one source per row is needed")
-    _lib.core().call("mrun_select_tokens", _ptr(ids), _ptr(previous), _ptr(source), _c_int(ids.numel()),
-                     _c_int(previous.numel()), _stream())
+    _lib.core().call("mrun_select_tokens", _ptr(ids), _ptr(previous), _ptr(source), ids.numel(),
+                     previous.numel(), _stream())
 
 
 
@@ -1039,10 +1039,10 @@ def gemm_f32_nt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> 
     n = w.shape[1]
     if w.shape != (batch, n, k) or out.shape != (batch, m, n) or x.stride(2) != 1 or out.stride(2) != 1:
         raise KernelError(f"gemm_f32_nt_batched: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
-    _lib.core().call("mrun_gemm_f32_nt_batched", _ptr(x), _ptr(w), _ptr(out), _c_int(batch), _c_int(m), _c_int(n),
-                     _c_int(k), _c_long(x.stride(1) if m > 1 else max(k, x.stride(1))),
-                     _c_long(out.stride(1) if m > 1 else max(n, out.stride(1))),
-                     _c_long(x.stride(0)), _c_long(n * k), _c_long(out.stride(0)), _stream())
+    _lib.core().call("mrun_gemm_f32_nt_batched", _ptr(x), _ptr(w), _ptr(out), batch, m, n,
+                     k, x.stride(1) if m > 1 else max(k, x.stride(1)),
+                     out.stride(1) if m > 1 else max(n, out.stride(1)),
+                     x.stride(0), n * k, out.stride(0), _stream())
     return out
 
 
@@ -1090,10 +1090,10 @@ def latent_prepare(down: torch.Tensor, q_weight: Optional[torch.Tensor], kv_weig
         _check(rot, "rot", torch.float32)
         if rot.shape != (tokens, rot_dims // 2, 2):
             raise KernelError(f"latent_prepare: rot is {tuple(rot.shape)}, expected {(tokens, rot_dims // 2, 2)}")
-    _lib.core().call("mrun_latent_prepare", _ptr(down), dtype_code(down.dtype), _c_long(down.stride(0)),
-                     _ptr(q_weight), _ptr(kv_weight), _c_float(eps), _ptr(rot), _c_int(rot_dims),
-                     _c_int(PAIRINGS[pairing]), _ptr(slots), _ptr(cq), _ptr(cache if slots is not None else None),
-                     _c_int(tokens), _c_int(q_rank), _c_int(kv_rank), _c_int(rot_dim), _c_int(width), _stream())
+    _lib.core().call("mrun_latent_prepare", _ptr(down), dtype_code(down.dtype), down.stride(0),
+                     _ptr(q_weight), _ptr(kv_weight), eps, _ptr(rot), rot_dims,
+                     PAIRINGS[pairing], _ptr(slots), _ptr(cq), _ptr(cache if slots is not None else None),
+                     tokens, q_rank, kv_rank, rot_dim, width, _stream())
 
 
 def latent_rows(cache: torch.Tensor, block_tables: torch.Tensor, seg_slot: torch.Tensor, seg_kv_len: torch.Tensor, rows: int,
@@ -1114,11 +1114,11 @@ def latent_rows(cache: torch.Tensor, block_tables: torch.Tensor, seg_slot: torch
         if keys.dim() != 4 or keys.shape[0] != segments or keys.shape[2] != rows or keys.shape[3] < rot_dim:
             raise KernelError(f"latent_rows: keys {tuple(keys.shape)} for {segments} segments of {rows} rows")
         heads, dim = keys.shape[1], keys.shape[3] - rot_dim
-    out = torch.empty((segments, rows, kv_rank), dtype=cache.dtype, device=cache.device)
-    _lib.core().call("mrun_latent_rows", _ptr(cache), dtype_code(cache.dtype), _ptr(block_tables), _c_int(block_tables.shape[1]),
-                     _ptr(seg_slot), _ptr(seg_kv_len), _ptr(out), _c_int(segments), _c_int(rows), _c_int(cache.shape[2]),
-                     _c_int(kv_rank), _c_int(cache.shape[3]), _ptr(keys if rot_dim else None), _c_int(heads), _c_int(dim),
-                     _c_int(rot_dim), _stream())
+    out = cache.new_empty((segments, rows, kv_rank))
+    _lib.core().call("mrun_latent_rows", _ptr(cache), dtype_code(cache.dtype), _ptr(block_tables), block_tables.shape[1],
+                     _ptr(seg_slot), _ptr(seg_kv_len), _ptr(out), segments, rows, cache.shape[2],
+                     kv_rank, cache.shape[3], _ptr(keys if rot_dim else None), heads, dim,
+                     rot_dim, _stream())
     return out
 
 
@@ -1129,8 +1129,8 @@ def latent_rotate(q: torch.Tensor, rot: torch.Tensor, rot_dims: int, pairing: st
     tokens = q.shape[0]
     if q.shape[1] != heads * (dim + rot_dim) or rot.shape != (tokens, rot_dims // 2, 2):
         raise KernelError(f"latent_rotate: q {tuple(q.shape)}, rot {tuple(rot.shape)}")
-    _lib.core().call("mrun_latent_rotate", _ptr(q), _c_long(ldq), dtype_code(q.dtype), _ptr(rot), _c_int(rot_dims),
-                     _c_int(PAIRINGS[pairing]), _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(rot_dim), _stream())
+    _lib.core().call("mrun_latent_rotate", _ptr(q), ldq, dtype_code(q.dtype), _ptr(rot), rot_dims,
+                     PAIRINGS[pairing], tokens, heads, dim, rot_dim, _stream())
 
 
 def latent_query(q: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: int, pairing: str, q_att: torch.Tensor,
@@ -1146,9 +1146,9 @@ def latent_query(q: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: int, pa
         _check(rot, "rot", torch.float32)
         if rot.shape != (tokens, rot_dims // 2, 2):
             raise KernelError(f"latent_query: rot is {tuple(rot.shape)}, expected {(tokens, rot_dims // 2, 2)}")
-    _lib.core().call("mrun_latent_query", _ptr(q), _c_long(ldq), dtype_code(q.dtype), _ptr(rot), _c_int(rot_dims),
-                     _c_int(PAIRINGS[pairing]), _ptr(q_att), _c_int(tokens), _c_int(heads), _c_int(dim),
-                     _c_int(rot_dim), _c_int(kv_rank), _c_int(q_att.shape[2]), _stream())
+    _lib.core().call("mrun_latent_query", _ptr(q), ldq, dtype_code(q.dtype), _ptr(rot), rot_dims,
+                     PAIRINGS[pairing], _ptr(q_att), tokens, heads, dim,
+                     rot_dim, kv_rank, q_att.shape[2], _stream())
 
 
 def post_norm_add(stream: torch.Tensor, branch: torch.Tensor, w_post: torch.Tensor, scale: float, eps_post: float,
@@ -1171,9 +1171,9 @@ def post_norm_add(stream: torch.Tensor, branch: torch.Tensor, w_post: torch.Tens
         code = dtype_code(out.dtype)
     if rows is not None:
         _check(rows, "rows", torch.int32)
-    _lib.core().call("mrun_post_norm_add", _ptr(stream), _ptr(branch), _ptr(w_post), _c_float(scale),
-                     _c_float(eps_post), _ptr(w_next), _c_float(eps_next), _ptr(out if w_next is not None else None),
-                     _c_int(code), _ptr(rows), _c_int(n_rows), _c_int(hidden), _stream())
+    _lib.core().call("mrun_post_norm_add", _ptr(stream), _ptr(branch), _ptr(w_post), scale,
+                     eps_post, _ptr(w_next), eps_next, _ptr(out if w_next is not None else None),
+                     code, _ptr(rows), n_rows, hidden, _stream())
     return out
 
 
@@ -1195,14 +1195,14 @@ def route_top_k(logits: torch.Tensor, top: int, score: str = "softmax", renormal
         _check(bias, "bias", torch.float32)
         if bias.numel() != experts:
             raise KernelError(f"route_top_k: bias has {bias.numel()} entries for {experts} experts")
-    weights = torch.empty((tokens, experts), dtype=torch.float32, device=logits.device)
+    weights = logits.new_empty((tokens, experts), dtype=torch.float32)
     if chosen is not None:
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"route_top_k: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_route_top_k", _ptr(logits), _c_long(logits.stride(0)), _ptr(bias), _ptr(weights), _ptr(chosen),
-                     _c_int(tokens), _c_int(experts), _c_int(top), _c_int(ROUTER_SCORES[score]),
-                     _c_int(1 if renormalize else 0), _stream())
+    _lib.core().call("mrun_route_top_k", _ptr(logits), logits.stride(0), _ptr(bias), _ptr(weights), _ptr(chosen),
+                     tokens, experts, top, ROUTER_SCORES[score],
+                     1 if renormalize else 0, _stream())
     return weights
 
 
@@ -1218,22 +1218,22 @@ def relu2_scaled(u: torch.Tensor, weights: Optional[torch.Tensor], experts: int,
     else:
         experts, ff = 0, columns
     act = torch.empty_like(u)
-    _lib.core().call("mrun_relu2_scaled", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(weights), _c_int(tokens),
-                     _c_int(columns), _c_int(experts), _c_int(max(1, ff)), _stream())
+    _lib.core().call("mrun_relu2_scaled", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(weights), tokens,
+                     columns, experts, max(1, ff), _stream())
     return act
 
 
 def soft_cap(x: torch.Tensor, cap: float) -> torch.Tensor:
     """x = cap * tanh(x / cap) in place on float32."""
     _check(x, "x", torch.float32)
-    _lib.core().call("mrun_soft_cap", _ptr(x), _c_long(x.numel()), _c_float(cap), _stream())
+    _lib.core().call("mrun_soft_cap", _ptr(x), x.numel(), cap, _stream())
     return x
 
 
 def scale(x: torch.Tensor, factor: float) -> torch.Tensor:
     """x *= factor in place on float32."""
     _check(x, "x", torch.float32)
-    _lib.core().call("mrun_scale_f32", _ptr(x), _c_long(x.numel()), _c_float(factor), _stream())
+    _lib.core().call("mrun_scale_f32", _ptr(x), x.numel(), factor, _stream())
     return x
 
 
@@ -1256,7 +1256,7 @@ def moe_sort(chosen: torch.Tensor, weights: torch.Tensor):
     books = zeros[:3 * experts].view(3, experts)                              # counts, ends, cursor
     source, row_weight = zeros[3 * experts:3 * experts + pairs], zeros[3 * experts + pairs:].view(torch.float32)
     dest = torch.empty((tokens, top), dtype=torch.int32, device=dev)
-    _lib.core().call("mrun_moe_sort", _ptr(chosen), _ptr(weights), _c_int(tokens), _c_int(experts), _c_int(top),
+    _lib.core().call("mrun_moe_sort", _ptr(chosen), _ptr(weights), tokens, experts, top,
                      _ptr(books[0]), _ptr(books[1]), _ptr(books[2]), _ptr(source), _ptr(row_weight), _ptr(dest), _stream())
     return books[1], source, row_weight, dest
 
@@ -1264,9 +1264,9 @@ def moe_sort(chosen: torch.Tensor, weights: torch.Tensor):
 def gather_rows(x: torch.Tensor, source: torch.Tensor) -> torch.Tensor:
     """out[r] = x[source[r]]."""
     _check(x, "x"); _check(source, "source", torch.int32)
-    out = torch.empty((source.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
-    _lib.core().call("mrun_gather_rows", _ptr(x), dtype_code(x.dtype), _ptr(source), _ptr(out), _c_int(source.numel()),
-                     _c_int(x.shape[1]), _stream())
+    out = x.new_empty((source.numel(), x.shape[1]))
+    _lib.core().call("mrun_gather_rows", _ptr(x), dtype_code(x.dtype), _ptr(source), _ptr(out), source.numel(),
+                     x.shape[1], _stream())
     return out
 
 
@@ -1276,8 +1276,8 @@ def relu2_rows(u: torch.Tensor, row_weight: torch.Tensor) -> torch.Tensor:
     if row_weight.numel() != u.shape[0]:
         raise KernelError("relu2_rows: one weight per row is needed")
     act = torch.empty_like(u)
-    _lib.core().call("mrun_relu2_rows", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(row_weight), _c_int(u.shape[0]),
-                     _c_int(u.shape[1]), _stream())
+    _lib.core().call("mrun_relu2_rows", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(row_weight), u.shape[0],
+                     u.shape[1], _stream())
     return act
 
 
@@ -1297,10 +1297,10 @@ def combine_rows(base: Optional[torch.Tensor], rows: torch.Tensor, dest: torch.T
         _check(extra, "extra", rows.dtype); _check(share, "share", torch.float32)
         if extra.shape != (tokens, width) or share.numel() != tokens:
             raise KernelError(f"combine_rows: extra {tuple(extra.shape)}, share {tuple(share.shape)}")
-    out = torch.empty((tokens, width), dtype=torch.float32, device=rows.device)
-    _lib.core().call("mrun_combine_rows", _ptr(base), _c_int(1 if base is not None and base.dtype == torch.float32 else 0),
-                     _ptr(rows), dtype_code(rows.dtype), _ptr(dest), _ptr(out), _c_int(tokens), _c_int(top),
-                     _c_int(width), _ptr(extra), _ptr(share), _stream())
+    out = rows.new_empty((tokens, width), dtype=torch.float32)
+    _lib.core().call("mrun_combine_rows", _ptr(base), 1 if base is not None and base.dtype == torch.float32 else 0,
+                     _ptr(rows), dtype_code(rows.dtype), _ptr(dest), _ptr(out), tokens, top,
+                     width, _ptr(extra), _ptr(share), _stream())
     return out
 
 
@@ -1322,8 +1322,8 @@ def embed_streams(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, cop
     tokens = ids.numel()
     if out.shape != (tokens, copies * hidden):
         raise KernelError(f"embed_streams: out is {tuple(out.shape)}, expected {(tokens, copies * hidden)}")
-    _lib.core().call("mrun_embed_streams", _ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), _c_int(tokens),
-                     _c_int(hidden), _c_int(vocab), _c_int(copies), _stream())
+    _lib.core().call("mrun_embed_streams", _ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), tokens,
+                     hidden, vocab, copies, _stream())
     return out
 
 
@@ -1345,10 +1345,10 @@ def embed_bigram(table: torch.Tensor, pairs: Optional[torch.Tensor], ids: torch.
         _check(pairs, "pairs", table.dtype); _check(state, "state", torch.int32)
         if pairs.shape != (buckets + 1, hidden):
             raise KernelError(f"embed_bigram: pairs is {tuple(pairs.shape)}, expected {(buckets + 1, hidden)}")
-        rows = torch.empty(tokens, dtype=torch.int32, device=ids.device)
+        rows = ids.new_empty(tokens, dtype=torch.int32)
     _lib.core().call("mrun_embed_bigram", _ptr(table), _ptr(pairs), dtype_code(table.dtype), _ptr(ids), _ptr(positions),
-                     _ptr(token_slot), _ptr(state), _ptr(rows), _ptr(out), _c_int(tokens), _c_int(hidden), _c_int(vocab),
-                     _c_int(copies), _c_float(scale), _c_int(buckets), _c_long(mul_prev), _c_long(mul_cur), _stream())
+                     _ptr(token_slot), _ptr(state), _ptr(rows), _ptr(out), tokens, hidden, vocab,
+                     copies, scale, buckets, mul_prev, mul_cur, _stream())
     return out
 
 
@@ -1392,16 +1392,16 @@ def streams_step(streams: torch.Tensor, pending: Optional[PendingStreams], in_c:
         _check(rows, "rows", torch.int32)
     h = u = None
     if want_sum:
-        u = torch.empty((n_rows, width), dtype=torch.float32, device=streams.device)
+        u = streams.new_empty((n_rows, width), dtype=torch.float32)
     else:
         _check(norm_weight, "norm_weight", torch.float32)
         if norm_weight.numel() != width:
             raise KernelError(f"streams_step: the norm weight has {norm_weight.numel()} entries, the width is {width}")
-        h = torch.empty((n_rows, width), dtype=out_dtype, device=streams.device)
+        h = streams.new_empty((n_rows, width), dtype=out_dtype)
     _lib.core().call("mrun_streams_step", _ptr(streams), _ptr(y), _ptr(mix), _ptr(out_c), _ptr(in_c),
-                     _ptr(None if want_sum else norm_weight), _c_float(eps), _ptr(h),
-                     _c_int(dtype_code(out_dtype if h is not None else torch.float32)), _ptr(u), _ptr(rows),
-                     _c_int(n_rows), _c_int(count), _c_int(width), _stream())
+                     _ptr(None if want_sum else norm_weight), eps, _ptr(h),
+                     dtype_code(out_dtype if h is not None else torch.float32), _ptr(u), _ptr(rows),
+                     n_rows, count, width, _stream())
     return u if want_sum else h
 
 
@@ -1423,11 +1423,11 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, ctx,
         _check(bias, "bias", torch.float32)
         if bias.numel() != channels:
             raise KernelError(f"causal_conv: bias has {bias.numel()} entries for {channels} channels")
-    out = torch.empty((tokens, channels), dtype=x.dtype, device=x.device)
-    _lib.core().call("mrun_causal_conv", _ptr(x), _c_long(x.stride(0)), _ptr(weight), _ptr(bias), _ptr(state), _ptr(out),
-                     _c_long(channels), dtype_code(x.dtype), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     _c_int(ctx.num_segments), _c_int(ctx.max_q_len), _c_int(channels), _c_int(taps),
-                     _c_int(1 if residual else 0), _c_int(1 if silu else 0), _stream())
+    out = x.new_empty((tokens, channels))
+    _lib.core().call("mrun_causal_conv", _ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(state), _ptr(out),
+                     channels, dtype_code(x.dtype), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
+                     ctx.num_segments, ctx.max_q_len, channels, taps,
+                     1 if residual else 0, 1 if silu else 0, _stream())
     return out
 
 
@@ -1515,9 +1515,9 @@ def _chunk_scratch(ctx, delta: bool, q, k, v, ld: int, a, bias, state, out, head
         return None
     size = _lib.core().function("mrun_chunked_scan_floats")
     size.restype = _c_long
-    floats = size(_c_int(1 if delta else 0), _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(dtype_code(q.dtype)), _ptr(a), _ptr(bias),
-                  _ptr(state), _ptr(out), _c_int(chunks), _c_int(heads), _c_int(dim), _c_int(vdim))
-    return (torch.empty(floats, dtype=torch.float32, device=q.device), chunks) if floats else None
+    floats = size(1 if delta else 0, _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(a), _ptr(bias),
+                  _ptr(state), _ptr(out), chunks, heads, dim, vdim)
+    return (q.new_empty(floats, dtype=torch.float32), chunks) if floats else None
 
 
 def _chunked_scan(q, k, v, ld: int, decay, silu_inputs: bool, a, bias, tau: float, state, ctx, out, heads: int, dim: int,
@@ -1526,9 +1526,9 @@ def _chunked_scan(q, k, v, ld: int, decay, silu_inputs: bool, a, bias, tau: floa
     found = _chunk_scratch(ctx, False, q, k, v, ld, a, bias, state, out, heads, dim, vdim)
     if found is None:
         return False
-    _lib.core().call("mrun_chunked_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _ptr(decay), _c_int(1 if silu_inputs else 0),
-                     _ptr(a), _ptr(bias), _c_float(tau), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
-                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(found[1]), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    _lib.core().call("mrun_chunked_scan", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(decay), 1 if silu_inputs else 0,
+                     _ptr(a), _ptr(bias), tau, _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
+                     _ptr(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _stream())
     return True
 
 
@@ -1538,9 +1538,9 @@ def _chunked_delta_scan(q, k, v, ld: int, a, b, ldb: int, a_log, dt_bias, state,
     found = _chunk_scratch(ctx, True, q, k, v, ld, a, dt_bias, state, out, heads, dim, vdim)
     if found is None:
         return False
-    _lib.core().call("mrun_chunked_delta_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), _c_int(heads // kv_heads), _ptr(a), _ptr(b),
-                     _c_long(ldb), _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
-                     _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(found[1]), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    _lib.core().call("mrun_chunked_delta_scan", _ptr(q), _ptr(k), _ptr(v), ld, heads // kv_heads, _ptr(a), _ptr(b),
+                     ldb, _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
+                     _ptr(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _stream())
     return True
 
 
@@ -1557,14 +1557,14 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if q.shape[1] != heads * dim or k.shape[1] != heads * dim or v.shape[1] != heads * vdim \
             or state.shape[1:] != (heads, dim, vdim) or decay.numel() != heads:
         raise KernelError("decay_scan: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    out = q.new_empty((tokens, heads * vdim), dtype=torch.float32)
     if _chunked_scan(q, k, v, ld, decay, silu_inputs, None, None, 1.0, state, ctx, out, heads, dim, vdim):
         return out
-    scratch = torch.empty(tokens * (2 * heads * dim + heads * vdim), dtype=torch.float32, device=q.device)
-    _lib.core().call("mrun_decay_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype), _ptr(decay),
+    scratch = q.new_empty(tokens * (2 * heads * dim + heads * vdim), dtype=torch.float32)
+    _lib.core().call("mrun_decay_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(decay),
                      _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     _c_int(ctx.num_segments), _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(vdim),
-                     _c_int(1 if silu_inputs else 0), _stream())
+                     ctx.num_segments, tokens, heads, dim, vdim,
+                     1 if silu_inputs else 0, _stream())
     return out
 
 
@@ -1586,14 +1586,14 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
             or a.shape != (tokens, heads * dim) or b.shape != (tokens, heads) or b.dtype != q.dtype \
             or a_log.numel() != heads or dt_bias.numel() != heads * dim or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("delta_scan: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    out = q.new_empty((tokens, heads * vdim), dtype=torch.float32)
     if _chunked_delta_scan(q, k, v, ld, a, b, ldb, a_log, dt_bias, state, ctx, out, heads, kv_heads, dim, vdim):
         return out
-    scratch = torch.empty(tokens * (2 * kv_heads * dim + heads * (vdim + dim + 1)), dtype=torch.float32, device=q.device)
-    _lib.core().call("mrun_delta_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype),
-                     _c_int(heads // kv_heads), _ptr(a), _ptr(b), _c_long(ldb), _ptr(a_log), _ptr(dt_bias), _ptr(state),
-                     _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), _c_int(ctx.num_segments),
-                     _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    scratch = q.new_empty(tokens * (2 * kv_heads * dim + heads * (vdim + dim + 1)), dtype=torch.float32)
+    _lib.core().call("mrun_delta_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype),
+                     heads // kv_heads, _ptr(a), _ptr(b), ldb, _ptr(a_log), _ptr(dt_bias), _ptr(state),
+                     _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments,
+                     tokens, heads, dim, vdim, _stream())
     return out
 
 
@@ -1612,13 +1612,13 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
     if q.shape[1] != heads * dim or k.shape[1] != heads * dim or v.shape[1] != heads * vdim \
             or a.shape != (tokens, heads * dim) or bias.numel() != heads * dim or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("gated_scan: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
+    out = q.new_empty((tokens, heads * vdim), dtype=torch.float32)
     if _chunked_scan(q, k, v, ld, None, False, a, bias, tau, state, ctx, out, heads, dim, vdim):
         return out
-    scratch = torch.empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32, device=q.device)
-    _lib.core().call("mrun_gated_scan", _ptr(q), _ptr(k), _ptr(v), _c_long(ld), dtype_code(q.dtype), _ptr(a), _ptr(bias),
-                     _c_float(tau), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     _c_int(ctx.num_segments), _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+    scratch = q.new_empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32)
+    _lib.core().call("mrun_gated_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(a), _ptr(bias),
+                     tau, _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
+                     ctx.num_segments, tokens, heads, dim, vdim, _stream())
     return out
 
 
@@ -1639,13 +1639,13 @@ def gated_norm(o: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, eps: f
     if gate.shape != o.shape or gate.dtype != out_dtype or weight.numel() not in (n, features) or n * groups != features:
         raise KernelError("gated_norm: sizes do not match")
     if out is None:
-        out = torch.empty((tokens, features), dtype=out_dtype, device=o.device)
+        out = o.new_empty((tokens, features), dtype=out_dtype)
     ldo = _strided_rows(out, "out")
     if out.shape != o.shape or out.dtype != out_dtype:
         raise KernelError(f"gated_norm: out is {tuple(out.shape)} {out.dtype}")
-    _lib.core().call("mrun_gated_norm", _ptr(o), _ptr(weight), _c_int(weight.numel()), _ptr(gate), _c_long(ldg),
-                     dtype_code(out_dtype), _c_float(eps), _ptr(out), _c_long(ldo), _c_float(scale), _c_int(tokens), _c_int(groups), _c_int(n),
-                     _c_int(GATE_SHAPES[gate_function]), _stream())
+    _lib.core().call("mrun_gated_norm", _ptr(o), _ptr(weight), weight.numel(), _ptr(gate), ldg,
+                     dtype_code(out_dtype), eps, _ptr(out), ldo, scale, tokens, groups, n,
+                     GATE_SHAPES[gate_function], _stream())
     return out
 
 
@@ -1661,10 +1661,10 @@ def skip_gate_norm(o: torch.Tensor, x: torch.Tensor, skip: torch.Tensor, z: torc
     if x.shape != o.shape or z.shape != o.shape or x.dtype != z.dtype or weight.numel() != features or features % groups \
             or features % skip.numel():
         raise KernelError(f"skip_gate_norm: o {tuple(o.shape)}, x {tuple(x.shape)}, z {tuple(z.shape)}, {groups} groups")
-    out = torch.empty((tokens, features), dtype=x.dtype, device=o.device)
-    _lib.core().call("mrun_skip_gate_norm", _ptr(o), _ptr(x), _c_long(ldx), _ptr(skip), _c_int(features // skip.numel()),
-                     _ptr(z), _c_long(ldz), _ptr(weight), _c_int(dtype_code(x.dtype)), _c_float(eps), _ptr(out),
-                     _c_int(tokens), _c_int(groups), _c_int(features // groups), _stream())
+    out = o.new_empty((tokens, features), dtype=x.dtype)
+    _lib.core().call("mrun_skip_gate_norm", _ptr(o), _ptr(x), ldx, _ptr(skip), features // skip.numel(),
+                     _ptr(z), ldz, _ptr(weight), dtype_code(x.dtype), eps, _ptr(out),
+                     tokens, groups, features // groups, _stream())
     return out
 
 
@@ -1677,10 +1677,10 @@ def token_blend(x: torch.Tensor, mu: torch.Tensor, state: torch.Tensor, ctx) -> 
     tokens, channels = x.shape
     if mu.dim() != 2 or mu.shape[1] != channels or state.shape[1:] != (1, channels):
         raise KernelError(f"token_blend: x {tuple(x.shape)}, mu {tuple(mu.shape)}, state {tuple(state.shape)}")
-    out = torch.empty((tokens, mu.shape[0], channels), dtype=x.dtype, device=x.device)
-    _lib.core().call("mrun_token_blend", _ptr(x), _c_long(ldx), _ptr(mu), _ptr(state), _ptr(out), _c_int(dtype_code(x.dtype)),
-                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(ctx.max_q_len),
-                     _c_int(channels), _c_int(mu.shape[0]), _stream())
+    out = x.new_empty((tokens, mu.shape[0], channels))
+    _lib.core().call("mrun_token_blend", _ptr(x), ldx, _ptr(mu), _ptr(state), _ptr(out), dtype_code(x.dtype),
+                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
+                     channels, mu.shape[0], _stream())
     return out
 
 
@@ -1702,14 +1702,14 @@ def bonus_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
             or a.shape != (tokens, heads * dim) or bias.numel() != heads * dim or bonus.numel() != heads * dim \
             or state.shape[1:] != (heads, dim, vdim):
         raise KernelError("bonus_scan: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=r.device)
+    out = r.new_empty((tokens, heads * vdim), dtype=torch.float32)
     scratch = None
-    if not _lib.core().function("mrun_scan_walks")(_c_int(0), _ptr(r), _ptr(k), _ptr(v), _c_long(ld), dtype_code(r.dtype), _ptr(a),
-                                                   _ptr(bias), _ptr(bonus), _ptr(state), _c_int(dim), _c_int(vdim)):
-        scratch = torch.empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32, device=r.device)
-    _lib.core().call("mrun_bonus_scan", _ptr(r), _ptr(k), _ptr(v), _c_long(ld), dtype_code(r.dtype), _ptr(a), _ptr(bias),
+    if not _lib.core().function("mrun_scan_walks")(0, _ptr(r), _ptr(k), _ptr(v), ld, dtype_code(r.dtype), _ptr(a),
+                                                   _ptr(bias), _ptr(bonus), _ptr(state), dim, vdim):
+        scratch = r.new_empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32)
+    _lib.core().call("mrun_bonus_scan", _ptr(r), _ptr(k), _ptr(v), ld, dtype_code(r.dtype), _ptr(a), _ptr(bias),
                      _ptr(bonus), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     _c_int(ctx.num_segments), _c_int(ctx.max_q_len), _c_int(tokens), _c_int(heads), _c_int(dim), _c_int(vdim), _stream())
+                     ctx.num_segments, ctx.max_q_len, tokens, heads, dim, vdim, _stream())
     return out
 
 
@@ -1730,15 +1730,15 @@ def ssm_scan(c: torch.Tensor, b: torch.Tensor, x: torch.Tensor, dt: torch.Tensor
             or dt.shape != (tokens, heads) or dt_bias.numel() != heads or a_log.numel() != heads \
             or state.shape[1:] != (heads, size, vdim):
         raise KernelError("ssm_scan: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=c.device)
+    out = c.new_empty((tokens, heads * vdim), dtype=torch.float32)
     scratch = None
-    if not _lib.core().function("mrun_scan_walks")(_c_int(1), _ptr(c), _ptr(b), _ptr(x), _c_long(ld), dtype_code(c.dtype), _ptr(None),
-                                                   _ptr(dt_bias), _ptr(None), _ptr(state), _c_int(size), _c_int(vdim)):
-        scratch = torch.empty(tokens * (2 * groups * size + heads * (vdim + 1)), dtype=torch.float32, device=c.device)
-    _lib.core().call("mrun_ssm_scan", _ptr(c), _ptr(b), _ptr(x), _c_long(ld), dtype_code(c.dtype), _c_int(heads // groups),
-                     _ptr(dt), _c_long(lddt), _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out), _ptr(scratch),
-                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(ctx.max_q_len), _c_int(tokens), _c_int(heads),
-                     _c_int(size), _c_int(vdim), _stream())
+    if not _lib.core().function("mrun_scan_walks")(1, _ptr(c), _ptr(b), _ptr(x), ld, dtype_code(c.dtype), _ptr(None),
+                                                   _ptr(dt_bias), _ptr(None), _ptr(state), size, vdim):
+        scratch = c.new_empty(tokens * (2 * groups * size + heads * (vdim + 1)), dtype=torch.float32)
+    _lib.core().call("mrun_ssm_scan", _ptr(c), _ptr(b), _ptr(x), ld, dtype_code(c.dtype), heads // groups,
+                     _ptr(dt), lddt, _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out), _ptr(scratch),
+                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len, tokens, heads,
+                     size, vdim, _stream())
     return out
 
 
@@ -1759,11 +1759,11 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, dt_bias: 
             or state.shape[1:] != (inner, states) or z.dtype != x.dtype or c.dtype != b.dtype \
             or b.dtype != (x.dtype if ctx.max_q_len == 1 else torch.float32):
         raise KernelError("selective_scan: sizes or types do not match")
-    out = torch.empty((tokens, inner), dtype=x.dtype, device=x.device)
-    _lib.core().call("mrun_selective_scan", _ptr(x), _c_long(ldx), _ptr(z), _c_long(ldz), _ptr(b), _ptr(c), _c_long(ldb),
-                     dtype_code(x.dtype), _ptr(dt), _c_long(lddt), _ptr(dt_bias), _ptr(a), _ptr(skip), _ptr(state), _ptr(out),
-                     _c_long(inner), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), _c_int(ctx.num_segments), _c_int(ctx.max_q_len),
-                     _c_int(tokens), _c_int(inner), _c_int(states), _stream())
+    out = x.new_empty((tokens, inner))
+    _lib.core().call("mrun_selective_scan", _ptr(x), ldx, _ptr(z), ldz, _ptr(b), _ptr(c), ldb,
+                     dtype_code(x.dtype), _ptr(dt), lddt, _ptr(dt_bias), _ptr(a), _ptr(skip), _ptr(state), _ptr(out),
+                     inner, _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
+                     tokens, inner, states, _stream())
     return out
 
 
@@ -1775,8 +1775,8 @@ def head_gate(y: torch.Tensor, gate: torch.Tensor, heads: int) -> torch.Tensor:
     tokens, features = y.shape
     if gate.shape != (tokens, heads) or gate.dtype != y.dtype or features % heads:
         raise KernelError("head_gate: sizes do not match")
-    _lib.core().call("mrun_head_gate", _ptr(y), _ptr(gate), _c_long(ldg), dtype_code(y.dtype), _c_int(tokens), _c_int(heads),
-                     _c_int(features // heads), _stream())
+    _lib.core().call("mrun_head_gate", _ptr(y), _ptr(gate), ldg, dtype_code(y.dtype), tokens, heads,
+                     features // heads, _stream())
     return y
 
 
@@ -1800,10 +1800,10 @@ def diff_rope_cache(qkv: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: in
             raise KernelError(f"diff_rope_cache: rot is {tuple(rot.shape)}")
     if slots is not None:
         _check(slots, "slots", torch.int32)
-    _lib.core().call("mrun_diff_rope_cache", _ptr(qkv), _c_long(qkv.stride(0)), dtype_code(qkv.dtype), _ptr(rot),
-                     _c_int(rot_dims if rot is not None else 0), _ptr(slots), _ptr(k_cache), _ptr(v_cache), _c_long(pages),
-                     _c_int(tokens), _c_int(heads), _c_int(kv_heads), _c_int(dim), _c_int(vdim), _c_int(vdim // chunks),
-                     _c_int(page_size), _stream())
+    _lib.core().call("mrun_diff_rope_cache", _ptr(qkv), qkv.stride(0), dtype_code(qkv.dtype), _ptr(rot),
+                     rot_dims if rot is not None else 0, _ptr(slots), _ptr(k_cache), _ptr(v_cache), pages,
+                     tokens, heads, kv_heads, dim, vdim, vdim // chunks,
+                     page_size, _stream())
 
 
 def diff_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor,
@@ -1821,12 +1821,12 @@ def diff_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     if maps != 2 or q.shape != (tokens, 2 * heads * dim) or v_cache.shape[1:4] != (pages, kv_heads, page_size) \
             or v_cache.shape[0] * v_cache.shape[4] != vdim:
         raise KernelError("diff_attention: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
-    _lib.core().call("mrun_diff_attention", _ptr(q), _c_long(ld), _ptr(out), _ptr(k_cache), _ptr(v_cache),
-                     dtype_code(q.dtype), _ptr(block_tables), _c_int(block_tables.shape[1]), _ptr(token_slot),
-                     _ptr(positions), _c_long(pages), _c_int(tokens), _c_int(heads), _c_int(kv_heads), _c_int(dim),
-                     _c_int(vdim), _c_int(v_cache.shape[4]), _c_int(page_size), _c_float(scale), _c_float(lam),
-                     _c_float(eps), _c_float(out_scale), _c_int(window), _stream())
+    out = q.new_empty((tokens, heads * vdim))
+    _lib.core().call("mrun_diff_attention", _ptr(q), ld, _ptr(out), _ptr(k_cache), _ptr(v_cache),
+                     dtype_code(q.dtype), _ptr(block_tables), block_tables.shape[1], _ptr(token_slot),
+                     _ptr(positions), pages, tokens, heads, kv_heads, dim,
+                     vdim, v_cache.shape[4], page_size, scale, lam,
+                     eps, out_scale, window, _stream())
     return out
 
 
@@ -1837,9 +1837,9 @@ def diff_combine(maps: torch.Tensor, heads: int, vdim: int, lam: float, eps: flo
     two, chunks, tokens, row = maps.shape
     if two != 2 or row * chunks != heads * vdim:
         raise KernelError("diff_combine: sizes do not match")
-    out = torch.empty((tokens, heads * vdim), dtype=maps.dtype, device=maps.device)
-    _lib.core().call("mrun_diff_combine", _ptr(maps), _ptr(out), dtype_code(maps.dtype), _c_int(tokens), _c_int(heads),
-                     _c_int(vdim), _c_int(vdim // chunks), _c_float(lam), _c_float(eps), _c_float(out_scale), _stream())
+    out = maps.new_empty((tokens, heads * vdim))
+    _lib.core().call("mrun_diff_combine", _ptr(maps), _ptr(out), dtype_code(maps.dtype), tokens, heads,
+                     vdim, vdim // chunks, lam, eps, out_scale, _stream())
     return out
 
 
@@ -1851,13 +1851,13 @@ def table_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, chos
     _check(token_ids, "token_ids", torch.int32); _check(table, "table", torch.int32)
     tokens = token_ids.numel()
     vocab, top = table.shape
-    weights = torch.empty((tokens, experts), dtype=torch.float32, device=token_ids.device)
+    weights = token_ids.new_empty((tokens, experts), dtype=torch.float32)
     if chosen is not None:
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"table_route: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_table_route", _ptr(token_ids), _ptr(table), _ptr(weights), _ptr(chosen), _c_int(tokens),
-                     _c_int(vocab), _c_int(experts), _c_int(top), _stream())
+    _lib.core().call("mrun_table_route", _ptr(token_ids), _ptr(table), _ptr(weights), _ptr(chosen), tokens,
+                     vocab, experts, top, _stream())
     return weights
 
 
@@ -1890,13 +1890,13 @@ def clamped_glu(u: torch.Tensor, weights: Optional[torch.Tensor], blocks: int, f
         if bias.numel() != blocks * 2 * ff:
             raise KernelError(f"clamped_glu: bias has {bias.numel()} entries, a row has {blocks * 2 * ff}")
     if out is None:
-        out = torch.empty((rows, blocks * ff), dtype=u.dtype, device=u.device)
+        out = u.new_empty((rows, blocks * ff))
     lda = _strided_rows(out, "out")
     if out.shape != (rows, blocks * ff) or out.dtype != u.dtype:
         raise KernelError(f"clamped_glu: out is {tuple(out.shape)} {out.dtype}")
-    _lib.core().call("mrun_clamped_glu", _ptr(u), _c_long(ldu), _ptr(out), _c_long(lda), dtype_code(u.dtype), _ptr(weights),
-                     _c_long(ldw), _c_int(per_block), _c_int(rows), _c_int(blocks), _c_int(ff), _c_float(limit),
-                     _c_float(alpha), _c_float(up_offset), _ptr(bias), _stream())
+    _lib.core().call("mrun_clamped_glu", _ptr(u), ldu, _ptr(out), lda, dtype_code(u.dtype), _ptr(weights),
+                     ldw, per_block, rows, blocks, ff, limit,
+                     alpha, up_offset, _ptr(bias), _stream())
     return out
 
 
@@ -1925,17 +1925,17 @@ def route_grouped(logits: torch.Tensor, experts: int, top: int, groups: int, kee
         _check(correction, "correction", torch.float32)
         if correction.numel() != total:
             raise KernelError(f"route_grouped: correction has {correction.numel()} entries for {total} experts")
-    weights = torch.empty((tokens, experts), dtype=torch.float32, device=logits.device)
-    shared = torch.empty(tokens, dtype=torch.float32, device=logits.device) if columns > total else None
-    unchanged = torch.empty(tokens, dtype=torch.float32, device=logits.device) if identity else None
+    weights = logits.new_empty((tokens, experts), dtype=torch.float32)
+    shared = logits.new_empty(tokens, dtype=torch.float32) if columns > total else None
+    unchanged = logits.new_empty(tokens, dtype=torch.float32) if identity else None
     if chosen is not None:
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"route_grouped: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_route_grouped", _ptr(logits), _c_long(logits.stride(0)), _c_int(ROUTER_SCORES[score]), _ptr(correction),
-                     _ptr(weights), _ptr(unchanged), _ptr(shared), _ptr(chosen), _c_int(tokens), _c_int(experts),
-                     _c_int(identity), _c_int(top), _c_int(groups), _c_int(keep), _c_int(group_top),
-                     _c_int(1 if renormalize else 0), _c_float(scale),
-                     *((_ptr(handed_on.sums), _c_int(handed_on.shape[1]), _c_float(handed_on.eps)) if handed_on is not None
-                       else (_ptr(None), _c_int(0), _c_float(0.0))), _stream())
+    _lib.core().call("mrun_route_grouped", _ptr(logits), logits.stride(0), ROUTER_SCORES[score], _ptr(correction),
+                     _ptr(weights), _ptr(unchanged), _ptr(shared), _ptr(chosen), tokens, experts,
+                     identity, top, groups, keep, group_top,
+                     1 if renormalize else 0, scale,
+                     *((_ptr(handed_on.sums), handed_on.shape[1], handed_on.eps) if handed_on is not None
+                       else (_ptr(None), 0, 0.0)), _stream())
     return weights, shared, unchanged

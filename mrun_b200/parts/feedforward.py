@@ -73,7 +73,7 @@ class GatedMLP:
             act = ops.gemm_tc5(x, self.w_gate_up, swiglu_rows=True, activation=name)
         else:
             gate_up = ops.linear(x, self.w_gate_up, bias=self.b_gate_up)
-            act = torch.empty((gate_up.shape[0], self.spec.intermediate), dtype=gate_up.dtype, device=gate_up.device)
+            act = gate_up.new_empty((gate_up.shape[0], self.spec.intermediate))
             ops.swiglu(gate_up, act, interleaved=self.interleaved, activation=name)
         if defer_output:
             return ops.linear_or_pending(act, self.w_down, self.b_down)

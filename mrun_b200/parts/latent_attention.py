@@ -155,11 +155,11 @@ class LatentAttention:
         """The heads' outputs over keys and values made from the contexts' latents: [tokens, heads * vdim].  ``q``
         is rotated in place."""
         s, n = self.spec, len(ctx.segments)
-        k = torch.empty((n, s.heads, rows, s.dim + s.rot_dim), dtype=q.dtype, device=q.device)
+        k = q.new_empty((n, s.heads, rows, s.dim + s.rot_dim))
         latents = ops.latent_rows(cache.k, group.block_tables, ctx.seg_slot[:n], ctx.seg_kv_len[:n], rows, s.kv_rank, k, s.rot_dim)
         if self.rot_dims:
             ops.latent_rotate(q, self.position.rotation(ctx), self.rot_dims, self.pairing, s.heads, s.dim, s.rot_dim)
-        v = torch.empty((n, s.heads, rows, s.vdim), dtype=q.dtype, device=q.device)
+        v = q.new_empty((n, s.heads, rows, s.vdim))
         for i, seg in enumerate(ctx.segments):
             used = -(-(seg.pos_start + seg.q_len) // 128) * 128
             c = latents[i, :used].expand(s.heads, used, s.kv_rank)
@@ -171,7 +171,7 @@ class LatentAttention:
             pages[[seg.slot for seg in ctx.segments]] = np.arange(n, dtype=np.int32)
             table = ctx.shared["segment_pages"] = ctx.upload(pages).view(-1, 1)
         scratch = _Pages(k, v, table)
-        out = torch.empty((q.shape[0], s.heads * s.vdim), dtype=q.dtype, device=q.device)
+        out = q.new_empty((q.shape[0], s.heads * s.vdim))
         return paged_attention(q, q.stride(0), out, scratch, scratch, ctx, s.heads, s.softmax_scale, 0)
 
     def cache_need(self):
@@ -192,7 +192,7 @@ class LatentAttention:
         rot = self.position.rotation(ctx) if self.position is not None else None
         slots = group.slot_mapping if cache.writable else None
         if s.q_rank:
-            cq = torch.empty((tokens, s.q_rank), dtype=x.dtype, device=x.device)
+            cq = down.new_empty((tokens, s.q_rank))
             ops.latent_prepare(down, self.q_norm, self.kv_norm, s.eps, rot, self.rot_dims, self.pairing, slots, cq,
                                cache.k, s.q_rank, s.kv_rank, s.rot_dim)
             q = ops.linear(cq, self.w_uq)
@@ -207,15 +207,15 @@ class LatentAttention:
             if gate is not None:
                 ops.head_gate(value, gate, s.heads)
             return ops.linear_or_pending(value, self.w_o) if defer_output else ops.linear(value, self.w_o)
-        q_att = torch.empty((tokens, s.heads, width), dtype=x.dtype, device=x.device)
+        q_att = down.new_empty((tokens, s.heads, width))
         ops.linears_batched(q.unflatten(1, (s.heads, s.dim + s.rot_dim))[:, :, :s.dim], self.w_uk_t,
                             out=q_att[:, :, :s.kv_rank])
         if width > s.kv_rank:       # a rotated part, or zeros up to the row's width
             ops.latent_query(q, rot, self.rot_dims, self.pairing, q_att, s.heads, s.dim, s.rot_dim, s.kv_rank)
-        mixed = torch.empty((tokens, s.heads * width), dtype=x.dtype, device=x.device)
+        mixed = down.new_empty((tokens, s.heads * width))
         paged_attention(q_att.view(tokens, s.heads * width), s.heads * width, mixed, cache, group, ctx, s.heads,
                         s.softmax_scale, s.window or 0, value_dim=s.kv_rank)
-        value = torch.empty((tokens, s.heads, s.vdim), dtype=x.dtype, device=x.device)
+        value = down.new_empty((tokens, s.heads, s.vdim))
         ops.linears_batched(mixed.view(tokens, s.heads, width)[:, :, :s.kv_rank], self.w_uv, gate=gate, out=value)
         value = value.view(tokens, s.heads * s.vdim)
         if defer_output:

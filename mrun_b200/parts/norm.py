@@ -41,7 +41,7 @@ class RMSNorm:
         if isinstance(delta, ops.PendingPostNorm):
             # a branch output that is normed and scaled before it joins the stream: one kernel
             # norms it, adds it and norms the new rows with this norm's weight
-            out = torch.empty(resid.shape, dtype=self.act, device=resid.device)
+            out = resid.new_empty(resid.shape, dtype=self.act)
             return ops.post_norm_add(resid, delta.branch, delta.weight, delta.scale, delta.eps, self.weight,
                                      self.eps, out)
         if isinstance(delta, (ops.PendingPairNorm, ops.PendingPostLayerNorm)):
@@ -55,12 +55,12 @@ class RMSNorm:
                 scaled, delta = delta.scaled, None         # rows that join with a factor: in the norm's pass
             else:
                 delta = delta.compute()
-        out = torch.empty(resid.shape, dtype=self.act, device=resid.device)
+        out = resid.new_empty(resid.shape, dtype=self.act)
         return ops.add_rmsnorm(resid, delta, self.weight, self.eps, out, scaled=scaled)
 
     def rows_forward(self, resid: torch.Tensor, delta, rows: torch.Tensor) -> torch.Tensor:
         if isinstance(delta, ops.PendingPostNorm):
-            out = torch.empty((rows.numel(), self.size), dtype=self.act, device=resid.device)
+            out = resid.new_empty((rows.numel(), self.size), dtype=self.act)
             return ops.post_norm_add(resid, delta.branch, delta.weight, delta.scale, delta.eps, self.weight,
                                      self.eps, out, rows=rows)
         if isinstance(delta, (ops.PendingPairNorm, ops.PendingPostLayerNorm)):
@@ -68,7 +68,7 @@ class RMSNorm:
         scaled = None
         if isinstance(delta, ops.PendingLinear):
             scaled, delta = delta.scaled, ops.linear(delta.x, delta.w)
-        out = torch.empty((rows.numel(), self.size), dtype=self.act, device=resid.device)
+        out = resid.new_empty((rows.numel(), self.size), dtype=self.act)
         return ops.add_rmsnorm(resid, delta, self.weight, self.eps, out, rows=rows, scaled=scaled)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
@@ -112,7 +112,7 @@ class LayerNorm:
         return delta
 
     def add_forward(self, resid: torch.Tensor, delta):
-        out = torch.empty(resid.shape, dtype=self.act, device=resid.device)
+        out = resid.new_empty(resid.shape, dtype=self.act)
         if isinstance(delta, ops.PendingPostLayerNorm):     # a branch still to be normed itself: one kernel
             return ops.post_layernorm_add(resid, delta, self.weight, self.bias, self.eps, out)
         if isinstance(delta, ops.PendingPairNorm) and self.bias is None:    # two branches still to be normed and averaged: one kernel
@@ -121,7 +121,7 @@ class LayerNorm:
         return ops.add_layernorm(resid, delta, self.weight, self.eps, out, bias=self.bias)
 
     def rows_forward(self, resid: torch.Tensor, delta, rows: torch.Tensor) -> torch.Tensor:
-        out = torch.empty((rows.numel(), self.size), dtype=self.act, device=resid.device)
+        out = resid.new_empty((rows.numel(), self.size), dtype=self.act)
         if isinstance(delta, ops.PendingPostLayerNorm):
             return ops.post_layernorm_add(resid, delta, self.weight, self.bias, self.eps, out, rows=rows)
         if isinstance(delta, ops.PendingPairNorm) and self.bias is None:
