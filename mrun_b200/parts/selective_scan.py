@@ -73,7 +73,7 @@ class SelectiveScan:
         xz = ops.linear(x, self.w_in)
         u = ops.causal_conv(xz[:, :s.inner], self.conv_weight, cache.states["conv"], ctx, residual=False, silu=True,
                             bias=self.conv_bias)
-        if ctx.max_q_len == 1:
+        if ctx.max_q_len == 1 or u.dtype == torch.float32:    # 32-bit products: a row's bits depend on the weights' sizes, not on the step
             rbc = ops.linear(u, self.w_x)
             r, bc = rbc[:, :self.rank], rbc[:, self.rank:]
         else:
