@@ -4,28 +4,36 @@
 // worked-on scores and gated outputs, attention_score.cuh: -DMRUN_SCORED=1).  Keys may have 192 features
 // where the values have 64 or 128 and the scores are plain: Q and two stages of K and V then take 209 KB.
 //
-// One thread block per (tile of query tokens, kv head).  The tile's 128 rows are (token, query
-// head of the kv head's group) pairs, so a key/value tile read once serves the whole group.  Keys
-// are consumed 128 at a time in position order with an online softmax:
+// One thread block per (tile of query tokens, kv head), in two streams of 128 rows that take turns: while the
+// tensor cores work for one, the softmax of the other runs.  A row is a (token, query head of the kv head's group)
+// pair, so a key/value tile read once serves the whole group.  A long tile's streams have rows of their own and both
+// take every key tile; a short tile's (and all with keys of 192 features, where a second Q has no place) share
+// their rows, each takes every second key tile, and the two accumulators meet at the end.  Keys are consumed 128 at a time in
+// position order with an online softmax:
 //
-//   warps 0..7   softmax.  Tensor-memory lane r is row r; warp w and warp w + 4 share the lanes
-//                32 (w % 4) .., the first takes the row's keys 0..63 of a tile, the second keys
-//                64..127.  A thread reads its half row of S = Q·Kᵀ (tcgen05.ld), masks it, meets
-//                its partner for the row's maximum (through shared memory and a barrier of the
-//                two warps), keeps the running maximum and its half of the sum in 32-bit, and
-//                writes P = exp2(s - max) as packed bf16 into tensor memory (tcgen05.st, one of
-//                two P buffers).  It rescales its half of the row of O when the
+//   warps 0..7   softmax, four warps a stream, a thread a row (tensor-memory lane r is row r).  A thread reads its row of
+//                S = Q·Kᵀ (tcgen05.ld), masks it, keeps the running maximum and sum in 32-bit, and writes P =
+//                exp2(s - max) as packed bf16 over the scores (tcgen05.st), the first half of the keys as soon as it is there.
+//                It rescales its row of O when the
 //                maximum has grown by more than 2^8 since the last rescale (until then P is
 //                taken against the older maximum, which is exact: the final division uses the
 //                same maximum);
-//   warp 8       one lane issues the products: S = Q·Kᵀ into one of two S accumulators, up to two
-//                tiles ahead of the softmax (an accumulator is free again once the softmax has
-//                its scores in registers), and O += P[j]·V[j] as soon as P[j] is written.  P is
+//   warp 8       issues the products: O += P[j]·V[j] in halves as P is written, then the stream's next S = Q·Kᵀ
+//                over the same columns.  P is
 //                read from tensor memory, Q, K and V from shared memory, V as the MN-major
 //                operand (its rows are keys, as the cache stores them);
 //   warp 9       brings K tiles from the pages into a ring of two stages by TMA: a lane per page
-//                of the tile looks the page up in the block table and copies its rows as
+//                of the tile looks the page up in the block table, a tile ahead, and copies its rows as
 //                [rows x 64] boxes with the 128-byte swizzle; warp 10 the V tiles likewise.
+//
+// Bound by the chain of a stream's row (scores out of tensor memory, maximum, exponentials, P back, two products), of which two
+// run side by side: a tile of 128 keys for 256 rows of 128 features takes 1.9 us (2,048 cycles of MMAs and as many of the
+// special-function units would be 1.1), for 128 shared rows 1.25.  1,531 tokens behind 9,000, 32 heads over 8, B200: 251 us,
+// 0.98 PFLOP/s; half rows a thread, all eight warps on one tile of 128 rows at a time, 296 us, 1.28 a tile.
+// What the parts gave, us a tile of a pair: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
+// step); one elected lane, every wait but P's taken before, and both products issued in a row 2.1 -> 1.9; P in halves 2.3 ->
+// 2.25; the page looked up ahead 1.40 -> 1.27 (shared rows).  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 ->
+// 1.96, a third stage of K or V nothing.
 //
 // The roles hand tiles to one another through mbarriers; every wait is bounded by a cycle budget.
 // When a wait runs out the block records a code in the status word, every role stops, the block
@@ -73,20 +81,22 @@ using namespace tc5;
 
 constexpr int D = MRUN_HEAD_DIM, DV = MRUN_VALUE_DIM;
 constexpr bool SCORED = MRUN_SCORED;
-constexpr int ROWS = 128;                    // query rows per block = MMA M
+constexpr int ROWS = 128;                    // query rows per stream = MMA M
 constexpr int KEYS = 128;                    // keys per tile = N of the first product, K of the second
 constexpr int SPANS_D = D / 64, SPANS_V = DV / 64;      // 64-wide spans of the head dimensions
 constexpr int SPAN_BYTES = 128 * 128;        // one swizzled tile of 128 rows x 64 bf16
 constexpr int K_BYTES = SPANS_D * SPAN_BYTES;           // one stage of K: 128 keys x D
 constexpr int V_BYTES = SPANS_V * SPAN_BYTES;           // one stage of V: 128 keys x DV
-constexpr int Q_BYTES = SPANS_D * SPAN_BYTES;
-constexpr int SMEM_BYTES = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + 1024;                // Q, two stages of K and of V
-constexpr int SOFTMAX_WARPS = 8, SOFTMAX_THREADS = SOFTMAX_WARPS * 32;
+constexpr int Q_BYTES = SPANS_D * SPAN_BYTES;           // the rows of one stream
+constexpr int MAX_Q = D <= 128 ? 2 : 1;      // streams with rows of their own that fit beside the stages
+constexpr int SMEM_BYTES = MAX_Q * Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + 1024;        // Q, two stages of K and of V
+constexpr int SOFTMAX_WARPS = 8, SOFTMAX_THREADS = SOFTMAX_WARPS * 32, STREAM_WARPS = 4;
 constexpr int MMA_WARP = 8, K_WARP = 9, V_WARP = 10;
-constexpr int THREADS = SOFTMAX_THREADS + 3 * 32;                        // 352
-constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256) P0 [256,320) P1 [320,384) O [384, 384 + DV)
-constexpr unsigned P_COL = 256, O_COL = 384;
-constexpr int O_HALF = DV / 2;                // columns of O a thread of a pair looks after
+constexpr int THREADS = SOFTMAX_THREADS + 4 * 32;                        // 384: registers are dealt to four warps together
+constexpr int SOFTMAX_REGISTERS = 216, OTHER_REGISTERS = 72, LAUNCH_REGISTERS = 168;
+static_assert(SOFTMAX_THREADS * SOFTMAX_REGISTERS + 128 * OTHER_REGISTERS <= THREADS * LAUNCH_REGISTERS, "more registers than the block has");
+constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256) O0 [256, 256 + DV) O1 [384, 384 + DV); P lies on its S
+constexpr unsigned O_COL = 256;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.f;          // log2 of the growth of a row maximum that forces a rescale
 constexpr long long WAIT_CYCLES = 3000000000LL;         // about 1.5 s at 2 GHz
@@ -112,7 +122,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// The two warps that share a quarter of the rows meet here (barrier 1 + quarter, 64 threads).
+// The two warps that share a quarter of the lanes meet here (barrier 1 + quarter, 64 threads).
 __device__ __forceinline__ void pair_sync(int quarter) {
     asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
 }
@@ -120,7 +130,7 @@ __device__ __forceinline__ void pair_sync(int quarter) {
 struct Barriers {
     unsigned long long q_full;
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];
-    unsigned long long s_full[2], s_empty[2], p_full[2], pv_done;
+    unsigned long long s_full[2], p_full[2][2], o_full;              // [stream], [stream][half of the keys]
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -133,21 +143,22 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* q_tile = base;
-    unsigned char* k_stages = q_tile + Q_BYTES;
+    unsigned char* k_stages = q_tile + MAX_Q * Q_BYTES;
     unsigned char* v_stages = k_stages + 2 * K_BYTES;
+
     __shared__ Barriers bars;
     __shared__ unsigned tmem_base_slot;
     __shared__ int aborted;
-    __shared__ float pair_max[2][2][ROWS];               // [tile parity][half][row]: the halves' maxima
-    __shared__ float pair_sum[2][ROWS];                  // [half][row]: the halves' sums, at the end
+    __shared__ float row_max[2][ROWS], row_sum[2][ROWS];     // of the two streams, where they share their rows
 
     // Blocks start in the order of their index, x first: all kv heads of the first tile of the
-    // list, which the host sorted by falling context length, then all of the second, ...
+    // list, which the host sorted by falling work, then all of the second, ...
     const int tile = blockIdx.y, kvh = blockIdx.x;
     const int group = heads / kv_heads;
     const int tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_rows = ntok * group;
+    const int per_stream = ROWS / group;                 // tokens
+    const bool apart = MAX_Q == 2 && ntok > per_stream;  // the streams have rows of their own and take every key tile
     // tokens of a tile are consecutive positions of one request
     const int pos_first = positions[tok0], pos_last = pos_first + ntok - 1;
     const int lo_tile = mrun::first_visible(pos_first, window);
@@ -162,10 +173,10 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             mbar_init(&bars.k_empty[s], 1);
             mbar_init(&bars.v_empty[s], 1);
             mbar_init(&bars.s_full[s], 1);
-            mbar_init(&bars.s_empty[s], SOFTMAX_WARPS);
-            mbar_init(&bars.p_full[s], SOFTMAX_WARPS);
+            mbar_init(&bars.p_full[s][0], STREAM_WARPS);
+            mbar_init(&bars.p_full[s][1], STREAM_WARPS);
         }
-        mbar_init(&bars.pv_done, 1);
+        mbar_init(&bars.o_full, 1);
         aborted = 0;
         mbar_init_fence();
     }
@@ -181,18 +192,19 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     const unsigned tmem_base = tmem_base_slot;
 
     if (warp < SOFTMAX_WARPS) {
-        // ------------------------------------------------------------------ softmax, half rows
-        const int quarter = warp & 3, half = warp >> 2;
+        // ------------------------------------------------------------------ softmax, a row a thread
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGISTERS));
+        const int quarter = warp & 3, stream = warp >> 2;
         const int row = quarter * 32 + lane;                          // 0..127
         const unsigned lane_base = tmem_base + ((unsigned)(quarter * 32) << 16);
-        // q rows: row r = (token r / group, head kvh * group + r % group); rows past n_rows are zero
-        for (int c = threadIdx.x; c < ROWS * (D / 8); c += SOFTMAX_THREADS) {
-            const int r = c / (D / 8), chunk = c - r * (D / 8);
-            const bool valid = r < n_rows;
+        // q rows: row r = (token r / group, head kvh * group + r % group); rows past the stream's are zero
+        for (int c = threadIdx.x; c < (apart ? 2 : 1) * ROWS * (D / 8); c += SOFTMAX_THREADS) {
+            const int part = c / (ROWS * (D / 8)), in = c - part * (ROWS * (D / 8));
+            const int r = in / (D / 8), chunk = in - r * (D / 8), token = part * per_stream + r / group;
+            const bool valid = r < per_stream * group && token < ntok;
             const bf16* src = q;
-            if (valid)
-                src = q + (size_t)(tok0 + r / group) * q_stride + (size_t)(kvh * group + r % group) * D + chunk * 8;
-            cp_async_16(q_tile + (chunk >> 3) * SPAN_BYTES + swizzled_offset(r, chunk & 7), src, valid);
+            if (valid) src = q + (size_t)(tok0 + token) * q_stride + (size_t)(kvh * group + r % group) * D + chunk * 8;
+            cp_async_16(q_tile + part * Q_BYTES + (chunk >> 3) * SPAN_BYTES + swizzled_offset(r, chunk & 7), src, valid);
         }
         cp_async_commit();
         cp_async_wait<0>();
@@ -200,117 +212,99 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.q_full);
 
-        const int row_pos = row < n_rows ? pos_first + row / group : -1;      // -1: padding row
+        const int token0 = apart ? stream * per_stream : 0;                       // the stream's tokens within the tile
+        const int tokens = min(ntok - token0, per_stream);
+        const int n_rows = tokens * group;
+        const int first_pos = pos_first + token0, last_pos = first_pos + tokens - 1;
+        const int row_pos = row < n_rows ? first_pos + row / group : -1;      // -1: padding row
         const int row_lo = mrun::first_visible(row_pos, window);
-        // the tile's last row sees the most recent keys, its first row the oldest
-        const int lo_last = mrun::first_visible(pos_last, window);
+        // the stream's last row sees the most recent keys, its first row the oldest
+        const int lo_last = mrun::first_visible(last_pos, window);
+        const int head = kvh * group + row % group;
         mrun::ScoreRow form_row = {};
         if constexpr (SCORED) form_row = mrun::score_row(form, scale_log2 / LOG2E, row_pos, kvh * group + min(row, n_rows - 1) % group);
-        float m_used = -INFINITY, l = 0.f;                           // l: this half's share of the row's sum
+        float m_used = -INFINITY, l = 0.f;
         bool alive = true;
-        // A warp that gave up on a wait still walks through the remaining tiles, doing nothing but
-        // meeting its partner at every barrier, so that no warp is left waiting at one.
-        for (int j = 0; j < n_tiles; ++j) {
-            const int buf = j & 1;
-            if (alive && !__all_sync(0xffffffffu, mbar_wait(&bars.s_full[buf], (j >> 1) & 1, WAIT_CYCLES, &aborted))) alive = false;
-            const int key_base = (first_block + j) * KEYS + half * 64;        // of this thread's first score
-            // every row of the block sees every key of the tile: no comparisons
-            const bool need_mask = (first_block + j) * KEYS + KEYS - 1 > pos_first || (first_block + j) * KEYS < lo_last ||
-                                   n_rows < ROWS;
-            float sc[64];
+        const int mine = apart ? n_tiles : (n_tiles + 1 - stream) / 2;        // this stream's items
+        for (int it = 0; it < mine; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&bars.s_full[stream], it & 1, WAIT_CYCLES, &aborted))) { alive = false; break; }
+            const int key_base = (first_block + (apart ? it : 2 * it + stream)) * KEYS;
+            // every row of the stream sees every key of the tile: no comparisons
+            const bool need_mask = key_base + KEYS - 1 > first_pos || key_base < lo_last || n_rows < ROWS;
+            float sc[KEYS];
             float mx = -INFINITY;
-            if (alive) {
-                tc_fence_after();
-                // the half row's 64 scores, read once
-                unsigned raw[64];
-                {
-                    unsigned (&lo32)[32] = *reinterpret_cast<unsigned (*)[32]>(&raw[0]);
-                    unsigned (&hi32)[32] = *reinterpret_cast<unsigned (*)[32]>(&raw[32]);
-                    tmem_load32_start(lane_base + buf * KEYS + half * 64, lo32);
-                    tmem_load32_start(lane_base + buf * KEYS + half * 64 + 32, hi32);
-                    tmem_load_wait();
-                }
-                // the scores are in registers: the product after next may overwrite the accumulator
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.s_empty[buf]);
+            tc_fence_after();
+            {
+                unsigned raw[KEYS];
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
+                for (int c = 0; c < KEYS; c += 32)
+                    tmem_load32_start(lane_base + stream * KEYS + c, *reinterpret_cast<unsigned (*)[32]>(&raw[c]));
+                tmem_load_wait();
+#pragma unroll
+                for (int i = 0; i < KEYS; ++i) {
                     pin(raw[i]);
                     sc[i] = __uint_as_float(raw[i]);
                 }
-                if constexpr (SCORED) {
-                    // scores in base-2 units from here on: two a step where the polynomial serves (every
-                    // row of the warp alike), then the bias, an entry a distance only near the query
-                    if (__all_sync(0xffffffffu, form_row.small)) {
-                        const float2 factor2 = make_float2(form_row.factor, form_row.factor);
-                        const float2 cap2 = make_float2(form_row.cap2, form_row.cap2);
-                        const float2 far2 = make_float2(form_row.far_bias, form_row.far_bias);
+            }
+            if constexpr (SCORED) {
+                // scores in base-2 units from here on: two a step where the polynomial serves (every
+                // row of the warp alike), then the bias, an entry a distance only near the query
+                if (__all_sync(0xffffffffu, form_row.small)) {
+                    const float2 factor2 = make_float2(form_row.factor, form_row.factor);
+                    const float2 cap2 = make_float2(form_row.cap2, form_row.cap2);
+                    const float2 far2 = make_float2(form_row.far_bias, form_row.far_bias);
 #pragma unroll
-                        for (int i = 0; i < 64; i += 2) {
-                            const float2 th = mrun::tanh_small2(__fmul2_rn(make_float2(sc[i], sc[i + 1]), factor2));
-                            const float2 v = __ffma2_rn(th, cap2, far2);
-                            sc[i] = v.x; sc[i + 1] = v.y;
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 64; ++i) sc[i] = mrun::capped_score(form_row, sc[i]) + form_row.far_bias;
-                    }
-                    if (form.bias != nullptr && pos_first - (key_base + 63) < form.bias_len - 1) {
-                        // every entry as its difference from the far one, which the scores hold already
-                        const float* table = form_row.bias;
-                        const int distance = row_pos - key_base;
-#pragma unroll
-                        for (int i = 0; i < 64; ++i)
-                            sc[i] += fmaf(__ldg(table + min(max(distance - i, 0), form_row.bias_last)), LOG2E, -form_row.far_bias);
-                    }
-                }
-                // the largest raw score first (the scale is positive, so it scales the maximum
-                // alike); masked scores become -inf and later give p = 0
-                if (need_mask) {
-                    const int lo_rel = row_lo - key_base, hi_rel = row_pos - key_base;
-#pragma unroll
-                    for (int i = 0; i < 64; ++i) {
-                        if (i > hi_rel || i < lo_rel) sc[i] = -INFINITY;
-                        mx = fmaxf(mx, sc[i]);
+                    for (int i = 0; i < KEYS; i += 2) {
+                        const float2 th = mrun::tanh_small2(__fmul2_rn(make_float2(sc[i], sc[i + 1]), factor2));
+                        const float2 v = __ffma2_rn(th, cap2, far2);
+                        sc[i] = v.x; sc[i + 1] = v.y;
                     }
                 } else {
-                    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                    for (int i = 0; i < 64; i += 4) {
-                        mx4[0] = fmaxf(mx4[0], sc[i]); mx4[1] = fmaxf(mx4[1], sc[i + 1]);
-                        mx4[2] = fmaxf(mx4[2], sc[i + 2]); mx4[3] = fmaxf(mx4[3], sc[i + 3]);
-                    }
-                    mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                    for (int i = 0; i < KEYS; ++i) sc[i] = mrun::capped_score(form_row, sc[i]) + form_row.far_bias;
+                }
+                if (form.bias != nullptr && first_pos - (key_base + KEYS - 1) < form.bias_len - 1) {
+                    // every entry as its difference from the far one, which the scores hold already
+                    const float* table = form_row.bias;
+                    const int distance = row_pos - key_base;
+#pragma unroll
+                    for (int i = 0; i < KEYS; ++i)
+                        sc[i] += fmaf(__ldg(table + min(max(distance - i, 0), form_row.bias_last)), LOG2E, -form_row.far_bias);
                 }
             }
-            // the other half of the row
-            pair_max[buf][half][row] = mx;
-            pair_sync(quarter);
-            if (!alive) continue;
-            mx = fmaxf(mx, pair_max[buf][half ^ 1][row]);
+            // the largest raw score first (the scale is positive, so it scales the maximum
+            // alike); masked scores become -inf and later give p = 0
+            if (need_mask) {
+                const int lo_rel = row_lo - key_base, hi_rel = row_pos - key_base;
+#pragma unroll
+                for (int i = 0; i < KEYS; ++i) {
+                    if (i > hi_rel || i < lo_rel) sc[i] = -INFINITY;
+                }
+            }
+            {
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int i = 0; i < KEYS; i += 8) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(fmaxf(mx4[c], sc[i + 2 * c]), sc[i + 2 * c + 1]);
+                }
+                mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            }
             if constexpr (!SCORED) mx *= scale_log2;
-            // the maximum the probabilities are taken against moves only by large steps; both
-            // halves of a row decide alike, from the same numbers
+            // the maximum the probabilities are taken against moves only by large steps
             float m_new = m_used;
             if (mx > m_used + RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY)) m_new = mx;
             const bool moved = m_new != m_used && m_used != -INFINITY;       // O holds something to rescale
-            const bool warp_moved = __any_sync(0xffffffffu, moved);
-            if (warp_moved) {
-                // O belongs to the second product of the tile before until that has finished
-                if (j > 0 && !__all_sync(0xffffffffu, mbar_wait(&bars.pv_done, (j - 1) & 1, WAIT_CYCLES, &aborted))) {
-                    alive = false;
-                    continue;
-                }
-                tc_fence_after();
+            if (__any_sync(0xffffffffu, moved)) {
+                // the second product of this stream's item before was issued before this one's first, so it has finished
                 const float corr = moved ? exp2f(m_used - m_new) : 1.f;
 #pragma unroll 1
-                for (int c = 0; c < O_HALF; c += 32) {
-                    float v[32];
-                    tmem_load32(lane_base + O_COL + half * O_HALF + c, v);
+                for (int c = 0; c < DV; c += 16) {
+                    float v[16];
+                    tmem_load16(lane_base + O_COL + stream * 128 + c, v);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] *= corr;
-                    tmem_store32(lane_base + O_COL + half * O_HALF + c, v);
+                    for (int i = 0; i < 16; ++i) v[i] *= corr;
+                    tmem_store16_start(lane_base + O_COL + stream * 128 + c, v);
                 }
                 l *= corr;
             }
@@ -318,158 +312,204 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             // p = 2^(s * scale - m): one fused multiply-add and one special-function call a score.
             // Masked scores are -inf and give 0; a row that has seen nothing yet keeps m_used = -inf.
             const float m_sub = m_used == -INFINITY ? 0.f : -m_used;
-            // Two scores an instruction where the hardware has one (fma.f32x2, add.f32x2): these
-            // warps are bound by the instructions they issue.
+            // Two scores an instruction where the hardware has one (fma.f32x2, add.f32x2)
             const float unit = SCORED ? 1.f : scale_log2;
             const float2 scale2 = make_float2(unit, unit), m_sub2 = make_float2(m_sub, m_sub);
             float2 sums = make_float2(0.f, 0.f);
-            float packed[32];                                         // two bf16 a word, even key low
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
-                const float2 x = __ffma2_rn(make_float2(sc[i], sc[i + 1]), scale2, m_sub2);
-                const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                sums = __fadd2_rn(sums, p);
-                packed[i >> 1] = __uint_as_float(pack_bf16(p.x, p.y));
+            for (int c = 0; c < KEYS; c += 32) {
+                float packed[16];                                     // two bf16 a word, even key low
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    const float2 x = __ffma2_rn(make_float2(sc[c + i], sc[c + i + 1]), scale2, m_sub2);
+                    const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                    sums = __fadd2_rn(sums, p);
+                    packed[i >> 1] = __uint_as_float(pack_bf16(p.x, p.y));
+                }
+                tmem_store16_start(lane_base + stream * KEYS + c / 2, packed);      // on this row's scores, which are in registers
+                if (c % 64 == 32) {                                   // half of the second product may begin
+                    tmem_store_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars.p_full[stream][c / 64]);
+                }
             }
             l += sums.x + sums.y;
-            // the P buffer of this tile was read by the second product of the tile before last
-            if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&bars.v_empty[buf], ((j >> 1) - 1) & 1, WAIT_CYCLES, &aborted))) {
-                alive = false;
-                continue;
-            }
-            tmem_store32(lane_base + P_COL + buf * 64 + half * 32, packed);       // this half's keys: words 32 half ..
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars.p_full[buf]);
         }
         // a warp leaves the loop as a whole, so every lane takes part in what follows
-        if (alive && !__all_sync(0xffffffffu, mbar_wait(&bars.pv_done, (n_tiles - 1) & 1, WAIT_CYCLES, &aborted))) alive = false;
+        if (alive && !__all_sync(0xffffffffu, mbar_wait(&bars.o_full, 0, WAIT_CYCLES, &aborted))) alive = false;
         if (!alive) {
             if (!*(volatile int*)&aborted) atomicExch(status, STATUS_SOFTMAX);
             atomicExch(&aborted, 1);
         }
-        // the row's sum is the two halves' (the partner may have given up: it still comes here)
-        pair_sum[half][row] = l;
-        pair_sync(quarter);
+        // Streams that share their rows meet (the other may have given up: it still comes here): each writes one half of the
+        // columns, both accumulators against the larger of the two maxima.
+        float m_all = m_used, scale[2] = {stream == 0 ? 1.f : 0.f, stream == 0 ? 0.f : 1.f};
+        int col0 = 0, col1 = DV;
+        if (!apart) {
+            row_max[stream][row] = m_used;
+            row_sum[stream][row] = l;
+            pair_sync(quarter);
+            const float m0 = row_max[0][row], m1 = row_max[1][row];
+            m_all = fmaxf(m0, m1);
+            scale[0] = m0 == -INFINITY ? 0.f : exp2f(m0 - m_all);
+            scale[1] = m1 == -INFINITY ? 0.f : exp2f(m1 - m_all);
+            l = row_sum[0][row] * scale[0] + row_sum[1][row] * scale[1];
+            col0 = stream * (DV / 2);
+            col1 = col0 + DV / 2;
+        }
         if (alive) {
             tc_fence_after();
-            const float total = with_sink(l + pair_sum[half ^ 1][row], m_used, sinks, kvh * group + row % group);
+            const float total = with_sink(l, m_all, sinks, head);
             const float inv = total > 0.f ? 1.f / total : 0.f;
-            const int col = (kvh * group + row % group) * DV + half * O_HALF;
-            bf16* dst = out + (size_t)(tok0 + row / group) * (SCORED ? form.out_stride : (long)heads * DV) + col;
+            const int token = tok0 + token0 + row / group;
+            bf16* dst = out + (size_t)token * (SCORED ? form.out_stride : (long)heads * DV) + head * DV;
+            // an accumulator that no product wrote holds anything
+            const bool use[2] = {apart ? stream == 0 : true, apart ? stream == 1 : n_tiles > 1};
 #pragma unroll 1
-            for (int c = 0; c < O_HALF; c += 32) {
-                float v[32];
-                tmem_load32(lane_base + O_COL + half * O_HALF + c, v);       // every lane of the warp takes part
+            for (int c = col0; c < col1; c += 16) {
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = 0.f;
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+                    if (use[part]) {
+                        float o[16];
+                        tmem_load16(lane_base + O_COL + part * 128 + c, o);       // every lane of the warp takes part
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = fmaf(o[i], scale[part], v[i]);
+                    }
                 if (row < n_rows) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] *= inv;
-                    if constexpr (SCORED) mrun::gate_outputs<32>(form, tok0 + row / group, col + c, v);
+                    for (int i = 0; i < 16; ++i) v[i] *= inv;
+                    if constexpr (SCORED) mrun::gate_outputs<16>(form, token, head * DV + c, v);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
+                    for (int k = 0; k < 2; ++k)
                         *reinterpret_cast<uint4*>(dst + c + 8 * k) =
                             make_uint4(pack_bf16(v[8 * k], v[8 * k + 1]), pack_bf16(v[8 * k + 2], v[8 * k + 3]),
                                        pack_bf16(v[8 * k + 4], v[8 * k + 5]), pack_bf16(v[8 * k + 6], v[8 * k + 7]));
                 }
             }
         }
-    } else if (warp == MMA_WARP) {
-        // ---------------------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGISTERS));
+        if (warp == MMA_WARP) {
+            // ------------------------------------------------------------------------ MMA issuer
             constexpr unsigned idesc_qk = instruction_descriptor(ROWS, KEYS);
             constexpr unsigned idesc_pv = instruction_descriptor(ROWS, DV, true);
-            // The operand descriptors of stage 0, made once: this warp shares its scheduler with
-            // two softmax warps, so every instruction it spends between two products delays them.
-            // Stage 1 lies K_BYTES (V_BYTES) further (the address field counts 16-byte units).
-            unsigned long long q_desc[D / 16], k_desc[D / 16], v_desc[KEYS / 16];
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                const int off = (kk >> 2) * SPAN_BYTES + (kk & 3) * 32;       // 32 bytes further along d per step
-                q_desc[kk] = smem_descriptor(q_tile + off);
-                k_desc[kk] = smem_descriptor(k_stages + off);
-            }
-#pragma unroll
-            for (int kk = 0; kk < KEYS / 16; ++kk)                            // sixteen rows (two groups) further per step
-                v_desc[kk] = smem_descriptor(v_stages + kk * 2048, SPAN_BYTES, 1024);
-            constexpr unsigned long long K_STEP = K_BYTES >> 4, V_STEP = V_BYTES >> 4;
-            bool alive = mbar_wait(&bars.q_full, 0, WAIT_CYCLES, &aborted);
-            auto issue_qk = [&](int j) -> bool {
-                const int s = j & 1;
-                if (!mbar_wait(&bars.k_full[s], (j >> 1) & 1, WAIT_CYCLES, &aborted)) return false;
-                if (j >= 2 && !mbar_wait(&bars.s_empty[s], ((j >> 1) - 1) & 1, WAIT_CYCLES, &aborted)) return false;
-                tc_fence_after();
-                const unsigned long long step = s * K_STEP;
-#pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk)
-                    umma_bf16(tmem_base + s * KEYS, q_desc[kk], k_desc[kk] + step, idesc_qk, kk > 0 ? 1u : 0u);
-                umma_commit(&bars.s_full[s]);
-                umma_commit(&bars.k_empty[s]);
-                return true;
+            const unsigned long long q_desc = smem_descriptor(q_tile), k_desc = smem_descriptor(k_stages);
+            const unsigned long long v_desc = smem_descriptor(v_stages, SPAN_BYTES, 1024);
+            auto wait = [&](unsigned long long* bar, unsigned parity) {
+                return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, WAIT_CYCLES, &aborted));
             };
-            // the first products run two tiles ahead of the softmax, the second follow it
-            if (alive) alive = issue_qk(0);
-            if (alive && n_tiles > 1) alive = issue_qk(1);
-            for (int j = 0; alive && j < n_tiles; ++j) {
-                const int s = j & 1;
-                if (!mbar_wait(&bars.v_full[s], (j >> 1) & 1, WAIT_CYCLES, &aborted)) { alive = false; break; }
-                if (!mbar_wait(&bars.p_full[s], (j >> 1) & 1, WAIT_CYCLES, &aborted)) { alive = false; break; }
-                tc_fence_after();
-                const unsigned long long step = s * V_STEP;
+            // Item i is stream i & 1's: key tile i / 2 (apart) or i.  Descriptors further on differ in their address field, which
+            // counts 16-byte units.
+            const int n_items = apart ? 2 * n_tiles : n_tiles;
+            auto issue_qk = [&](int stream, int s) {                      // by the elected lane; s: K's stage
+                const unsigned long long qd = q_desc + (apart ? stream * (Q_BYTES >> 4) : 0), kd = k_desc + s * (K_BYTES >> 4);
 #pragma unroll
-                for (int kk = 0; kk < KEYS / 16; ++kk)                        // P: eight columns (16 keys) further per step
-                    umma_bf16_a_tmem(tmem_base + O_COL, tmem_base + P_COL + s * 64 + kk * 8, v_desc[kk] + step, idesc_pv,
-                                     (j > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(&bars.v_empty[s]);
-                umma_commit(&bars.pv_done);
-                if (j + 2 < n_tiles && !issue_qk(j + 2)) { alive = false; break; }
+                for (int kk = 0; kk < D / 16; ++kk) {                     // 32 bytes further along d per step
+                    const int off = ((kk >> 2) * SPAN_BYTES + (kk & 3) * 32) >> 4;
+                    umma_bf16(tmem_base + stream * KEYS, qd + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
+                }
+                umma_commit(&bars.s_full[stream]);
+                if (!apart || stream == 1) umma_commit(&bars.k_empty[s]);
+            };
+            bool alive = wait(&bars.q_full, 0);
+            for (int i = 0; alive && i < 2 && i < n_items; ++i) {
+                const int s = apart ? 0 : i;
+                alive = wait(&bars.k_full[s], 0);
+                if (!alive) break;
+                if (elect_one()) issue_qk(i, s);
+                __syncwarp();
+            }
+            for (int i = 0; alive && i < n_items; ++i) {
+                const int stream = i & 1, j = apart ? i >> 1 : i, s = j & 1;
+                const int next = apart ? j + 1 : j + 2, next_s = next & 1;        // the key tile of the stream's next item
+                const bool more = i + 2 < n_items;
+                const unsigned long long vd = v_desc + s * (V_BYTES >> 4);
+                // P comes last, so what waits for it goes on at once; the stream's next scores go where its P lies, behind the
+                // product that reads it
+                if (!wait(&bars.v_full[s], (j >> 1) & 1) || (more && !wait(&bars.k_full[next_s], (next >> 1) & 1)) ||
+                    !wait(&bars.p_full[stream][0], (i >> 1) & 1)) {
+                    alive = false;
+                    break;
+                }
+                auto issue_pv = [&](int half) {                           // P: eight columns (16 keys) further per step; V: sixteen rows
+#pragma unroll
+                    for (int kk = 0; kk < KEYS / 32; ++kk) {
+                        const int at = half * (KEYS / 32) + kk;
+                        umma_bf16_a_tmem(tmem_base + O_COL + stream * 128, tmem_base + stream * KEYS + at * 8, vd + at * (2048 >> 4), idesc_pv,
+                                         (i > 1 || at > 0) ? 1u : 0u);
+                    }
+                };
+                tc_fence_after();
+                if (elect_one()) issue_pv(0);
+                __syncwarp();
+                if (!wait(&bars.p_full[stream][1], (i >> 1) & 1)) { alive = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
+                    issue_pv(1);
+                    if (!apart || stream == 1) umma_commit(&bars.v_empty[s]);
+                    if (more) issue_qk(stream, next_s);
+                    if (i + 1 == n_items) umma_commit(&bars.o_full);
+                }
+                __syncwarp();
             }
             if (!alive) {
                 if (!*(volatile int*)&aborted) atomicExch(status, STATUS_MMA);
                 atomicExch(&aborted, 1);
             }
-        }
-    } else {
-        // ------------------------------------------------------------------------------- loaders
-        const bool keys_role = warp == K_WARP;                        // one warp for K, one for V
-        const CUtensorMap* map = keys_role ? &map_k : &map_v;
-        unsigned char* stages = keys_role ? k_stages : v_stages;
-        unsigned long long* full = keys_role ? bars.k_full : bars.v_full;
-        unsigned long long* empty = keys_role ? bars.k_empty : bars.v_empty;
-        const int* table = block_tables + (size_t)token_slot[tok0] * max_blocks;
-        // pages of up to 128 keys: 128 / page_size boxes of page_size rows; larger pages: one box
-        const int box_rows = page_size < KEYS ? page_size : KEYS;
-        const int boxes = KEYS / box_rows;
-        bool alive = true;
-        for (int j = 0; j < n_tiles; ++j) {
-            const int s = j & 1;
-            const bool free_now = j < 2 || mbar_wait(&empty[s], ((j >> 1) - 1) & 1, WAIT_CYCLES, &aborted);
-            if (!__all_sync(0xffffffffu, free_now)) { alive = false; break; }
-            const int key0 = (first_block + j) * KEYS;
-            unsigned char* stage = stages + s * (keys_role ? K_BYTES : V_BYTES);
-            // a lane's boxes: lane, lane + 32, ...  It announces their bytes, then copies them.
-            unsigned bytes = 0;
-            for (int b = lane; b < boxes; b += 32) {
-                const int first_key = key0 + b * box_rows;
-                if (first_key <= pos_last && first_key + box_rows - 1 >= lo_tile && table[first_key >> page_shift] >= 0)
-                    bytes += (unsigned)(box_rows * (keys_role ? D : DV) * 2);
-            }
-            if (bytes) mbar_expect_tx(&full[s], bytes);
-            else mbar_arrive(&full[s]);
-            for (int b = lane; b < boxes; b += 32) {
-                const int first_key = key0 + b * box_rows;
-                if (first_key > pos_last || first_key + box_rows - 1 < lo_tile) continue;
-                const int page = table[first_key >> page_shift];
-                if (page < 0) continue;
+        } else if (warp <= V_WARP) {
+            // --------------------------------------------------------------------------- loaders
+            const bool keys_role = warp == K_WARP;                        // one warp for K, one for V
+            const CUtensorMap* map = keys_role ? &map_k : &map_v;
+            unsigned char* stages = keys_role ? k_stages : v_stages;
+            unsigned long long* full = keys_role ? bars.k_full : bars.v_full;
+            unsigned long long* empty = keys_role ? bars.k_empty : bars.v_empty;
+            const int* table = block_tables + (size_t)token_slot[tok0] * max_blocks;
+            // pages of up to 128 keys: 128 / page_size boxes of page_size rows; larger pages: one box
+            const int box_rows = page_size < KEYS ? page_size : KEYS;
+            const int boxes = KEYS / box_rows;
+            // The pages of a lane's boxes (lane, lane + 32, ...), looked up a tile ahead: -1 where nothing is to be copied.
+            constexpr int MAX_BOXES = KEYS / 32;
+            int pages[MAX_BOXES];
+            auto look_up = [&](int j) {
 #pragma unroll
-                for (int h = 0; h < (SPANS_D > SPANS_V ? SPANS_D : SPANS_V); ++h)
-                    if (h < (keys_role ? SPANS_D : SPANS_V))
-                        tma_load_4d(stage + h * SPAN_BYTES + b * box_rows * 128, map, h * 64,
-                                first_key & (page_size - 1), kvh, page, &full[s]);
+                for (int u = 0; u < MAX_BOXES; ++u) {
+                    const int b = lane + 32 * u, first_key = (first_block + j) * KEYS + b * box_rows;
+                    const bool wanted = j < n_tiles && b < boxes && first_key <= pos_last && first_key + box_rows - 1 >= lo_tile;
+                    pages[u] = wanted ? table[first_key >> page_shift] : -1;
+                }
+            };
+            look_up(0);
+            bool alive = true;
+            for (int j = 0; j < n_tiles; ++j) {
+                const int s = j & 1;
+                const bool free_now = j < 2 || mbar_wait(&empty[s], ((j >> 1) - 1) & 1, WAIT_CYCLES, &aborted);
+                if (!__all_sync(0xffffffffu, free_now)) { alive = false; break; }
+                unsigned char* stage = stages + s * (keys_role ? K_BYTES : V_BYTES);
+                unsigned bytes = 0;                               // a lane announces its boxes' bytes, then copies them
+#pragma unroll
+                for (int u = 0; u < MAX_BOXES; ++u) bytes += pages[u] >= 0 ? (unsigned)(box_rows * (keys_role ? D : DV) * 2) : 0u;
+                if (bytes) mbar_expect_tx(&full[s], bytes);
+                else mbar_arrive(&full[s]);
+#pragma unroll
+                for (int u = 0; u < MAX_BOXES; ++u) {
+                    if (pages[u] < 0) continue;
+                    const int b = lane + 32 * u, first_key = (first_block + j) * KEYS + b * box_rows;
+#pragma unroll
+                    for (int h = 0; h < (SPANS_D > SPANS_V ? SPANS_D : SPANS_V); ++h)
+                        if (h < (keys_role ? SPANS_D : SPANS_V))
+                            tma_load_4d(stage + h * SPAN_BYTES + b * box_rows * 128, map, h * 64,
+                                        first_key & (page_size - 1), kvh, pages[u], &full[s]);
+                }
+                look_up(j + 1);
             }
-        }
-        if (!alive) {
-            if (!*(volatile int*)&aborted) atomicExch(status, STATUS_LOADER);
-            atomicExch(&aborted, 1);
+            if (!alive) {
+                if (!*(volatile int*)&aborted) atomicExch(status, STATUS_LOADER);
+                atomicExch(&aborted, 1);
+            }
         }
     }
 
@@ -488,13 +528,17 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 
 #endif  // MRUN_ATTN_TC5
 
-// 1 when this library holds the tcgen05 prefill kernel (head sizes 64 and 128, and keys of 192).
-MRUN_API int mrun_attn_prefill_tc5_available() { return MRUN_ATTN_TC5; }
+// Rows per block of the tcgen05 kernel (head sizes 64 and 128, and keys of 192): a tile of the list holds at most this
+// divided by heads / kv_heads tokens, cut into streams of 128 / (heads / kv_heads).  0: not in this library.
+MRUN_API int mrun_attn_prefill_tc5_rows() {
+#if MRUN_ATTN_TC5
+    return MAX_Q * ROWS;
+#else
+    return 0;
+#endif
+}
 
-// Rows per tile of the tcgen05 kernel: a tile holds at most 128 / (heads / kv_heads) tokens.
-MRUN_API int mrun_attn_prefill_tc5_rows() { return 128; }
-
-// As mrun_attn_prefill, with tiles of at most 128 / (heads / kv_heads) tokens, a page size that is
+// As mrun_attn_prefill, with tiles of as many tokens as mrun_attn_prefill_tc5_rows() says, a page size that is
 // a power of two, and `pages` the number of pages of the two cache tensors.  `status` is one
 // int on the device, zero before the first call; a non-zero value afterwards names the role whose
 // wait ran out (1 loader, 2 products, 3 softmax) and the outputs of that launch are void.
@@ -534,6 +578,10 @@ MRUN_API int mrun_attn_prefill_tc5(const void* q, long q_stride, void* out, cons
     if (!configured) {
         MRUN_CHECK_CUDA(cudaFuncSetAttribute(prefill_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              SMEM_BYTES), "attn_prefill_tc5");
+        cudaFuncAttributes has;
+        MRUN_CHECK_CUDA(cudaFuncGetAttributes(&has, prefill_tc5_kernel), "attn_prefill_tc5");
+        MRUN_REQUIRE(has.numRegs == LAUNCH_REGISTERS, "attn_prefill_tc5: built with %d registers a thread, %d are dealt out", has.numRegs,
+                     LAUNCH_REGISTERS);
         configured = true;
     }
     for (int done = 0; done < n_tiles; done += 65535) {          // the grid's second dimension ends at 65535

@@ -14,14 +14,15 @@ the fused norm/rotary/cache kernel just before.
   into a ring for those head and page sizes, else copied with cp.async.
 * bfloat16 otherwise: a step with prompt portions.  Its single-token segments (the decoding
   requests beside the prompts) go through the TMA decode kernel as a selection of the step's rows
-  where that kernel takes the shape; the rest as follows.  Head sizes 64 and 128, and keys of 192: the tcgen05 kernel (128-row tiles
-  of tokens x group heads, accumulators in tensor memory) for every segment with more rows than
+  where that kernel takes the shape; the rest as follows.  Head sizes 64 and 128, and keys of 192: the tcgen05 kernel (tiles of 128 or 256
+  rows of tokens x group heads, accumulators in tensor memory) for every segment with more rows than
   one tile of the older kernel; the mma.sync kernel (64-row tiles) for the rest of the step (the
   single decode tokens of a mixed step, short tails) and for the other head sizes.
 """
 from __future__ import annotations
 
 import ctypes
+import heapq
 import math
 from typing import Optional
 
@@ -183,6 +184,70 @@ def prefill_tiles(ctx, tokens_per_tile: int, longer_than: int = 0, up_to: int = 
         first, count = [tile[1] for tile in found], [tile[2] for tile in found]
         n = len(first)
         both = ctx.upload(np.asarray(first + count, dtype=np.int32)) if n else None
+        tiles = ctx.shared[key] = (both[:n], both[n:], n) if n else (None, None, 0)
+    return tiles
+
+
+# A block of the tcgen05 prompt kernel, us: what it takes whatever its keys, a tile of 128 keys for a pair of streams
+# (rows of their own each), and for streams that share their rows and take every second tile each.
+TC5_BLOCK, TC5_PAIR_TILE, TC5_SHARED_TILE = 5.0, 1.9, 1.25
+
+
+def _makespan(costs, machines: int) -> float:
+    """When the last of ``machines`` is done, each taking the next of ``costs`` as it gets free."""
+    if len(costs) <= machines:
+        return max(costs, default=0.0)
+    free = [0.0] * machines
+    for cost in costs:
+        heapq.heapreplace(free, free[0] + cost)
+    return max(free)
+
+
+def tc5_tiles(ctx, tokens: int, longer_than: int, streams: int, window: int, blocks_at_once: float):
+    """(first token row, token count) of the blocks of the tcgen05 prompt kernel over the segments with more than
+    ``longer_than`` tokens, the longest first, as device int32 arrays; made once per step and choice of sizes.
+
+    A stream of the kernel takes up to ``tokens`` tokens.  A block whose two ``streams`` have tokens of their own reads keys
+    and values once for both and costs less a row; a block of one stream's tokens, which both walk over, is done sooner and
+    leaves fewer multiprocessors idle at the end.  So the longest blocks are pairs and the rest are not; how many are is
+    what ends first by the costs above, of none, all, and as many as fill the device evenly (``blocks_at_once`` a kv head).
+    """
+    key = ("attention_tc5_tiles", tokens, longer_than, streams, window, blocks_at_once)
+    tiles = ctx.shared.get(key)
+    if tiles is None:
+        def keys_of(end, count):              # tiles of 128 keys
+            low = end - count                 # the first token's position
+            low = 0 if window == 0 else max(0, low - window + 1) if window > 0 else low // -window * -window
+            return (end - 1) // 128 - low // 128 + 1
+        wide = []
+        for seg in ctx.segments:
+            if seg.q_len > longer_than:
+                for t0 in range(0, seg.q_len, streams * tokens):
+                    count = min(streams * tokens, seg.q_len - t0)
+                    end = seg.pos_start + t0 + count
+                    wide.append((keys_of(end, count), end, seg.q_start + t0, count))
+        wide.sort(key=lambda tile: (-tile[0], -tile[1]))        # a stable sort: the order depends on the segments only
+        found = [(TC5_SHARED_TILE * keys + TC5_BLOCK, first, count) for keys, _, first, count in wide]
+        if streams == 2 and any(tile[3] > tokens for tile in wide):
+            machines = max(1, int(blocks_at_once))
+            best = None
+            for pairs in sorted({len(wide), int(len(wide) // blocks_at_once * blocks_at_once), 0}, reverse=True):
+                blocks = []
+                for i, (keys, end, first, count) in enumerate(wide):
+                    if count <= tokens:
+                        blocks.append((TC5_SHARED_TILE * keys + TC5_BLOCK, first, count))
+                    elif i < pairs:
+                        blocks.append((TC5_PAIR_TILE * keys + TC5_BLOCK, first, count))
+                    else:
+                        rest = count - tokens
+                        blocks.append((TC5_SHARED_TILE * keys_of(end, rest) + TC5_BLOCK, first + tokens, rest))
+                        blocks.append((TC5_SHARED_TILE * keys_of(end - rest, tokens) + TC5_BLOCK, first, tokens))
+                blocks.sort(key=lambda block: -block[0])
+                ends = _makespan([block[0] for block in blocks], machines)
+                if best is None or ends < best:
+                    best, found = ends, blocks
+        n = len(found)
+        both = ctx.upload(np.asarray([b[1] for b in found] + [b[2] for b in found], dtype=np.int32)) if n else None
         tiles = ctx.shared[key] = (both[:n], both[n:], n) if n else (None, None, 0)
     return tiles
 
@@ -420,9 +485,10 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
             shortest = 1
     short_up_to = 1 << 30
     if prefill_uses_tcgen05(library, ratio, page_size):
-        # segments with more rows than a 64-row tile go to the 128-row tcgen05 kernel
+        # segments with more rows than a 64-row tile go to the tcgen05 kernel, whose streams take 128 rows
         short_up_to = (64 // ratio) if ratio <= 64 else 0
-        first, count, n_tiles = prefill_tiles(ctx, 128 // ratio, longer_than=max(short_up_to, shortest))
+        first, count, n_tiles = tc5_tiles(ctx, 128 // ratio, max(short_up_to, shortest), _tc5_prefill[library.path] // 128, window,
+                                          ops.sm_count(q.device) / kv_heads)
         if n_tiles:
             status = ops.status_word(q.device, "attn_prefill_tc5",
                                      {1: "a key/value loader", 2: "the MMA issuer", 3: "the softmax warps"})
@@ -437,7 +503,7 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
 
 
 TC5_PREFILL = True       # False: the mma.sync kernel for every prompt portion (tests compare the two)
-_tc5_prefill = {}
+_tc5_prefill = {}        # library -> rows of a block of its tcgen05 kernel (0: none)
 
 
 def prefill_uses_tcgen05(library, ratio: int, page_size: int) -> bool:
@@ -447,5 +513,5 @@ def prefill_uses_tcgen05(library, ratio: int, page_size: int) -> bool:
         return False
     have = _tc5_prefill.get(library.path)
     if have is None:
-        have = _tc5_prefill[library.path] = bool(library._dll.mrun_attn_prefill_tc5_available())
-    return have
+        have = _tc5_prefill[library.path] = int(library._dll.mrun_attn_prefill_tc5_rows())
+    return have > 0
