@@ -4,22 +4,23 @@
 // worked-on scores and gated outputs, attention_score.cuh: -DMRUN_SCORED=1).  Keys may have 192 features
 // where the values have 64 or 128 and the scores are plain: Q and two stages of K and V then take 209 KB.
 //
-// One thread block per (tile of query tokens, kv head), in two streams of 128 rows that take turns: while the
-// tensor cores work for one, the softmax of the other runs.  A row is a (token, query head of the kv head's group)
-// pair, so a key/value tile read once serves the whole group.  A long tile's streams have rows of their own and both
-// take every key tile; a short tile's (and all with keys of 192 features, where a second Q has no place) share
-// their rows, each takes every second key tile, and the two accumulators meet at the end.  Keys are consumed 128 at a time in
-// position order with an online softmax:
+// One thread block per (tile of query tokens, kv head).  A row is a (token, query head of the kv head's group) pair, so a
+// key/value tile read once serves the whole group.  Rows come in streams of 128; keys are consumed 128 at a time in position order
+// with an online softmax.  A long tile is a pair of streams that take turns: while the tensor cores work for one, the softmax of the other runs, and both
+// take every key tile.  A short tile (and all with keys of 192 features, where a second Q has no place) is a single stream, half a
+// row a thread.  Both ways do the same arithmetic in the same order on a row, so its bits do not depend on how the step is cut:
 //
-//   warps 0..7   softmax, four warps a stream, a thread a row (tensor-memory lane r is row r).  A thread reads its row of
-//                S = Q·Kᵀ (tcgen05.ld), masks it, keeps the running maximum and sum in 32-bit, and writes P =
-//                exp2(s - max) as packed bf16 over the scores (tcgen05.st), the first half of the keys as soon as it is there.
-//                It rescales its row of O when the
+//   warps 0..7   softmax.  Of a pair four warps a stream, a thread a row (tensor-memory lane r is row r).  A thread reads its row of
+//                S = Q·Kᵀ (tcgen05.ld), masks it, keeps the running maximum and the sums of either half of the keys in 32-bit, and writes P =
+//                exp2(s - max) as packed bf16 (tcgen05.st), the first half of the keys as soon as it is there.
+//                Of a single stream warp w and warp w + 4 share the lanes 32 (w % 4) .., the first takes keys 0..63 of a tile, the
+//                second keys 64..127; they meet for the row's maximum through shared memory and a barrier of the two warps, and for the sum at the end.
+//                A row of O is rescaled when the
 //                maximum has grown by more than 2^8 since the last rescale (until then P is
 //                taken against the older maximum, which is exact: the final division uses the
 //                same maximum);
-//   warp 8       issues the products: O += P[j]·V[j] in halves as P is written, then the stream's next S = Q·Kᵀ
-//                over the same columns.  P is
+//   warp 8       issues the products.  Of a pair: O += P[j]·V[j] in halves as P is written, then the stream's next S = Q·Kᵀ.  Of a
+//                single stream: O += P[j]·V[j] as P is there, S up to two tiles ahead of the softmax.  P is
 //                read from tensor memory, Q, K and V from shared memory, V as the MN-major
 //                operand (its rows are keys, as the cache stores them);
 //   warp 9       brings K tiles from the pages into a ring of two stages by TMA: a lane per page
@@ -27,13 +28,12 @@
 //                [rows x 64] boxes with the 128-byte swizzle; warp 10 the V tiles likewise.
 //
 // Bound by the chain of a stream's row (scores out of tensor memory, maximum, exponentials, P back, two products), of which two
-// run side by side: a tile of 128 keys for 256 rows of 128 features takes 1.9 us (2,048 cycles of MMAs and as many of the
-// special-function units would be 1.1), for 128 shared rows 1.25.  1,531 tokens behind 9,000, 32 heads over 8, B200: 251 us,
-// 0.98 PFLOP/s; half rows a thread, all eight warps on one tile of 128 rows at a time, 296 us, 1.28 a tile.
-// What the parts gave, us a tile of a pair: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
+// run side by side in a pair: a tile of 128 keys for 256 rows of 128 features takes 2.05 us (2,048 cycles of MMAs and as many of the
+// special-function units would be 1.1), for a single stream's 128 rows 1.32.  1,531 tokens behind 9,000, 32 heads over 8, B200:
+// 260 us, 0.95 PFLOP/s; single streams alone 299.
+// What the parts of a pair gave, us a tile: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
 // step); one elected lane, every wait but P's taken before, and both products issued in a row 2.1 -> 1.9; P in halves 2.3 ->
-// 2.25; the page looked up ahead 1.40 -> 1.27 (shared rows).  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 ->
-// 1.96, a third stage of K or V nothing.
+// 2.25.  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 -> 1.96, a third stage of K or V nothing.
 //
 // The roles hand tiles to one another through mbarriers; every wait is bounded by a cycle budget.
 // When a wait runs out the block records a code in the status word, every role stops, the block
@@ -82,7 +82,7 @@ using namespace tc5;
 constexpr int D = MRUN_HEAD_DIM, DV = MRUN_VALUE_DIM;
 constexpr bool SCORED = MRUN_SCORED;
 constexpr int ROWS = 128;                    // query rows per stream = MMA M
-constexpr int KEYS = 128;                    // keys per tile = N of the first product, K of the second
+constexpr int KEYS = 128, HALF = 64;         // keys per tile = N of the first product, K of the second
 constexpr int SPANS_D = D / 64, SPANS_V = DV / 64;      // 64-wide spans of the head dimensions
 constexpr int SPAN_BYTES = 128 * 128;        // one swizzled tile of 128 rows x 64 bf16
 constexpr int K_BYTES = SPANS_D * SPAN_BYTES;           // one stage of K: 128 keys x D
@@ -95,8 +95,9 @@ constexpr int MMA_WARP = 8, K_WARP = 9, V_WARP = 10;
 constexpr int THREADS = SOFTMAX_THREADS + 4 * 32;                        // 384: registers are dealt to four warps together
 constexpr int SOFTMAX_REGISTERS = 216, OTHER_REGISTERS = 72, LAUNCH_REGISTERS = 168;
 static_assert(SOFTMAX_THREADS * SOFTMAX_REGISTERS + 128 * OTHER_REGISTERS <= THREADS * LAUNCH_REGISTERS, "more registers than the block has");
-constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256) O0 [256, 256 + DV) O1 [384, 384 + DV); P lies on its S
-constexpr unsigned O_COL = 256;
+constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256), then of a pair O0 [256, 256 + DV) O1 [384, 384 + DV), each
+                                             // P on its S; of a single stream P0 [256,320) P1 [320,384) O [384, 384 + DV)
+constexpr unsigned O_COL = 256, P_COL = 256, SINGLE_O_COL = 384;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.f;          // log2 of the growth of a row maximum that forces a rescale
 constexpr long long WAIT_CYCLES = 3000000000LL;         // about 1.5 s at 2 GHz
@@ -130,8 +131,100 @@ __device__ __forceinline__ void pair_sync(int quarter) {
 struct Barriers {
     unsigned long long q_full;
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];
-    unsigned long long s_full[2], p_full[2][2], o_full;              // [stream], [stream][half of the keys]
+    unsigned long long s_full[2], s_empty[2];                        // of a pair's streams, of a single stream's two accumulators
+    unsigned long long p_full[2][2];                                 // [stream or buffer][half of the keys, of a pair]
+    unsigned long long pv_done, o_full;                              // of a single stream's tile; of all
 };
+
+// ------------------------------------------------------------------------------------------ a row's keys, half a tile at a time
+// Both ways of taking a tile use these on the same 64 keys, in the same order, so a row has the same bits in a pair and alone.
+
+// Worked-on scores, in base-2 units: two a step where the polynomial serves (every row of the warp alike), then the bias, an entry
+// a distance only near the query.  first_pos: the position of the stream's first row.
+__device__ __forceinline__ void work_on(float (&sc)[HALF], const mrun_score_form& form, const mrun::ScoreRow& form_row, int key_base,
+                                        int first_pos, int row_pos) {
+    if constexpr (SCORED) {
+        if (__all_sync(0xffffffffu, form_row.small)) {
+            const float2 factor2 = make_float2(form_row.factor, form_row.factor);
+            const float2 cap2 = make_float2(form_row.cap2, form_row.cap2);
+            const float2 far2 = make_float2(form_row.far_bias, form_row.far_bias);
+#pragma unroll
+            for (int i = 0; i < HALF; i += 2) {
+                const float2 th = mrun::tanh_small2(__fmul2_rn(make_float2(sc[i], sc[i + 1]), factor2));
+                const float2 v = __ffma2_rn(th, cap2, far2);
+                sc[i] = v.x; sc[i + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < HALF; ++i) sc[i] = mrun::capped_score(form_row, sc[i]) + form_row.far_bias;
+        }
+        if (form.bias != nullptr && first_pos - (key_base + HALF - 1) < form.bias_len - 1) {
+            // every entry as its difference from the far one, which the scores hold already
+            const float* table = form_row.bias;
+            const int distance = row_pos - key_base;
+#pragma unroll
+            for (int i = 0; i < HALF; ++i)
+                sc[i] += fmaf(__ldg(table + min(max(distance - i, 0), form_row.bias_last)), LOG2E, -form_row.far_bias);
+        }
+    }
+}
+
+// Keys outside lo..hi, counted from the first of these, become -inf and later give p = 0.
+__device__ __forceinline__ void mask_out(float (&sc)[HALF], int lo, int hi) {
+#pragma unroll
+    for (int i = 0; i < HALF; ++i)
+        if (i > hi || i < lo) sc[i] = -INFINITY;
+}
+
+__device__ __forceinline__ float largest(const float (&sc)[HALF]) {
+    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < HALF; i += 8)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(fmaxf(mx4[c], sc[i + 2 * c]), sc[i + 2 * c + 1]);
+    return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+}
+
+// The maximum the probabilities are taken against moves only by large steps.  mx: the largest raw score (the scale is positive,
+// so it scales the maximum alike).
+__device__ __forceinline__ float next_max(float mx, float m_used, float scale_log2) {
+    if constexpr (!SCORED) mx *= scale_log2;
+    return mx > m_used + RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY) ? mx : m_used;
+}
+
+// A row's columns of O times corr.
+__device__ __forceinline__ void rescale(unsigned address, int columns, float corr) {
+#pragma unroll 1
+    for (int c = 0; c < columns; c += 16) {
+        float v[16];
+        tmem_load16(address + c, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] *= corr;
+        tmem_store16_start(address + c, v);
+    }
+}
+
+// P = 2^(s * unit - m): one fused multiply-add and one special-function call a score, two scores an instruction where the hardware
+// has one (fma.f32x2, add.f32x2), stored as packed bf16 from `address` on.  Masked scores are -inf and give 0; a row that has
+// seen nothing yet keeps m = -inf.  Returns the sum.
+__device__ __forceinline__ float probabilities(const float (&sc)[HALF], float unit, float m, unsigned address) {
+    const float m_sub = m == -INFINITY ? 0.f : -m;
+    const float2 scale2 = make_float2(unit, unit), m_sub2 = make_float2(m_sub, m_sub);
+    float2 sums = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < HALF; c += 32) {
+        float packed[16];                                             // two bf16 a word, even key low
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            const float2 x = __ffma2_rn(make_float2(sc[c + i], sc[c + i + 1]), scale2, m_sub2);
+            const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+            sums = __fadd2_rn(sums, p);
+            packed[i >> 1] = __uint_as_float(pack_bf16(p.x, p.y));
+        }
+        tmem_store16_start(address + c / 2, packed);
+    }
+    return sums.x + sums.y;
+}
 
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -149,7 +242,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     __shared__ Barriers bars;
     __shared__ unsigned tmem_base_slot;
     __shared__ int aborted;
-    __shared__ float row_max[2][ROWS], row_sum[2][ROWS];     // of the two streams, where they share their rows
+    __shared__ float half_max[2][2][ROWS];               // of a single stream: [tile parity][half of the keys][row]
+    __shared__ float half_sum[2][ROWS];                  // [half][row], at the end
 
     // Blocks start in the order of their index, x first: all kv heads of the first tile of the
     // list, which the host sorted by falling work, then all of the second, ...
@@ -158,7 +252,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     const int tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int per_stream = ROWS / group;                 // tokens
-    const bool apart = MAX_Q == 2 && ntok > per_stream;  // the streams have rows of their own and take every key tile
+    const bool pair = MAX_Q == 2 && ntok > per_stream;   // two streams of rows
     // tokens of a tile are consecutive positions of one request
     const int pos_first = positions[tok0], pos_last = pos_first + ntok - 1;
     const int lo_tile = mrun::first_visible(pos_first, window);
@@ -173,9 +267,11 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             mbar_init(&bars.k_empty[s], 1);
             mbar_init(&bars.v_empty[s], 1);
             mbar_init(&bars.s_full[s], 1);
-            mbar_init(&bars.p_full[s][0], STREAM_WARPS);
+            mbar_init(&bars.s_empty[s], SOFTMAX_WARPS);
+            mbar_init(&bars.p_full[s][0], pair ? STREAM_WARPS : SOFTMAX_WARPS);
             mbar_init(&bars.p_full[s][1], STREAM_WARPS);
         }
+        mbar_init(&bars.pv_done, 1);
         mbar_init(&bars.o_full, 1);
         aborted = 0;
         mbar_init_fence();
@@ -192,13 +288,13 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     const unsigned tmem_base = tmem_base_slot;
 
     if (warp < SOFTMAX_WARPS) {
-        // ------------------------------------------------------------------ softmax, a row a thread
+        // ------------------------------------------------------------------------------- softmax
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SOFTMAX_REGISTERS));
-        const int quarter = warp & 3, stream = warp >> 2;
+        const int quarter = warp & 3, side = warp >> 2;               // a pair: the stream; a single stream: the half of the keys
         const int row = quarter * 32 + lane;                          // 0..127
         const unsigned lane_base = tmem_base + ((unsigned)(quarter * 32) << 16);
         // q rows: row r = (token r / group, head kvh * group + r % group); rows past the stream's are zero
-        for (int c = threadIdx.x; c < (apart ? 2 : 1) * ROWS * (D / 8); c += SOFTMAX_THREADS) {
+        for (int c = threadIdx.x; c < (pair ? 2 : 1) * ROWS * (D / 8); c += SOFTMAX_THREADS) {
             const int part = c / (ROWS * (D / 8)), in = c - part * (ROWS * (D / 8));
             const int r = in / (D / 8), chunk = in - r * (D / 8), token = part * per_stream + r / group;
             const bool valid = r < per_stream * group && token < ntok;
@@ -212,7 +308,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars.q_full);
 
-        const int token0 = apart ? stream * per_stream : 0;                       // the stream's tokens within the tile
+        const int token0 = pair ? side * per_stream : 0;                          // the stream's tokens within the tile
         const int tokens = min(ntok - token0, per_stream);
         const int n_rows = tokens * group;
         const int first_pos = pos_first + token0, last_pos = first_pos + tokens - 1;
@@ -223,168 +319,149 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         const int head = kvh * group + row % group;
         mrun::ScoreRow form_row = {};
         if constexpr (SCORED) form_row = mrun::score_row(form, scale_log2 / LOG2E, row_pos, kvh * group + min(row, n_rows - 1) % group);
-        float m_used = -INFINITY, l = 0.f;
+        const float unit = SCORED ? 1.f : scale_log2;
+        float m_used = -INFINITY;
+        float sum[2] = {0.f, 0.f};                    // of the row's keys 0..63 and 64..127 of every tile; a half's thread: its own first
         bool alive = true;
-        const int mine = apart ? n_tiles : (n_tiles + 1 - stream) / 2;        // this stream's items
-        for (int it = 0; it < mine; ++it) {
-            if (!__all_sync(0xffffffffu, mbar_wait(&bars.s_full[stream], it & 1, WAIT_CYCLES, &aborted))) { alive = false; break; }
-            const int key_base = (first_block + (apart ? it : 2 * it + stream)) * KEYS;
-            // every row of the stream sees every key of the tile: no comparisons
-            const bool need_mask = key_base + KEYS - 1 > first_pos || key_base < lo_last || n_rows < ROWS;
-            float sc[KEYS];
-            float mx = -INFINITY;
-            tc_fence_after();
-            {
-                unsigned raw[KEYS];
+        // every row of the stream sees every key of the tile: no comparisons
+        auto needs_mask = [&](int key0) { return key0 + KEYS - 1 > first_pos || key0 < lo_last || n_rows < ROWS; };
+        if (pair) {
+            for (int it = 0; it < n_tiles; ++it) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&bars.s_full[side], it & 1, WAIT_CYCLES, &aborted))) { alive = false; break; }
+                const int key0 = (first_block + it) * KEYS;
+                float sc[2][HALF];
+                tc_fence_after();
+                {
+                    unsigned raw[KEYS];
 #pragma unroll
-                for (int c = 0; c < KEYS; c += 32)
-                    tmem_load32_start(lane_base + stream * KEYS + c, *reinterpret_cast<unsigned (*)[32]>(&raw[c]));
-                tmem_load_wait();
+                    for (int c = 0; c < KEYS; c += 32)
+                        tmem_load32_start(lane_base + side * KEYS + c, *reinterpret_cast<unsigned (*)[32]>(&raw[c]));
+                    tmem_load_wait();
 #pragma unroll
-                for (int i = 0; i < KEYS; ++i) {
-                    pin(raw[i]);
-                    sc[i] = __uint_as_float(raw[i]);
-                }
-            }
-            if constexpr (SCORED) {
-                // scores in base-2 units from here on: two a step where the polynomial serves (every
-                // row of the warp alike), then the bias, an entry a distance only near the query
-                if (__all_sync(0xffffffffu, form_row.small)) {
-                    const float2 factor2 = make_float2(form_row.factor, form_row.factor);
-                    const float2 cap2 = make_float2(form_row.cap2, form_row.cap2);
-                    const float2 far2 = make_float2(form_row.far_bias, form_row.far_bias);
-#pragma unroll
-                    for (int i = 0; i < KEYS; i += 2) {
-                        const float2 th = mrun::tanh_small2(__fmul2_rn(make_float2(sc[i], sc[i + 1]), factor2));
-                        const float2 v = __ffma2_rn(th, cap2, far2);
-                        sc[i] = v.x; sc[i + 1] = v.y;
+                    for (int i = 0; i < KEYS; ++i) {
+                        pin(raw[i]);
+                        sc[i / HALF][i % HALF] = __uint_as_float(raw[i]);
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < KEYS; ++i) sc[i] = mrun::capped_score(form_row, sc[i]) + form_row.far_bias;
                 }
-                if (form.bias != nullptr && first_pos - (key_base + KEYS - 1) < form.bias_len - 1) {
-                    // every entry as its difference from the far one, which the scores hold already
-                    const float* table = form_row.bias;
-                    const int distance = row_pos - key_base;
+                const bool mask = needs_mask(key0);
+                float mx = -INFINITY;
 #pragma unroll
-                    for (int i = 0; i < KEYS; ++i)
-                        sc[i] += fmaf(__ldg(table + min(max(distance - i, 0), form_row.bias_last)), LOG2E, -form_row.far_bias);
+                for (int h = 0; h < 2; ++h) {
+                    work_on(sc[h], form, form_row, key0 + h * HALF, first_pos, row_pos);
+                    if (mask) mask_out(sc[h], row_lo - key0 - h * HALF, row_pos - key0 - h * HALF);
+                    mx = fmaxf(mx, largest(sc[h]));
                 }
-            }
-            // the largest raw score first (the scale is positive, so it scales the maximum
-            // alike); masked scores become -inf and later give p = 0
-            if (need_mask) {
-                const int lo_rel = row_lo - key_base, hi_rel = row_pos - key_base;
-#pragma unroll
-                for (int i = 0; i < KEYS; ++i) {
-                    if (i > hi_rel || i < lo_rel) sc[i] = -INFINITY;
+                const float m_new = next_max(mx, m_used, scale_log2);
+                const bool moved = m_new != m_used && m_used != -INFINITY;       // O holds something to rescale
+                if (__any_sync(0xffffffffu, moved)) {
+                    // the second product of this stream's item before was issued before this one's first, so it has finished
+                    const float corr = moved ? exp2f(m_used - m_new) : 1.f;
+                    rescale(lane_base + O_COL + side * 128, DV, corr);
+                    sum[0] *= corr;
+                    sum[1] *= corr;
                 }
-            }
-            {
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                m_used = m_new;
 #pragma unroll
-                for (int i = 0; i < KEYS; i += 8) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(fmaxf(mx4[c], sc[i + 2 * c]), sc[i + 2 * c + 1]);
-                }
-                mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            }
-            if constexpr (!SCORED) mx *= scale_log2;
-            // the maximum the probabilities are taken against moves only by large steps
-            float m_new = m_used;
-            if (mx > m_used + RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY)) m_new = mx;
-            const bool moved = m_new != m_used && m_used != -INFINITY;       // O holds something to rescale
-            if (__any_sync(0xffffffffu, moved)) {
-                // the second product of this stream's item before was issued before this one's first, so it has finished
-                const float corr = moved ? exp2f(m_used - m_new) : 1.f;
-#pragma unroll 1
-                for (int c = 0; c < DV; c += 16) {
-                    float v[16];
-                    tmem_load16(lane_base + O_COL + stream * 128 + c, v);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] *= corr;
-                    tmem_store16_start(lane_base + O_COL + stream * 128 + c, v);
-                }
-                l *= corr;
-            }
-            m_used = m_new;
-            // p = 2^(s * scale - m): one fused multiply-add and one special-function call a score.
-            // Masked scores are -inf and give 0; a row that has seen nothing yet keeps m_used = -inf.
-            const float m_sub = m_used == -INFINITY ? 0.f : -m_used;
-            // Two scores an instruction where the hardware has one (fma.f32x2, add.f32x2)
-            const float unit = SCORED ? 1.f : scale_log2;
-            const float2 scale2 = make_float2(unit, unit), m_sub2 = make_float2(m_sub, m_sub);
-            float2 sums = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int c = 0; c < KEYS; c += 32) {
-                float packed[16];                                     // two bf16 a word, even key low
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float2 x = __ffma2_rn(make_float2(sc[c + i], sc[c + i + 1]), scale2, m_sub2);
-                    const float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-                    sums = __fadd2_rn(sums, p);
-                    packed[i >> 1] = __uint_as_float(pack_bf16(p.x, p.y));
-                }
-                tmem_store16_start(lane_base + stream * KEYS + c / 2, packed);      // on this row's scores, which are in registers
-                if (c % 64 == 32) {                                   // half of the second product may begin
+                for (int h = 0; h < 2; ++h) {
+                    // on this row's scores, which are in registers
+                    sum[h] += probabilities(sc[h], unit, m_used, lane_base + side * KEYS + h * (HALF / 2));
                     tmem_store_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars.p_full[stream][c / 64]);
+                    if (lane == 0) mbar_arrive(&bars.p_full[side][h]);           // half of the second product may begin
                 }
             }
-            l += sums.x + sums.y;
+        } else {
+            // A warp that gave up on a wait still walks through the remaining tiles, doing nothing but meeting its partner at
+            // every barrier, so that no warp is left waiting at one.
+            for (int j = 0; j < n_tiles; ++j) {
+                const int buf = j & 1;
+                if (alive && !__all_sync(0xffffffffu, mbar_wait(&bars.s_full[buf], (j >> 1) & 1, WAIT_CYCLES, &aborted))) alive = false;
+                const int key0 = (first_block + j) * KEYS, half0 = key0 + side * HALF;
+                float sc[HALF];
+                float mx = -INFINITY;
+                if (alive) {
+                    tc_fence_after();
+                    unsigned raw[HALF];
+#pragma unroll
+                    for (int c = 0; c < HALF; c += 32)
+                        tmem_load32_start(lane_base + buf * KEYS + side * HALF + c, *reinterpret_cast<unsigned (*)[32]>(&raw[c]));
+                    tmem_load_wait();
+                    // the scores are in registers: the product after next may overwrite the accumulator
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars.s_empty[buf]);
+#pragma unroll
+                    for (int i = 0; i < HALF; ++i) {
+                        pin(raw[i]);
+                        sc[i] = __uint_as_float(raw[i]);
+                    }
+                    work_on(sc, form, form_row, half0, first_pos, row_pos);
+                    if (needs_mask(key0)) mask_out(sc, row_lo - half0, row_pos - half0);
+                    mx = largest(sc);
+                }
+                half_max[buf][side][row] = mx;
+                pair_sync(quarter);
+                if (!alive) continue;
+                // both halves of a row decide alike, from the same numbers
+                const float m_new = next_max(fmaxf(mx, half_max[buf][side ^ 1][row]), m_used, scale_log2);
+                const bool moved = m_new != m_used && m_used != -INFINITY;
+                if (__any_sync(0xffffffffu, moved)) {
+                    // O belongs to the second product of the tile before until that has finished (the one before it has: its
+                    // scores' barrier came behind it)
+                    if (j > 0 && !__all_sync(0xffffffffu, mbar_wait(&bars.pv_done, (j - 1) & 1, WAIT_CYCLES, &aborted))) {
+                        alive = false;
+                        continue;
+                    }
+                    tc_fence_after();
+                    const float corr = moved ? exp2f(m_used - m_new) : 1.f;
+                    rescale(lane_base + SINGLE_O_COL + side * (DV / 2), DV / 2, corr);
+                    sum[0] *= corr;
+                }
+                m_used = m_new;
+                // the P buffer of this tile was read by the second product of the tile before last
+                if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&bars.v_empty[buf], ((j >> 1) - 1) & 1, WAIT_CYCLES, &aborted))) {
+                    alive = false;
+                    continue;
+                }
+                sum[0] += probabilities(sc, unit, m_used, lane_base + P_COL + buf * (KEYS / 2) + side * (HALF / 2));
+                tmem_store_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars.p_full[buf][0]);
+            }
         }
-        // a warp leaves the loop as a whole, so every lane takes part in what follows
+        // A warp leaves the loop as a whole, so every lane takes part in what follows.  o_full has one phase: of pv_done's, any of
+        // the last three may be open when a warp comes here, and a parity tells a phase from its neighbours only.
         if (alive && !__all_sync(0xffffffffu, mbar_wait(&bars.o_full, 0, WAIT_CYCLES, &aborted))) alive = false;
         if (!alive) {
             if (!*(volatile int*)&aborted) atomicExch(status, STATUS_SOFTMAX);
             atomicExch(&aborted, 1);
         }
-        // Streams that share their rows meet (the other may have given up: it still comes here): each writes one half of the
-        // columns, both accumulators against the larger of the two maxima.
-        float m_all = m_used, scale[2] = {stream == 0 ? 1.f : 0.f, stream == 0 ? 0.f : 1.f};
-        int col0 = 0, col1 = DV;
-        if (!apart) {
-            row_max[stream][row] = m_used;
-            row_sum[stream][row] = l;
+        if (!pair) {                                  // the other half's sum (its warp may have given up: it still comes here)
+            half_sum[side][row] = sum[0];
             pair_sync(quarter);
-            const float m0 = row_max[0][row], m1 = row_max[1][row];
-            m_all = fmaxf(m0, m1);
-            scale[0] = m0 == -INFINITY ? 0.f : exp2f(m0 - m_all);
-            scale[1] = m1 == -INFINITY ? 0.f : exp2f(m1 - m_all);
-            l = row_sum[0][row] * scale[0] + row_sum[1][row] * scale[1];
-            col0 = stream * (DV / 2);
-            col1 = col0 + DV / 2;
+            sum[1] = half_sum[side ^ 1][row];
         }
         if (alive) {
             tc_fence_after();
-            const float total = with_sink(l, m_all, sinks, head);
+            const float total = with_sink(sum[0] + sum[1], m_used, sinks, head);
             const float inv = total > 0.f ? 1.f / total : 0.f;
             const int token = tok0 + token0 + row / group;
+            // a pair's thread writes its row, a half's thread half of the columns
+            const unsigned src = lane_base + (pair ? O_COL + side * 128 : SINGLE_O_COL);
+            const int col0 = pair ? 0 : side * (DV / 2), col1 = pair ? DV : col0 + DV / 2;
             bf16* dst = out + (size_t)token * (SCORED ? form.out_stride : (long)heads * DV) + head * DV;
-            // an accumulator that no product wrote holds anything
-            const bool use[2] = {apart ? stream == 0 : true, apart ? stream == 1 : n_tiles > 1};
 #pragma unroll 1
-            for (int c = col0; c < col1; c += 16) {
-                float v[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] = 0.f;
-#pragma unroll
-                for (int part = 0; part < 2; ++part)
-                    if (use[part]) {
-                        float o[16];
-                        tmem_load16(lane_base + O_COL + part * 128 + c, o);       // every lane of the warp takes part
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = fmaf(o[i], scale[part], v[i]);
-                    }
+            for (int c = col0; c < col1; c += 32) {
+                float v[32];
+                tmem_load32(src + c, v);              // every lane of the warp takes part
                 if (row < n_rows) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] *= inv;
-                    if constexpr (SCORED) mrun::gate_outputs<16>(form, token, head * DV + c, v);
+                    for (int i = 0; i < 32; ++i) v[i] *= inv;
+                    if constexpr (SCORED) mrun::gate_outputs<32>(form, token, head * DV + c, v);
 #pragma unroll
-                    for (int k = 0; k < 2; ++k)
+                    for (int k = 0; k < 4; ++k)
                         *reinterpret_cast<uint4*>(dst + c + 8 * k) =
                             make_uint4(pack_bf16(v[8 * k], v[8 * k + 1]), pack_bf16(v[8 * k + 2], v[8 * k + 3]),
                                        pack_bf16(v[8 * k + 4], v[8 * k + 5]), pack_bf16(v[8 * k + 6], v[8 * k + 7]));
@@ -402,59 +479,73 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             auto wait = [&](unsigned long long* bar, unsigned parity) {
                 return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, WAIT_CYCLES, &aborted));
             };
-            // Item i is stream i & 1's: key tile i / 2 (apart) or i.  Descriptors further on differ in their address field, which
-            // counts 16-byte units.
-            const int n_items = apart ? 2 * n_tiles : n_tiles;
-            auto issue_qk = [&](int stream, int s) {                      // by the elected lane; s: K's stage
-                const unsigned long long qd = q_desc + (apart ? stream * (Q_BYTES >> 4) : 0), kd = k_desc + s * (K_BYTES >> 4);
+            // Descriptors further on differ in their address field, which counts 16-byte units.
+            auto issue_qk = [&](int acc, int q_part, int s) {             // by the elected lane; s: K's stage
+                const unsigned long long qd = q_desc + q_part * (Q_BYTES >> 4), kd = k_desc + s * (K_BYTES >> 4);
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {                     // 32 bytes further along d per step
                     const int off = ((kk >> 2) * SPAN_BYTES + (kk & 3) * 32) >> 4;
-                    umma_bf16(tmem_base + stream * KEYS, qd + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
+                    umma_bf16(tmem_base + acc * KEYS, qd + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
                 }
-                umma_commit(&bars.s_full[stream]);
-                if (!apart || stream == 1) umma_commit(&bars.k_empty[s]);
+                umma_commit(&bars.s_full[acc]);
+                if (!pair || acc == 1) umma_commit(&bars.k_empty[s]);
+            };
+            // P: eight columns (16 keys) further per step; V: sixteen rows.  Steps [from, to) of the tile's eight.
+            auto issue_pv = [&](unsigned o, unsigned p, int s, int from, int to, bool first) {
+                const unsigned long long vd = v_desc + s * (V_BYTES >> 4);
+#pragma unroll
+                for (int kk = 0; kk < KEYS / 16; ++kk)
+                    if (kk >= from && kk < to)
+                        umma_bf16_a_tmem(tmem_base + o, tmem_base + p + kk * 8, vd + kk * (2048 >> 4), idesc_pv, (!first || kk > 0) ? 1u : 0u);
             };
             bool alive = wait(&bars.q_full, 0);
+            // Item i of a pair is stream i & 1's, key tile i / 2; a single stream's is key tile i.
+            const int n_items = pair ? 2 * n_tiles : n_tiles;
             for (int i = 0; alive && i < 2 && i < n_items; ++i) {
-                const int s = apart ? 0 : i;
+                const int s = pair ? 0 : i;
                 alive = wait(&bars.k_full[s], 0);
                 if (!alive) break;
-                if (elect_one()) issue_qk(i, s);
+                if (elect_one()) issue_qk(i, pair ? i : 0, s);
                 __syncwarp();
             }
             for (int i = 0; alive && i < n_items; ++i) {
-                const int stream = i & 1, j = apart ? i >> 1 : i, s = j & 1;
-                const int next = apart ? j + 1 : j + 2, next_s = next & 1;        // the key tile of the stream's next item
+                const int acc = i & 1, j = pair ? i >> 1 : i, s = j & 1;
+                const int next = pair ? j + 1 : j + 2, next_s = next & 1;         // the key tile of the accumulator's next item
                 const bool more = i + 2 < n_items;
-                const unsigned long long vd = v_desc + s * (V_BYTES >> 4);
-                // P comes last, so what waits for it goes on at once; the stream's next scores go where its P lies, behind the
-                // product that reads it
+                // what is waited for comes in the order of its arrival, P last, so that it goes on at once then
                 if (!wait(&bars.v_full[s], (j >> 1) & 1) || (more && !wait(&bars.k_full[next_s], (next >> 1) & 1)) ||
-                    !wait(&bars.p_full[stream][0], (i >> 1) & 1)) {
+                    !wait(&bars.p_full[acc][0], (i >> 1) & 1)) {
                     alive = false;
                     break;
                 }
-                auto issue_pv = [&](int half) {                           // P: eight columns (16 keys) further per step; V: sixteen rows
-#pragma unroll
-                    for (int kk = 0; kk < KEYS / 32; ++kk) {
-                        const int at = half * (KEYS / 32) + kk;
-                        umma_bf16_a_tmem(tmem_base + O_COL + stream * 128, tmem_base + stream * KEYS + at * 8, vd + at * (2048 >> 4), idesc_pv,
-                                         (i > 1 || at > 0) ? 1u : 0u);
+                tc_fence_after();
+                if (pair) {
+                    const unsigned o = O_COL + acc * 128, p = acc * KEYS;
+                    if (elect_one()) issue_pv(o, p, s, 0, KEYS / 32, i < 2);
+                    __syncwarp();
+                    if (!wait(&bars.p_full[acc][1], (i >> 1) & 1)) { alive = false; break; }
+                    tc_fence_after();
+                    if (elect_one()) {
+                        issue_pv(o, p, s, KEYS / 32, KEYS / 16, i < 2);
+                        if (acc == 1) umma_commit(&bars.v_empty[s]);
+                        // the stream's next scores go where its P lies, behind the product that reads it
+                        if (more) issue_qk(acc, acc, next_s);
+                        if (i + 1 == n_items) umma_commit(&bars.o_full);
                     }
-                };
-                tc_fence_after();
-                if (elect_one()) issue_pv(0);
-                __syncwarp();
-                if (!wait(&bars.p_full[stream][1], (i >> 1) & 1)) { alive = false; break; }
-                tc_fence_after();
-                if (elect_one()) {
-                    issue_pv(1);
-                    if (!apart || stream == 1) umma_commit(&bars.v_empty[s]);
-                    if (more) issue_qk(stream, next_s);
-                    if (i + 1 == n_items) umma_commit(&bars.o_full);
+                    __syncwarp();
+                } else {
+                    if (elect_one()) {
+                        issue_pv(SINGLE_O_COL, P_COL + acc * (KEYS / 2), s, 0, KEYS / 16, i == 0);
+                        umma_commit(&bars.v_empty[s]);
+                        umma_commit(&bars.pv_done);
+                        if (i + 1 == n_items) umma_commit(&bars.o_full);
+                    }
+                    __syncwarp();
+                    // the scores before are in registers
+                    if (more && !wait(&bars.s_empty[acc], (i >> 1) & 1)) { alive = false; break; }
+                    if (more && elect_one()) issue_qk(acc, 0, next_s);
+                    __syncwarp();
                 }
-                __syncwarp();
             }
             if (!alive) {
                 if (!*(volatile int*)&aborted) atomicExch(status, STATUS_MMA);

@@ -188,9 +188,9 @@ def prefill_tiles(ctx, tokens_per_tile: int, longer_than: int = 0, up_to: int = 
     return tiles
 
 
-# A block of the tcgen05 prompt kernel, us: what it takes whatever its keys, a tile of 128 keys for a pair of streams
-# (rows of their own each), and for streams that share their rows and take every second tile each.
-TC5_BLOCK, TC5_PAIR_TILE, TC5_SHARED_TILE = 5.0, 1.9, 1.25
+# A block of the tcgen05 prompt kernel, us: what it takes whatever its keys, a tile of 128 keys for a pair of streams, and for a
+# single stream (32 heads over 8 of 128 features, B200).
+TC5_BLOCK, TC5_PAIR_TILE, TC5_SINGLE_TILE = 5.0, 2.05, 1.32
 
 
 def _makespan(costs, machines: int) -> float:
@@ -207,10 +207,10 @@ def tc5_tiles(ctx, tokens: int, longer_than: int, streams: int, window: int, blo
     """(first token row, token count) of the blocks of the tcgen05 prompt kernel over the segments with more than
     ``longer_than`` tokens, the longest first, as device int32 arrays; made once per step and choice of sizes.
 
-    A stream of the kernel takes up to ``tokens`` tokens.  A block whose two ``streams`` have tokens of their own reads keys
-    and values once for both and costs less a row; a block of one stream's tokens, which both walk over, is done sooner and
-    leaves fewer multiprocessors idle at the end.  So the longest blocks are pairs and the rest are not; how many are is
-    what ends first by the costs above, of none, all, and as many as fill the device evenly (``blocks_at_once`` a kv head).
+    A stream of the kernel takes up to ``tokens`` tokens.  A block of two ``streams`` reads keys and values once for both and costs
+    less a row; a block of a single stream is done sooner and leaves fewer multiprocessors idle at the end.  So the longest
+    blocks are pairs and the rest are not; how many are is what ends first by the costs above, of none, all, and as many as
+    fill the device evenly (``blocks_at_once`` a kv head).  A row's result has the same bits in either.
     """
     key = ("attention_tc5_tiles", tokens, longer_than, streams, window, blocks_at_once)
     tiles = ctx.shared.get(key)
@@ -227,7 +227,7 @@ def tc5_tiles(ctx, tokens: int, longer_than: int, streams: int, window: int, blo
                     end = seg.pos_start + t0 + count
                     wide.append((keys_of(end, count), end, seg.q_start + t0, count))
         wide.sort(key=lambda tile: (-tile[0], -tile[1]))        # a stable sort: the order depends on the segments only
-        found = [(TC5_SHARED_TILE * keys + TC5_BLOCK, first, count) for keys, _, first, count in wide]
+        found = [(TC5_SINGLE_TILE * keys + TC5_BLOCK, first, count) for keys, _, first, count in wide]
         if streams == 2 and any(tile[3] > tokens for tile in wide):
             machines = max(1, int(blocks_at_once))
             best = None
@@ -235,13 +235,13 @@ def tc5_tiles(ctx, tokens: int, longer_than: int, streams: int, window: int, blo
                 blocks = []
                 for i, (keys, end, first, count) in enumerate(wide):
                     if count <= tokens:
-                        blocks.append((TC5_SHARED_TILE * keys + TC5_BLOCK, first, count))
+                        blocks.append((TC5_SINGLE_TILE * keys + TC5_BLOCK, first, count))
                     elif i < pairs:
                         blocks.append((TC5_PAIR_TILE * keys + TC5_BLOCK, first, count))
                     else:
                         rest = count - tokens
-                        blocks.append((TC5_SHARED_TILE * keys_of(end, rest) + TC5_BLOCK, first + tokens, rest))
-                        blocks.append((TC5_SHARED_TILE * keys_of(end - rest, tokens) + TC5_BLOCK, first, tokens))
+                        blocks.append((TC5_SINGLE_TILE * keys_of(end, rest) + TC5_BLOCK, first + tokens, rest))
+                        blocks.append((TC5_SINGLE_TILE * keys_of(end - rest, tokens) + TC5_BLOCK, first, tokens))
                 blocks.sort(key=lambda block: -block[0])
                 ends = _makespan([block[0] for block in blocks], machines)
                 if best is None or ends < best:
