@@ -28,9 +28,9 @@
 //                [rows x 64] boxes with the 128-byte swizzle; warp 10 the V tiles likewise.
 //
 // Bound by the chain of a stream's row (scores out of tensor memory, maximum, exponentials, P back, two products), of which two
-// run side by side in a pair: a tile of 128 keys for 256 rows of 128 features takes 2.05 us (2,048 cycles of MMAs and as many of the
+// run side by side in a pair: a tile of 128 keys for 256 rows of 128 features takes 2.25 us (2,048 cycles of MMAs and as many of the
 // special-function units would be 1.1), for a single stream's 128 rows 1.32.  1,531 tokens behind 9,000, 32 heads over 8, B200:
-// 260 us, 0.95 PFLOP/s; single streams alone 299.
+// 270 us, 0.91 PFLOP/s; single streams alone 299.
 // What the parts of a pair gave, us a tile: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
 // step); one elected lane, every wait but P's taken before, and both products issued in a row 2.1 -> 1.9; P in halves 2.3 ->
 // 2.25.  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 -> 1.96, a third stage of K or V nothing.
@@ -95,9 +95,11 @@ constexpr int MMA_WARP = 8, K_WARP = 9, V_WARP = 10;
 constexpr int THREADS = SOFTMAX_THREADS + 4 * 32;                        // 384: registers are dealt to four warps together
 constexpr int SOFTMAX_REGISTERS = 216, OTHER_REGISTERS = 72, LAUNCH_REGISTERS = 168;
 static_assert(SOFTMAX_THREADS * SOFTMAX_REGISTERS + 128 * OTHER_REGISTERS <= THREADS * LAUNCH_REGISTERS, "more registers than the block has");
-constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256), then of a pair O0 [256, 256 + DV) O1 [384, 384 + DV), each
-                                             // P on its S; of a single stream P0 [256,320) P1 [320,384) O [384, 384 + DV)
+constexpr unsigned TMEM_COLS = 512;          // S0 [0,128) S1 [128,256), then of a pair O0 [256, 256 + DV) O1 [384, 384 + DV);
+                                             // of a single stream P0 [256,320) P1 [320,384) O [384, 384 + DV)
 constexpr unsigned O_COL = 256, P_COL = 256, SINGLE_O_COL = 384;
+constexpr bool P_ON_S = DV > 64;             // a pair's P: over the scores it was made of, or beside its O where that is narrow
+constexpr unsigned PAIR_P_COL = P_ON_S ? 0 : O_COL + 64;              // of stream 0; stream 1's 128 further
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.f;          // log2 of the growth of a row maximum that forces a rescale
 constexpr long long WAIT_CYCLES = 3000000000LL;         // about 1.5 s at 2 GHz
@@ -133,7 +135,7 @@ struct Barriers {
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];
     unsigned long long s_full[2], s_empty[2];                        // of a pair's streams, of a single stream's two accumulators
     unsigned long long p_full[2][2];                                 // [stream or buffer][half of the keys, of a pair]
-    unsigned long long pv_done, o_full;                              // of a single stream's tile; of all
+    unsigned long long pv_done, p_read[2], o_full;                   // of a single stream's tile, of a pair's [stream]; of all
 };
 
 // ------------------------------------------------------------------------------------------ a row's keys, half a tile at a time
@@ -268,6 +270,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             mbar_init(&bars.v_empty[s], 1);
             mbar_init(&bars.s_full[s], 1);
             mbar_init(&bars.s_empty[s], SOFTMAX_WARPS);
+            mbar_init(&bars.p_read[s], 1);
             mbar_init(&bars.p_full[s][0], pair ? STREAM_WARPS : SOFTMAX_WARPS);
             mbar_init(&bars.p_full[s][1], STREAM_WARPS);
         }
@@ -363,8 +366,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 m_used = m_new;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    // on this row's scores, which are in registers
-                    sum[h] += probabilities(sc[h], unit, m_used, lane_base + side * KEYS + h * (HALF / 2));
+                    sum[h] += probabilities(sc[h], unit, m_used, lane_base + PAIR_P_COL + side * 128 + h * (HALF / 2));
                     tmem_store_wait();
                     tc_fence_before();
                     __syncwarp();
@@ -520,7 +522,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 }
                 tc_fence_after();
                 if (pair) {
-                    const unsigned o = O_COL + acc * 128, p = acc * KEYS;
+                    const unsigned o = O_COL + acc * 128, p = PAIR_P_COL + acc * 128;
                     if (elect_one()) issue_pv(o, p, s, 0, KEYS / 32, i < 2);
                     __syncwarp();
                     if (!wait(&bars.p_full[acc][1], (i >> 1) & 1)) { alive = false; break; }
@@ -528,10 +530,16 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                     if (elect_one()) {
                         issue_pv(o, p, s, KEYS / 32, KEYS / 16, i < 2);
                         if (acc == 1) umma_commit(&bars.v_empty[s]);
-                        // the stream's next scores go where its P lies, behind the product that reads it
-                        if (more) issue_qk(acc, acc, next_s);
+                        if (P_ON_S) umma_commit(&bars.p_read[acc]);
                         if (i + 1 == n_items) umma_commit(&bars.o_full);
                     }
+                    __syncwarp();
+                    // The stream's next scores go where its P lies.  Products into different accumulators have no promised order, so
+                    // the ones that read P end first: 2.25 us a tile in place of 2.05.  (Held back behind the other stream's product
+                    // where that could go on 2.37; the upper 64 keys' scores, which lie beside P, at once 2.4.)
+                    if (P_ON_S && more && !wait(&bars.p_read[acc], (i >> 1) & 1)) { alive = false; break; }
+                    tc_fence_after();
+                    if (more && elect_one()) issue_qk(acc, acc, next_s);
                     __syncwarp();
                 } else {
                     if (elect_one()) {

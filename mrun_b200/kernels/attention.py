@@ -190,7 +190,7 @@ def prefill_tiles(ctx, tokens_per_tile: int, longer_than: int = 0, up_to: int = 
 
 # A block of the tcgen05 prompt kernel, us: what it takes whatever its keys, a tile of 128 keys for a pair of streams, and for a
 # single stream (32 heads over 8 of 128 features, B200).
-TC5_BLOCK, TC5_PAIR_TILE, TC5_SINGLE_TILE = 5.0, 2.05, 1.32
+TC5_BLOCK, TC5_PAIR_TILE, TC5_SINGLE_TILE = 5.0, 2.25, 1.32
 
 
 def _makespan(costs, machines: int) -> float:
