@@ -31,7 +31,7 @@ import torch
 
 from . import lib as _lib
 from . import ops
-from .ops import _c_float, _c_int, _c_long, _ptr, _stream
+from .ops import _address, _queue
 
 COUNTER_CAPACITY = 1 << 16     # (token, kv head) pairs of one decode launch that may be split
 
@@ -156,9 +156,9 @@ def decode_plan(ctx, library, window: int, kv_heads: int, blocks: int, splits: i
         n = positions.shape[0]
         prefix = positions.new_empty(2 * (n + 1) + 1, dtype=torch.int32)
         assignment = positions.new_empty(blocks * 8, dtype=torch.int32)
-        library.call("mrun_attn_decode_plan", _ptr(positions), n, window,
-                     kv_heads, blocks, MIN_TILES, splits, _ptr(prefix),
-                     _ptr(assignment), _stream())
+        library.call("mrun_attn_decode_plan", _address(positions), n, window,
+                     kv_heads, blocks, MIN_TILES, splits, _address(prefix),
+                     _address(assignment), _queue())
         plan = ctx.shared[key] = (prefix, assignment)
     return plan
 
@@ -391,7 +391,7 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
     pages, kv_heads, page_size, head_dim = cache.k.shape
     v_dim = cache.v.shape[3]
     ops.check_sink(sink, heads)
-    formed = ctypes.byref(form) if form is not None else _ptr(None)
+    formed = ctypes.byref(form) if form is not None else _address(None)
     ratio = heads // kv_heads
     if (value_dim and cache.v is cache.k and kv_heads == 1 and window == 0 and raw is None and sink is None and form is None
             and (not supports_tensor_cores(q.dtype, head_dim, ratio)
@@ -408,11 +408,11 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
             cols = int(_lib.core()._dll.mrun_latent_attention_wide_piece_cols(value_dim))
             part_o = q.new_empty((blocks * splits, 16, cols), dtype=torch.float32)
             part_ml = q.new_empty((blocks * splits, 16, 2), dtype=torch.float32)
-        _lib.core().call("mrun_latent_attention_wide", _ptr(q), q_stride, _ptr(out), _ptr(cache.k),
-                         _ptr(group.block_tables), group.max_blocks, _ptr(ctx.token_slot), _ptr(ctx.positions),
+        _lib.core().call("mrun_latent_attention_wide", _address(q), q_stride, _address(out), _address(cache.k),
+                         _address(group.block_tables), group.max_blocks, _address(ctx.token_slot), _address(ctx.positions),
                          ctx.num_tokens, heads, head_dim, value_dim, page_size,
-                         pages * page_size, scale, splits, _ptr(part_o), _ptr(part_ml),
-                         _stream())
+                         pages * page_size, scale, splits, _address(part_o), _address(part_ml),
+                         _queue())
         return out
     if sink is None and form is None and f32_tiles_ok(q, q_stride, out, cache, ratio):
         return _paged_attention_f32(q, q_stride, out, cache, group, ctx, heads, scale, window)
@@ -421,23 +421,23 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
                                            ctx.token_slot, ctx.positions, heads, scale, window, sink=sink, form=form)
     library = _lib.attention(head_dim, v_dim, form is not None)
     tokens = ctx.num_tokens
-    common = (_ptr(cache.k), _ptr(cache.v), _ptr(group.block_tables), group.max_blocks,
-              _ptr(ctx.token_slot), _ptr(ctx.positions))
+    common = (_address(cache.k), _address(cache.v), _address(group.block_tables), group.max_blocks,
+              _address(ctx.token_slot), _address(ctx.positions))
     tail = (heads, kv_heads, head_dim, page_size, scale,
-            window, _ptr(sink), _stream())
+            window, _address(sink), _queue())
     if ctx.all_decode and ratio <= 16:
         if tokens * kv_heads > COUNTER_CAPACITY:
             raise ValueError(f"a decode step of {tokens} tokens x {kv_heads} kv heads exceeds {COUNTER_CAPACITY} pairs")
-        fused = (0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None))
+        fused = (0, _address(None), _address(None), 0.0, _address(None), 0, _address(None))
         if raw is not None:
             q_weight, k_weight, eps, rot, rotary_dim, slots = raw
-            fused = (1, _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot), rotary_dim,
-                     _ptr(slots))
+            fused = (1, _address(q_weight), _address(k_weight), eps, _address(rot), rotary_dim,
+                     _address(slots))
         cluster = decode_cluster(library, ratio, page_size, tokens, kv_heads, ctx.max_kv_len)
         if cluster:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_cluster", _ptr(q), q_stride, _ptr(out), *common, tokens,
-                         cluster, *tail[:-1], *fused, _ptr(None), pages, formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_decode_cluster", _address(q), q_stride, _address(out), *common, tokens,
+                         cluster, *tail[:-1], *fused, _address(None), pages, formed, _address(status), tail[-1])
             return out
         tma = decode_uses_tma(library, ratio, page_size)
         blocks, splits = decode_launch(tokens, kv_heads, decode_slots(library, ratio, page_size))
@@ -447,10 +447,10 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         extra = (formed,)
         if tma:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            extra = (_ptr(None), pages, formed, _ptr(status))
-        library.call("mrun_attn_decode_tma" if tma else "mrun_attn_decode", _ptr(q), q_stride, _ptr(out),
-                     *common, _ptr(prefix), _ptr(assignment), tokens, _ptr(part_o), _ptr(part_ml),
-                     _ptr(_split_counters(q.device)), blocks, *tail[:-1], *fused, *extra, tail[-1])
+            extra = (_address(None), pages, formed, _address(status))
+        library.call("mrun_attn_decode_tma" if tma else "mrun_attn_decode", _address(q), q_stride, _address(out),
+                     *common, _address(prefix), _address(assignment), tokens, _address(part_o), _address(part_ml),
+                     _address(_split_counters(q.device)), blocks, *tail[:-1], *fused, *extra, tail[-1])
         return out
     if raw is not None:
         raise ValueError("raw q, k, v rows are taken by the decode kernel only")
@@ -464,11 +464,11 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         cluster = decode_cluster(library, ratio, page_size, n_single, kv_heads, ctx.max_kv_len) if n_single else 0
         if cluster:
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_cluster", _ptr(q), q_stride, _ptr(out), _ptr(cache.k), _ptr(cache.v),
-                         _ptr(group.block_tables), group.max_blocks, _ptr(row_slots), _ptr(row_positions),
+            library.call("mrun_attn_decode_cluster", _address(q), q_stride, _address(out), _address(cache.k), _address(cache.v),
+                         _address(group.block_tables), group.max_blocks, _address(row_slots), _address(row_positions),
                          n_single, cluster, *tail[:-1],
-                         0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None),
-                         _ptr(rows), pages, formed, _ptr(status), tail[-1])
+                         0, _address(None), _address(None), 0.0, _address(None), 0, _address(None),
+                         _address(rows), pages, formed, _address(status), tail[-1])
             shortest = 1
         elif n_single and n_single * kv_heads <= COUNTER_CAPACITY:
             blocks, splits = decode_launch(n_single, kv_heads, decode_slots(library, ratio, page_size))
@@ -476,12 +476,12 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
             part_ml = q.new_empty((blocks, 2, 16, 2), dtype=torch.float32)
             prefix, assignment = decode_plan(ctx, library, window, kv_heads, blocks, splits, positions=row_positions)
             status = ops.status_word(q.device, "attn_decode_tma", {1: "the TMA producer", 2: "the consumer warps"})
-            library.call("mrun_attn_decode_tma", _ptr(q), q_stride, _ptr(out), _ptr(cache.k), _ptr(cache.v),
-                         _ptr(group.block_tables), group.max_blocks, _ptr(row_slots), _ptr(row_positions),
-                         _ptr(prefix), _ptr(assignment), n_single, _ptr(part_o), _ptr(part_ml),
-                         _ptr(_split_counters(q.device)), blocks, *tail[:-1],
-                         0, _ptr(None), _ptr(None), 0.0, _ptr(None), 0, _ptr(None),
-                         _ptr(rows), pages, formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_decode_tma", _address(q), q_stride, _address(out), _address(cache.k), _address(cache.v),
+                         _address(group.block_tables), group.max_blocks, _address(row_slots), _address(row_positions),
+                         _address(prefix), _address(assignment), n_single, _address(part_o), _address(part_ml),
+                         _address(_split_counters(q.device)), blocks, *tail[:-1],
+                         0, _address(None), _address(None), 0.0, _address(None), 0, _address(None),
+                         _address(rows), pages, formed, _address(status), tail[-1])
             shortest = 1
     short_up_to = 1 << 30
     if prefill_uses_tcgen05(library, ratio, page_size):
@@ -492,13 +492,13 @@ def paged_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache, gr
         if n_tiles:
             status = ops.status_word(q.device, "attn_prefill_tc5",
                                      {1: "a key/value loader", 2: "the MMA issuer", 3: "the softmax warps"})
-            library.call("mrun_attn_prefill_tc5", _ptr(q), q_stride, _ptr(out), *common, _ptr(first),
-                         _ptr(count), n_tiles, *tail[:-1], pages, formed, _ptr(status), tail[-1])
+            library.call("mrun_attn_prefill_tc5", _address(q), q_stride, _address(out), *common, _address(first),
+                         _address(count), n_tiles, *tail[:-1], pages, formed, _address(status), tail[-1])
     if short_up_to > shortest:
         first, count, n_tiles = prefill_tiles(ctx, 64 // ratio, longer_than=shortest, up_to=short_up_to)
         if n_tiles:
-            library.call("mrun_attn_prefill", _ptr(q), q_stride, _ptr(out), *common, _ptr(first),
-                         _ptr(count), n_tiles, *tail[:-1], formed, tail[-1])
+            library.call("mrun_attn_prefill", _address(q), q_stride, _address(out), *common, _address(first),
+                         _address(count), n_tiles, *tail[:-1], formed, tail[-1])
     return out
 
 

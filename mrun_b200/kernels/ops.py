@@ -24,14 +24,26 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise KernelError(f"dtype {dtype} has no kernel (float32 and bfloat16 do)")
 
 
-def _stream() -> int:
+def _queue() -> int:
     """The current stream of the current device.  Asked for by its raw handle: a Stream object took 29 % of an
     uncaptured step's host time (a mixer's decode step of five kernels on B200: 119 us a pass, 96 without)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
+def _address(t: Optional[torch.Tensor]) -> Optional[int]:
+    """For :meth:`Library.call` only, which knows the parameters' types: ctypes passes a plain number as a 32-bit int wherever
+    they are not declared."""
     return None if t is None else t.data_ptr()
+
+
+def _stream() -> ctypes.c_void_p:
+    """The current stream for a function of any library, its parameters' types declared or not."""
+    return ctypes.c_void_p(_queue())
+
+
+def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
+    """A tensor's address for a function of any library, its parameters' types declared or not."""
+    return ctypes.c_void_p(_address(t))
 
 
 def _check(t: torch.Tensor, name: str, dtype: Optional[torch.dtype] = None, dense: bool = True) -> None:
@@ -50,8 +62,8 @@ def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor) -> torch.Te
     tokens = ids.numel()
     if out.shape != (tokens, hidden):
         raise KernelError(f"embed: out is {tuple(out.shape)}, expected {(tokens, hidden)}")
-    _lib.core().call("mrun_embed", _ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out),
-                     tokens, hidden, vocab, _stream())
+    _lib.core().call("mrun_embed", _address(table), dtype_code(table.dtype), _address(ids), _address(out),
+                     tokens, hidden, vocab, _queue())
     return out
 
 
@@ -78,9 +90,9 @@ def add_rmsnorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: torc
     if weight.numel() != hidden or out.shape != (n_rows, hidden):
         raise KernelError(f"add_rmsnorm: weight {tuple(weight.shape)}, out {tuple(out.shape)}, "
                           f"expected hidden {hidden}, rows {n_rows}")
-    _lib.core().call("mrun_add_rmsnorm", _ptr(resid), _ptr(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
-                     _ptr(weight), eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden,
-                     _ptr(extra), _ptr(share), _stream())
+    _lib.core().call("mrun_add_rmsnorm", _address(resid), _address(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
+                     _address(weight), eps, _address(out), dtype_code(out.dtype), _address(rows), n_rows, hidden,
+                     _address(extra), _address(share), _queue())
     return out
 
 
@@ -89,8 +101,8 @@ def add_scaled_rows(y: torch.Tensor, x: torch.Tensor, share: torch.Tensor) -> to
     _check(y, "y"); _check(x, "x"); _check(share, "share", torch.float32)
     if y.dim() != 2 or x.shape != y.shape or share.numel() != y.shape[0]:
         raise KernelError(f"add_scaled_rows: y {tuple(y.shape)}, x {tuple(x.shape)}, share {tuple(share.shape)}")
-    _lib.core().call("mrun_add_scaled_rows", _ptr(y), dtype_code(y.dtype), _ptr(x), dtype_code(x.dtype), _ptr(share),
-                     y.shape[0], y.shape[1], _stream())
+    _lib.core().call("mrun_add_scaled_rows", _address(y), dtype_code(y.dtype), _address(x), dtype_code(x.dtype), _address(share),
+                     y.shape[0], y.shape[1], _queue())
     return y
 
 
@@ -117,9 +129,9 @@ def add_layernorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: to
     if weight.numel() != hidden or out.shape != (n_rows, hidden):
         raise KernelError(f"add_layernorm: weight {tuple(weight.shape)}, out {tuple(out.shape)}, "
                           f"expected hidden {hidden}, rows {n_rows}")
-    _lib.core().call("mrun_add_layernorm", _ptr(resid), _ptr(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
-                     _ptr(weight), _ptr(bias), eps, _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows,
-                     hidden, _stream())
+    _lib.core().call("mrun_add_layernorm", _address(resid), _address(delta), dtype_code(delta.dtype if delta is not None else out.dtype),
+                     _address(weight), _address(bias), eps, _address(out), dtype_code(out.dtype), _address(rows), n_rows,
+                     hidden, _queue())
     return out
 
 
@@ -153,9 +165,9 @@ def post_layernorm_add(stream: torch.Tensor, pending, next_weight: Optional[torc
             raise KernelError(f"post_layernorm_add: out {tuple(out.shape)}, expected {(n_rows, hidden)}")
     if rows is not None:
         _check(rows, "rows", torch.int32)
-    _lib.core().call("mrun_post_layernorm_add", _ptr(stream), _ptr(branch), _ptr(weight), _ptr(bias), eps,
-                     _ptr(next_weight), _ptr(next_bias), next_eps, _ptr(out), code, _ptr(rows),
-                     n_rows, hidden, _stream())
+    _lib.core().call("mrun_post_layernorm_add", _address(stream), _address(branch), _address(weight), _address(bias), eps,
+                     _address(next_weight), _address(next_bias), next_eps, _address(out), code, _address(rows),
+                     n_rows, hidden, _queue())
     return out
 
 
@@ -169,8 +181,8 @@ def pair_norm_mean(a: torch.Tensor, b: torch.Tensor, weight_a: torch.Tensor, wei
     if b.shape != a.shape or weight_a.numel() != hidden or weight_b.numel() != hidden:
         raise KernelError(f"pair_norm_mean: a {tuple(a.shape)}, b {tuple(b.shape)}, weights {weight_a.numel()} / {weight_b.numel()}")
     out = torch.empty_like(a)
-    _lib.core().call("mrun_pair_norm_mean", _ptr(a), _ptr(b), _ptr(weight_a), _ptr(weight_b), eps,
-                     share, _ptr(out), rows, hidden, _stream())
+    _lib.core().call("mrun_pair_norm_mean", _address(a), _address(b), _address(weight_a), _address(weight_b), eps,
+                     share, _address(out), rows, hidden, _queue())
     return out
 
 
@@ -190,9 +202,9 @@ def pair_norm_add_layernorm(resid: torch.Tensor, pending, weight: torch.Tensor, 
             or pending.weight_a.numel() != hidden or pending.weight_b.numel() != hidden or out.shape != (n_rows, hidden):
         raise KernelError(f"pair_norm_add_layernorm: resid {tuple(resid.shape)}, a {tuple(pending.a.shape)}, "
                           f"b {tuple(pending.b.shape)}, out {tuple(out.shape)}")
-    _lib.core().call("mrun_pair_norm_add_layernorm", _ptr(resid), _ptr(pending.a), _ptr(pending.b), _ptr(pending.weight_a),
-                     _ptr(pending.weight_b), pending.eps, pending.share, _ptr(weight), eps,
-                     _ptr(out), dtype_code(out.dtype), _ptr(rows), n_rows, hidden, _stream())
+    _lib.core().call("mrun_pair_norm_add_layernorm", _address(resid), _address(pending.a), _address(pending.b), _address(pending.weight_a),
+                     _address(pending.weight_b), pending.eps, pending.share, _address(weight), eps,
+                     _address(out), dtype_code(out.dtype), _address(rows), n_rows, hidden, _queue())
     return out
 
 
@@ -204,8 +216,8 @@ def rotary_table(positions: torch.Tensor, inv_freq: torch.Tensor, out: torch.Ten
     tokens, half = positions.numel(), inv_freq.numel()
     if out.shape != (tokens, half, 2):
         raise KernelError(f"rotary_table: out is {tuple(out.shape)}, expected {(tokens, half, 2)}")
-    _lib.core().call("mrun_rotary_table", _ptr(positions), _ptr(inv_freq), _ptr(out), tokens,
-                     half, magnitude, _stream())
+    _lib.core().call("mrun_rotary_table", _address(positions), _address(inv_freq), _address(out), tokens,
+                     half, magnitude, _queue())
     return out
 
 
@@ -239,10 +251,10 @@ def qk_norm_rope_cache(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: i
             if c.dim() != 4 or c.shape[1:] != (kv_heads, page_size, head_dim):
                 raise KernelError(f"qk_norm_rope_cache: {name} is {tuple(c.shape)}, expected "
                                   f"[pages, {kv_heads}, {page_size}, {head_dim}]")
-    _lib.core().call("mrun_qk_norm_rope_cache", _ptr(qkv), dtype_code(qkv.dtype), _ptr(q_weight),
-                     _ptr(k_weight), eps, _ptr(rot), rotary_dim if rot is not None else 0,
-                     _ptr(slots), _ptr(k_cache), _ptr(v_cache), tokens, heads,
-                     kv_heads, head_dim, page_size, _stream())
+    _lib.core().call("mrun_qk_norm_rope_cache", _address(qkv), dtype_code(qkv.dtype), _address(q_weight),
+                     _address(k_weight), eps, _address(rot), rotary_dim if rot is not None else 0,
+                     _address(slots), _address(k_cache), _address(v_cache), tokens, heads,
+                     kv_heads, head_dim, page_size, _queue())
 
 
 def proj_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: int, kv_heads: int, dim: int,
@@ -275,11 +287,11 @@ def proj_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, he
     width = x.shape[1]
     if q_off + heads * dim > width or (k_off >= 0 and (k_off + kv_heads * dim > width or v_off + kv_heads * vdim > width)):
         raise KernelError("proj_norm_rope_cache: the heads do not fit the rows")
-    _lib.core().call("mrun_proj_norm_rope_cache", _ptr(x), ld, q_off, k_off, v_off,
-                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot),
+    _lib.core().call("mrun_proj_norm_rope_cache", _address(x), ld, q_off, k_off, v_off,
+                     dtype_code(x.dtype), _address(q_weight), _address(k_weight), eps, _address(rot),
                      rotary_dim if rot is not None else 0, PAIRINGS[pairing],
-                     _ptr(slots if k_off >= 0 else None), _ptr(k_cache), _ptr(v_cache), tokens, heads,
-                     kv_heads, dim, vdim, page_size, _stream())
+                     _address(slots if k_off >= 0 else None), _address(k_cache), _address(v_cache), tokens, heads,
+                     kv_heads, dim, vdim, page_size, _queue())
 
 
 def head_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: int, kv_heads: int, dim: int,
@@ -326,12 +338,12 @@ def head_norm_rope_cache(x: torch.Tensor, q_off: int, k_off: int, v_off: int, he
     width = x.shape[1]
     if q_off + heads * dim > width or k_off + kv_heads * dim > width or (v_off >= 0 and v_off + kv_heads * vdim > width):
         raise KernelError("head_norm_rope_cache: the heads do not fit the rows")
-    _lib.core().call("mrun_head_norm_rope_cache", _ptr(x), ld, q_off, k_off, v_off,
-                     dtype_code(x.dtype), _ptr(q_weight), _ptr(k_weight), eps, _ptr(rot),
-                     rotary_dim if rot is not None else 0, PAIRINGS[pairing], _ptr(slots), _ptr(k_cache),
-                     _ptr(v_cache), tokens, heads, kv_heads, dim, vdim,
-                     page_size, _ptr(bias), _ptr(first), strides[1], share, _ptr(keep),
-                     strides[0], _stream())
+    _lib.core().call("mrun_head_norm_rope_cache", _address(x), ld, q_off, k_off, v_off,
+                     dtype_code(x.dtype), _address(q_weight), _address(k_weight), eps, _address(rot),
+                     rotary_dim if rot is not None else 0, PAIRINGS[pairing], _address(slots), _address(k_cache),
+                     _address(v_cache), tokens, heads, kv_heads, dim, vdim,
+                     page_size, _address(bias), _address(first), strides[1], share, _address(keep),
+                     strides[0], _queue())
 
 
 def check_sink(sink: Optional[torch.Tensor], heads: int) -> None:
@@ -374,12 +386,12 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
         gate_stride = _strided_rows(gate, "gate")
         if gate.shape != (tokens, heads) or gate.dtype != q.dtype:
             raise KernelError(f"paged_attention: gate is {tuple(gate.shape)} {gate.dtype}, expected {(tokens, heads)} {q.dtype}")
-    _lib.core().call("mrun_paged_attention_generic", _ptr(q), q_stride, _ptr(out), _ptr(k_cache),
-                     _ptr(v_cache), dtype_code(q.dtype), _ptr(block_tables), block_tables.shape[1],
-                     _ptr(token_slot), _ptr(positions), tokens, heads, kv_heads,
+    _lib.core().call("mrun_paged_attention_generic", _address(q), q_stride, _address(out), _address(k_cache),
+                     _address(v_cache), dtype_code(q.dtype), _address(block_tables), block_tables.shape[1],
+                     _address(token_slot), _address(positions), tokens, heads, kv_heads,
                      head_dim, value_dim, page_size, pages * kv_heads * page_size,
-                     scale, window, _ptr(sink), _ptr(gate), gate_stride,
-                     ctypes.byref(form) if form is not None else _ptr(None), _stream())
+                     scale, window, _address(sink), _address(gate), gate_stride,
+                     ctypes.byref(form) if form is not None else _address(None), _queue())
     return out
 
 
@@ -410,10 +422,10 @@ def paged_attention_f32(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cac
                 raise KernelError(f"paged_attention_f32: {name} has {t.numel()} entries for {tiles} tiles")
     if first is None and tiles != tokens:
         raise KernelError(f"paged_attention_f32: {tiles} tiles of single tokens for {tokens} tokens")
-    _lib.core().call("mrun_paged_attention_f32", _ptr(q), q_stride, _ptr(out), _ptr(k_cache), _ptr(v_cache),
-                     _ptr(block_tables), block_tables.shape[1], _ptr(token_slot), _ptr(positions), _ptr(first), _ptr(count),
+    _lib.core().call("mrun_paged_attention_f32", _address(q), q_stride, _address(out), _address(k_cache), _address(v_cache),
+                     _address(block_tables), block_tables.shape[1], _address(token_slot), _address(positions), _address(first), _address(count),
                      tiles, tile_tokens, heads, kv_heads, head_dim, page_size,
-                     pages * kv_heads * page_size, scale, window, _stream())
+                     pages * kv_heads * page_size, scale, window, _queue())
     return out
 
 
@@ -435,8 +447,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False, 
     tokens, inter = out.shape
     if gate_up.shape != (tokens, 2 * inter):
         raise KernelError(f"swiglu: gate_up {tuple(gate_up.shape)} vs out {tuple(out.shape)}")
-    _lib.core().call("mrun_swiglu", _ptr(gate_up), _ptr(out), dtype_code(out.dtype), tokens,
-                     inter, 8 if interleaved else 0, gate_code(activation), _stream())
+    _lib.core().call("mrun_swiglu", _address(gate_up), _address(out), dtype_code(out.dtype), tokens,
+                     inter, 8 if interleaved else 0, gate_code(activation), _queue())
     return out
 
 
@@ -445,8 +457,8 @@ def add_bias(y: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
     _check(y, "y"); _check(bias, "bias", torch.float32)
     if y.dim() != 2 or bias.numel() != y.shape[1]:
         raise KernelError(f"add_bias: y {tuple(y.shape)} vs bias {tuple(bias.shape)}")
-    _lib.core().call("mrun_add_bias", _ptr(y), dtype_code(y.dtype), _ptr(bias), y.shape[0],
-                     y.shape[1], _stream())
+    _lib.core().call("mrun_add_bias", _address(y), dtype_code(y.dtype), _address(bias), y.shape[0],
+                     y.shape[1], _queue())
     return y
 
 
@@ -490,8 +502,8 @@ class NormedRows:
     def finish(self) -> torch.Tensor:
         tokens, width = self.xw.shape
         out = torch.empty_like(self.xw)
-        _lib.core().call("mrun_norm_finish", _ptr(self.xw), _ptr(self.sums), self.eps, _ptr(out),
-                         tokens, width, _stream())
+        _lib.core().call("mrun_norm_finish", _address(self.xw), _address(self.sums), self.eps, _address(out),
+                         tokens, width, _queue())
         return out
 
 
@@ -602,8 +614,8 @@ PENDING = (PendingLinear, PendingPostNorm, PendingPairNorm, PendingPostLayerNorm
 def _normed(x):
     """(rows, totals pointer, eps) of a product's x, which may be :class:`NormedRows`."""
     if isinstance(x, NormedRows):
-        return x.xw, _ptr(x.sums), x.eps
-    return x, _ptr(None), 0.0
+        return x.xw, _address(x.sums), x.eps
+    return x, _address(None), 0.0
 
 
 def gemm_skinny(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
@@ -621,11 +633,11 @@ def gemm_skinny(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16,
     if w.shape[1] != k:
         raise KernelError(f"gemm_skinny: x {tuple(x.shape)} vs w {tuple(w.shape)}")
     out = x.new_empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype)
-    _lib.core().call("mrun_gemm_skinny", _ptr(x), _ptr(w), _ptr(out), dtype_code(out_dtype),
+    _lib.core().call("mrun_gemm_skinny", _address(x), _address(w), _address(out), dtype_code(out_dtype),
                      gate_code(activation) if swiglu_rows else 0, m, n, k,
                      x.stride(0) if m > 1 else max(k, x.stride(0)), out.shape[1],
-                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), rows, _ptr(None), 0, _ptr(None),
-                     _stream())
+                     sums, eps, _address(None), _address(None), _address(None), _address(None), rows, _address(None), 0, _address(None),
+                     _queue())
     return out
 
 
@@ -662,13 +674,13 @@ def linear_into_norm(pending: PendingLinear, resid: torch.Tensor, weight: torch.
             add_scaled_rows(resid, extra.contiguous(), share)
     xw = x.new_empty((m, n), dtype=torch.bfloat16)
     out_sums = RowSums.take(x.device, m)
-    head = (_ptr(x), _ptr(w), _ptr(None), dtype_code(torch.bfloat16), 0, m, n, k,
-            x.stride(0) if m > 1 else max(k, x.stride(0)), n, in_sums, in_eps, _ptr(resid),
-            _ptr(weight), _ptr(xw), _ptr(out_sums))
+    head = (_address(x), _address(w), _address(None), dtype_code(torch.bfloat16), 0, m, n, k,
+            x.stride(0) if m > 1 else max(k, x.stride(0)), n, in_sums, in_eps, _address(resid),
+            _address(weight), _address(xw), _address(out_sums))
     if skinny:
-        _lib.core().call("mrun_gemm_skinny", *head, rows, _ptr(extra), ld_extra, _ptr(share), _stream())
+        _lib.core().call("mrun_gemm_skinny", *head, rows, _address(extra), ld_extra, _address(share), _queue())
     else:
-        _lib.core().call("mrun_gemm_tc5", *head, 0, _ptr(_tc5_status(x.device)), _stream())
+        _lib.core().call("mrun_gemm_tc5", *head, 0, _address(_tc5_status(x.device)), _queue())
     return NormedRows(xw, out_sums, eps)
 
 
@@ -686,8 +698,8 @@ def gemm_f32_nt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     _check(out, "out", torch.float32)
     if out.shape != (m, n):
         raise KernelError(f"gemm_f32_nt: out is {tuple(out.shape)}, expected {(m, n)}")
-    _lib.core().call("mrun_gemm_f32_nt", _ptr(x), _ptr(w), _ptr(out), m, n, k,
-                     x.stride(0) if m > 1 else k, n, _stream())
+    _lib.core().call("mrun_gemm_f32_nt", _address(x), _address(w), _address(out), m, n, k,
+                     x.stride(0) if m > 1 else k, n, _queue())
     return out
 
 
@@ -727,9 +739,9 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
                                                    4: "the MMA issuer", 5: "the sums"})
     for at in range(0, m, rows):
         part, to = x[at:at + rows], out[at:at + rows]
-        _lib.core().call("mrun_gemm_f32_tc", _ptr(part), _ptr(w), _ptr(to), _ptr(parts), part.shape[0], n, k,
-                         x.stride(0) if m > 1 else k, n, ranges, tile, cluster, _ptr(status),
-                         _stream())
+        _lib.core().call("mrun_gemm_f32_tc", _address(part), _address(w), _address(to), _address(parts), part.shape[0], n, k,
+                         x.stride(0) if m > 1 else k, n, ranges, tile, cluster, _address(status),
+                         _queue())
     return out
 
 
@@ -780,11 +792,11 @@ def gemm_tc5(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, swiglu
     if w.shape[1] != k:
         raise KernelError(f"gemm_tc5: x {tuple(x.shape)} vs w {tuple(w.shape)}")
     out = x.new_empty((m, n // 2 if swiglu_rows else n), dtype=out_dtype)
-    _lib.core().call("mrun_gemm_tc5", _ptr(x), _ptr(w), _ptr(out), dtype_code(out_dtype),
+    _lib.core().call("mrun_gemm_tc5", _address(x), _address(w), _address(out), dtype_code(out_dtype),
                      gate_code(activation) if swiglu_rows else 0, m, n, k,
                      x.stride(0) if m > 1 else max(k, x.stride(0)), out.shape[1],
-                     sums, eps, _ptr(None), _ptr(None), _ptr(None), _ptr(None), split,
-                     _ptr(_tc5_status(x.device)), _stream())
+                     sums, eps, _address(None), _address(None), _address(None), _address(None), split,
+                     _address(_tc5_status(x.device)), _queue())
     return out
 
 
@@ -846,8 +858,8 @@ def plain_act(x: torch.Tensor, activation: str, out_dtype: Optional[torch.dtype]
     """act(x) element by element in 32-bit."""
     _check(x, "x")
     out = x.new_empty(x.shape, dtype=out_dtype or x.dtype)
-    _lib.core().call("mrun_plain_act", _ptr(x), dtype_code(x.dtype), _ptr(out), dtype_code(out.dtype),
-                     x.numel(), ACTIVATIONS[activation], _stream())
+    _lib.core().call("mrun_plain_act", _address(x), dtype_code(x.dtype), _address(out), dtype_code(out.dtype),
+                     x.numel(), ACTIVATIONS[activation], _queue())
     return out
 
 
@@ -888,11 +900,11 @@ def linears_batched(x: torch.Tensor, w: torch.Tensor, activation: Optional[str] 
         ld_gate = _strided_rows(gate, "gate")
         if gate.shape != (rows, batch) or gate.dtype != x.dtype:
             raise KernelError(f"linears_batched: gate {tuple(gate.shape)} {gate.dtype}")
-    _lib.core().call("mrun_gemm_skinny_batched", _ptr(x), _ptr(w), _ptr(out), dtype_code(out.dtype),
+    _lib.core().call("mrun_gemm_skinny_batched", _address(x), _address(w), _address(out), dtype_code(out.dtype),
                      ACTIVATIONS[activation] if activation else 0, batch, rows, n, k,
                      x.stride(0) if rows > 1 else max(k, x.stride(0)), out.stride(0) if rows > 1 else max(n, out.stride(0)),
-                     x.stride(1) if batch > 1 else 0, out.stride(1) if batch > 1 else n, _ptr(None), _ptr(None), 0,
-                     0, 0, 0.0, _ptr(gate), ld_gate, _ptr(None), 0.0, _stream())
+                     x.stride(1) if batch > 1 else 0, out.stride(1) if batch > 1 else n, _address(None), _address(None), 0,
+                     0, 0, 0.0, _address(gate), ld_gate, _address(None), 0.0, _queue())
     return out
 
 
@@ -918,11 +930,11 @@ def linear_blended(x, w: torch.Tensor, bias: Optional[torch.Tensor] = None, blen
         if rows.shape[0] != m or rows.dtype != torch.bfloat16:
             raise KernelError(f"linear_blended: blend {tuple(rows.shape)} {rows.dtype}")
     out = x.new_empty((m, n), dtype=torch.bfloat16)
-    _lib.core().call("mrun_gemm_skinny_batched", _ptr(x), _ptr(w), _ptr(out), dtype_code(out.dtype),
+    _lib.core().call("mrun_gemm_skinny_batched", _address(x), _address(w), _address(out), dtype_code(out.dtype),
                      ACTIVATIONS[activation] if activation else 0, 1,
                      m, n, k, x.stride(0) if m > 1 else max(k, x.stride(0)), n, 0,
-                     n, _ptr(bias), _ptr(rows), ld_rows, column, columns, share, _ptr(None),
-                     0, sums, eps, _stream())
+                     n, _address(bias), _address(rows), ld_rows, column, columns, share, _address(None),
+                     0, sums, eps, _queue())
     return out
 
 
@@ -968,8 +980,8 @@ def sample(logits: torch.Tensor, out: torch.Tensor, temperature: Optional[torch.
                 raise KernelError(f"sample: {name} has {t.numel()} entries for {rows} rows")
     if out.numel() < rows:
         raise KernelError(f"sample: out has {out.numel()} entries for {rows} rows")
-    _lib.core().call("mrun_sample", _ptr(logits), rows, vocab, _ptr(temperature), _ptr(top_p),
-                     _ptr(top_k), _ptr(min_p), _ptr(keys), _ptr(out), _stream())
+    _lib.core().call("mrun_sample", _address(logits), rows, vocab, _address(temperature), _address(top_p),
+                     _address(top_k), _address(min_p), _address(keys), _address(out), _queue())
     return out
 
 
@@ -981,8 +993,8 @@ def top_logprobs(logits: torch.Tensor, n: int):
     n = max(1, min(int(n), vocab))
     ids = logits.new_empty((rows, n), dtype=torch.int32)
     values = logits.new_empty((rows, n), dtype=torch.float32)
-    _lib.core().call("mrun_top_logprobs", _ptr(logits), rows, vocab, n, _ptr(ids),
-                     _ptr(values), _stream())
+    _lib.core().call("mrun_top_logprobs", _address(logits), rows, vocab, n, _address(ids),
+                     _address(values), _queue())
     return ids, values
 
 
@@ -994,8 +1006,8 @@ def apply_token_mask(logits: torch.Tensor, rows: torch.Tensor, words: torch.Tens
     masks = rows.numel()
     if words.dim() != 2 or words.shape[0] != masks or mask_vocab.numel() != masks:
         raise KernelError(f"apply_token_mask: {masks} rows, words {tuple(words.shape)}, {mask_vocab.numel()} vocabularies")
-    _lib.core().call("mrun_apply_token_mask", _ptr(logits), logits.shape[1], _ptr(rows), _ptr(words),
-                     words.shape[1], _ptr(mask_vocab), masks, _stream())
+    _lib.core().call("mrun_apply_token_mask", _address(logits), logits.shape[1], _address(rows), _address(words),
+                     words.shape[1], _address(mask_vocab), masks, _queue())
 
 
 def repetition_penalty(logits: torch.Tensor, recent: torch.Tensor, penalty: torch.Tensor) -> None:
@@ -1005,8 +1017,8 @@ def repetition_penalty(logits: torch.Tensor, recent: torch.Tensor, penalty: torc
     rows, vocab = logits.shape
     if recent.dim() != 2 or recent.shape[0] != rows or penalty.numel() < rows:
         raise KernelError(f"repetition_penalty: recent {tuple(recent.shape)}, penalty {penalty.numel()}, rows {rows}")
-    _lib.core().call("mrun_repetition_penalty", _ptr(logits), rows, vocab, _ptr(recent),
-                     recent.shape[1], _ptr(penalty), _stream())
+    _lib.core().call("mrun_repetition_penalty", _address(logits), rows, vocab, _address(recent),
+                     recent.shape[1], _address(penalty), _queue())
 
 
 def scatter_i32(dst: torch.Tensor, index: torch.Tensor, value: torch.Tensor) -> None:
@@ -1014,8 +1026,8 @@ def scatter_i32(dst: torch.Tensor, index: torch.Tensor, value: torch.Tensor) -> 
     _check(dst, "dst", torch.int32); _check(index, "index", torch.int32); _check(value, "value", torch.int32)
     if index.numel() != value.numel():
         raise KernelError("scatter_i32: index and value differ in length")
-    _lib.core().call("mrun_scatter_i32", _ptr(dst), _ptr(index), _ptr(value), index.numel(),
-                     dst.numel(), _stream())
+    _lib.core().call("mrun_scatter_i32", _address(dst), _address(index), _address(value), index.numel(),
+                     dst.numel(), _queue())
 
 
 def select_tokens(ids: torch.Tensor, previous: torch.Tensor, source: torch.Tensor) -> None:
@@ -1023,8 +1035,8 @@ def select_tokens(ids: torch.Tensor, previous: torch.Tensor, source: torch.Tenso
     _check(ids, "ids", torch.int32); _check(previous, "previous", torch.int32); _check(source, "source", torch.int32)
     if source.numel() != ids.numel():
         raise KernelError("select_tokens: one source per row is needed")
-    _lib.core().call("mrun_select_tokens", _ptr(ids), _ptr(previous), _ptr(source), ids.numel(),
-                     previous.numel(), _stream())
+    _lib.core().call("mrun_select_tokens", _address(ids), _address(previous), _address(source), ids.numel(),
+                     previous.numel(), _queue())
 
 
 
@@ -1039,10 +1051,10 @@ def gemm_f32_nt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> 
     n = w.shape[1]
     if w.shape != (batch, n, k) or out.shape != (batch, m, n) or x.stride(2) != 1 or out.stride(2) != 1:
         raise KernelError(f"gemm_f32_nt_batched: x {tuple(x.shape)} w {tuple(w.shape)} out {tuple(out.shape)}")
-    _lib.core().call("mrun_gemm_f32_nt_batched", _ptr(x), _ptr(w), _ptr(out), batch, m, n,
+    _lib.core().call("mrun_gemm_f32_nt_batched", _address(x), _address(w), _address(out), batch, m, n,
                      k, x.stride(1) if m > 1 else max(k, x.stride(1)),
                      out.stride(1) if m > 1 else max(n, out.stride(1)),
-                     x.stride(0), n * k, out.stride(0), _stream())
+                     x.stride(0), n * k, out.stride(0), _queue())
     return out
 
 
@@ -1090,10 +1102,10 @@ def latent_prepare(down: torch.Tensor, q_weight: Optional[torch.Tensor], kv_weig
         _check(rot, "rot", torch.float32)
         if rot.shape != (tokens, rot_dims // 2, 2):
             raise KernelError(f"latent_prepare: rot is {tuple(rot.shape)}, expected {(tokens, rot_dims // 2, 2)}")
-    _lib.core().call("mrun_latent_prepare", _ptr(down), dtype_code(down.dtype), down.stride(0),
-                     _ptr(q_weight), _ptr(kv_weight), eps, _ptr(rot), rot_dims,
-                     PAIRINGS[pairing], _ptr(slots), _ptr(cq), _ptr(cache if slots is not None else None),
-                     tokens, q_rank, kv_rank, rot_dim, width, _stream())
+    _lib.core().call("mrun_latent_prepare", _address(down), dtype_code(down.dtype), down.stride(0),
+                     _address(q_weight), _address(kv_weight), eps, _address(rot), rot_dims,
+                     PAIRINGS[pairing], _address(slots), _address(cq), _address(cache if slots is not None else None),
+                     tokens, q_rank, kv_rank, rot_dim, width, _queue())
 
 
 def latent_rows(cache: torch.Tensor, block_tables: torch.Tensor, seg_slot: torch.Tensor, seg_kv_len: torch.Tensor, rows: int,
@@ -1115,10 +1127,10 @@ def latent_rows(cache: torch.Tensor, block_tables: torch.Tensor, seg_slot: torch
             raise KernelError(f"latent_rows: keys {tuple(keys.shape)} for {segments} segments of {rows} rows")
         heads, dim = keys.shape[1], keys.shape[3] - rot_dim
     out = cache.new_empty((segments, rows, kv_rank))
-    _lib.core().call("mrun_latent_rows", _ptr(cache), dtype_code(cache.dtype), _ptr(block_tables), block_tables.shape[1],
-                     _ptr(seg_slot), _ptr(seg_kv_len), _ptr(out), segments, rows, cache.shape[2],
-                     kv_rank, cache.shape[3], _ptr(keys if rot_dim else None), heads, dim,
-                     rot_dim, _stream())
+    _lib.core().call("mrun_latent_rows", _address(cache), dtype_code(cache.dtype), _address(block_tables), block_tables.shape[1],
+                     _address(seg_slot), _address(seg_kv_len), _address(out), segments, rows, cache.shape[2],
+                     kv_rank, cache.shape[3], _address(keys if rot_dim else None), heads, dim,
+                     rot_dim, _queue())
     return out
 
 
@@ -1129,8 +1141,8 @@ def latent_rotate(q: torch.Tensor, rot: torch.Tensor, rot_dims: int, pairing: st
     tokens = q.shape[0]
     if q.shape[1] != heads * (dim + rot_dim) or rot.shape != (tokens, rot_dims // 2, 2):
         raise KernelError(f"latent_rotate: q {tuple(q.shape)}, rot {tuple(rot.shape)}")
-    _lib.core().call("mrun_latent_rotate", _ptr(q), ldq, dtype_code(q.dtype), _ptr(rot), rot_dims,
-                     PAIRINGS[pairing], tokens, heads, dim, rot_dim, _stream())
+    _lib.core().call("mrun_latent_rotate", _address(q), ldq, dtype_code(q.dtype), _address(rot), rot_dims,
+                     PAIRINGS[pairing], tokens, heads, dim, rot_dim, _queue())
 
 
 def latent_query(q: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: int, pairing: str, q_att: torch.Tensor,
@@ -1146,9 +1158,9 @@ def latent_query(q: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: int, pa
         _check(rot, "rot", torch.float32)
         if rot.shape != (tokens, rot_dims // 2, 2):
             raise KernelError(f"latent_query: rot is {tuple(rot.shape)}, expected {(tokens, rot_dims // 2, 2)}")
-    _lib.core().call("mrun_latent_query", _ptr(q), ldq, dtype_code(q.dtype), _ptr(rot), rot_dims,
-                     PAIRINGS[pairing], _ptr(q_att), tokens, heads, dim,
-                     rot_dim, kv_rank, q_att.shape[2], _stream())
+    _lib.core().call("mrun_latent_query", _address(q), ldq, dtype_code(q.dtype), _address(rot), rot_dims,
+                     PAIRINGS[pairing], _address(q_att), tokens, heads, dim,
+                     rot_dim, kv_rank, q_att.shape[2], _queue())
 
 
 def post_norm_add(stream: torch.Tensor, branch: torch.Tensor, w_post: torch.Tensor, scale: float, eps_post: float,
@@ -1171,9 +1183,9 @@ def post_norm_add(stream: torch.Tensor, branch: torch.Tensor, w_post: torch.Tens
         code = dtype_code(out.dtype)
     if rows is not None:
         _check(rows, "rows", torch.int32)
-    _lib.core().call("mrun_post_norm_add", _ptr(stream), _ptr(branch), _ptr(w_post), scale,
-                     eps_post, _ptr(w_next), eps_next, _ptr(out if w_next is not None else None),
-                     code, _ptr(rows), n_rows, hidden, _stream())
+    _lib.core().call("mrun_post_norm_add", _address(stream), _address(branch), _address(w_post), scale,
+                     eps_post, _address(w_next), eps_next, _address(out if w_next is not None else None),
+                     code, _address(rows), n_rows, hidden, _queue())
     return out
 
 
@@ -1200,9 +1212,9 @@ def route_top_k(logits: torch.Tensor, top: int, score: str = "softmax", renormal
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"route_top_k: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_route_top_k", _ptr(logits), logits.stride(0), _ptr(bias), _ptr(weights), _ptr(chosen),
+    _lib.core().call("mrun_route_top_k", _address(logits), logits.stride(0), _address(bias), _address(weights), _address(chosen),
                      tokens, experts, top, ROUTER_SCORES[score],
-                     1 if renormalize else 0, _stream())
+                     1 if renormalize else 0, _queue())
     return weights
 
 
@@ -1218,22 +1230,22 @@ def relu2_scaled(u: torch.Tensor, weights: Optional[torch.Tensor], experts: int,
     else:
         experts, ff = 0, columns
     act = torch.empty_like(u)
-    _lib.core().call("mrun_relu2_scaled", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(weights), tokens,
-                     columns, experts, max(1, ff), _stream())
+    _lib.core().call("mrun_relu2_scaled", _address(u), _address(act), dtype_code(u.dtype), _address(weights), tokens,
+                     columns, experts, max(1, ff), _queue())
     return act
 
 
 def soft_cap(x: torch.Tensor, cap: float) -> torch.Tensor:
     """x = cap * tanh(x / cap) in place on float32."""
     _check(x, "x", torch.float32)
-    _lib.core().call("mrun_soft_cap", _ptr(x), x.numel(), cap, _stream())
+    _lib.core().call("mrun_soft_cap", _address(x), x.numel(), cap, _queue())
     return x
 
 
 def scale(x: torch.Tensor, factor: float) -> torch.Tensor:
     """x *= factor in place on float32."""
     _check(x, "x", torch.float32)
-    _lib.core().call("mrun_scale_f32", _ptr(x), x.numel(), factor, _stream())
+    _lib.core().call("mrun_scale_f32", _address(x), x.numel(), factor, _queue())
     return x
 
 
@@ -1256,8 +1268,8 @@ def moe_sort(chosen: torch.Tensor, weights: torch.Tensor):
     books = zeros[:3 * experts].view(3, experts)                              # counts, ends, cursor
     source, row_weight = zeros[3 * experts:3 * experts + pairs], zeros[3 * experts + pairs:].view(torch.float32)
     dest = torch.empty((tokens, top), dtype=torch.int32, device=dev)
-    _lib.core().call("mrun_moe_sort", _ptr(chosen), _ptr(weights), tokens, experts, top,
-                     _ptr(books[0]), _ptr(books[1]), _ptr(books[2]), _ptr(source), _ptr(row_weight), _ptr(dest), _stream())
+    _lib.core().call("mrun_moe_sort", _address(chosen), _address(weights), tokens, experts, top,
+                     _address(books[0]), _address(books[1]), _address(books[2]), _address(source), _address(row_weight), _address(dest), _queue())
     return books[1], source, row_weight, dest
 
 
@@ -1265,8 +1277,8 @@ def gather_rows(x: torch.Tensor, source: torch.Tensor) -> torch.Tensor:
     """out[r] = x[source[r]]."""
     _check(x, "x"); _check(source, "source", torch.int32)
     out = x.new_empty((source.numel(), x.shape[1]))
-    _lib.core().call("mrun_gather_rows", _ptr(x), dtype_code(x.dtype), _ptr(source), _ptr(out), source.numel(),
-                     x.shape[1], _stream())
+    _lib.core().call("mrun_gather_rows", _address(x), dtype_code(x.dtype), _address(source), _address(out), source.numel(),
+                     x.shape[1], _queue())
     return out
 
 
@@ -1276,8 +1288,8 @@ def relu2_rows(u: torch.Tensor, row_weight: torch.Tensor) -> torch.Tensor:
     if row_weight.numel() != u.shape[0]:
         raise KernelError("relu2_rows: one weight per row is needed")
     act = torch.empty_like(u)
-    _lib.core().call("mrun_relu2_rows", _ptr(u), _ptr(act), dtype_code(u.dtype), _ptr(row_weight), u.shape[0],
-                     u.shape[1], _stream())
+    _lib.core().call("mrun_relu2_rows", _address(u), _address(act), dtype_code(u.dtype), _address(row_weight), u.shape[0],
+                     u.shape[1], _queue())
     return act
 
 
@@ -1298,9 +1310,9 @@ def combine_rows(base: Optional[torch.Tensor], rows: torch.Tensor, dest: torch.T
         if extra.shape != (tokens, width) or share.numel() != tokens:
             raise KernelError(f"combine_rows: extra {tuple(extra.shape)}, share {tuple(share.shape)}")
     out = rows.new_empty((tokens, width), dtype=torch.float32)
-    _lib.core().call("mrun_combine_rows", _ptr(base), 1 if base is not None and base.dtype == torch.float32 else 0,
-                     _ptr(rows), dtype_code(rows.dtype), _ptr(dest), _ptr(out), tokens, top,
-                     width, _ptr(extra), _ptr(share), _stream())
+    _lib.core().call("mrun_combine_rows", _address(base), 1 if base is not None and base.dtype == torch.float32 else 0,
+                     _address(rows), dtype_code(rows.dtype), _address(dest), _address(out), tokens, top,
+                     width, _address(extra), _address(share), _queue())
     return out
 
 
@@ -1322,8 +1334,8 @@ def embed_streams(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, cop
     tokens = ids.numel()
     if out.shape != (tokens, copies * hidden):
         raise KernelError(f"embed_streams: out is {tuple(out.shape)}, expected {(tokens, copies * hidden)}")
-    _lib.core().call("mrun_embed_streams", _ptr(table), dtype_code(table.dtype), _ptr(ids), _ptr(out), tokens,
-                     hidden, vocab, copies, _stream())
+    _lib.core().call("mrun_embed_streams", _address(table), dtype_code(table.dtype), _address(ids), _address(out), tokens,
+                     hidden, vocab, copies, _queue())
     return out
 
 
@@ -1346,9 +1358,9 @@ def embed_bigram(table: torch.Tensor, pairs: Optional[torch.Tensor], ids: torch.
         if pairs.shape != (buckets + 1, hidden):
             raise KernelError(f"embed_bigram: pairs is {tuple(pairs.shape)}, expected {(buckets + 1, hidden)}")
         rows = ids.new_empty(tokens, dtype=torch.int32)
-    _lib.core().call("mrun_embed_bigram", _ptr(table), _ptr(pairs), dtype_code(table.dtype), _ptr(ids), _ptr(positions),
-                     _ptr(token_slot), _ptr(state), _ptr(rows), _ptr(out), tokens, hidden, vocab,
-                     copies, scale, buckets, mul_prev, mul_cur, _stream())
+    _lib.core().call("mrun_embed_bigram", _address(table), _address(pairs), dtype_code(table.dtype), _address(ids), _address(positions),
+                     _address(token_slot), _address(state), _address(rows), _address(out), tokens, hidden, vocab,
+                     copies, scale, buckets, mul_prev, mul_cur, _queue())
     return out
 
 
@@ -1398,10 +1410,10 @@ def streams_step(streams: torch.Tensor, pending: Optional[PendingStreams], in_c:
         if norm_weight.numel() != width:
             raise KernelError(f"streams_step: the norm weight has {norm_weight.numel()} entries, the width is {width}")
         h = streams.new_empty((n_rows, width), dtype=out_dtype)
-    _lib.core().call("mrun_streams_step", _ptr(streams), _ptr(y), _ptr(mix), _ptr(out_c), _ptr(in_c),
-                     _ptr(None if want_sum else norm_weight), eps, _ptr(h),
-                     dtype_code(out_dtype if h is not None else torch.float32), _ptr(u), _ptr(rows),
-                     n_rows, count, width, _stream())
+    _lib.core().call("mrun_streams_step", _address(streams), _address(y), _address(mix), _address(out_c), _address(in_c),
+                     _address(None if want_sum else norm_weight), eps, _address(h),
+                     dtype_code(out_dtype if h is not None else torch.float32), _address(u), _address(rows),
+                     n_rows, count, width, _queue())
     return u if want_sum else h
 
 
@@ -1424,10 +1436,10 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, ctx,
         if bias.numel() != channels:
             raise KernelError(f"causal_conv: bias has {bias.numel()} entries for {channels} channels")
     out = x.new_empty((tokens, channels))
-    _lib.core().call("mrun_causal_conv", _ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(state), _ptr(out),
-                     channels, dtype_code(x.dtype), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
+    _lib.core().call("mrun_causal_conv", _address(x), x.stride(0), _address(weight), _address(bias), _address(state), _address(out),
+                     channels, dtype_code(x.dtype), _address(ctx.seg_q_start), _address(ctx.seg_slot),
                      ctx.num_segments, ctx.max_q_len, channels, taps,
-                     1 if residual else 0, 1 if silu else 0, _stream())
+                     1 if residual else 0, 1 if silu else 0, _queue())
     return out
 
 
@@ -1515,8 +1527,8 @@ def _chunk_scratch(ctx, delta: bool, q, k, v, ld: int, a, bias, state, out, head
         return None
     size = _lib.core().function("mrun_chunked_scan_floats")
     size.restype = _c_long
-    floats = size(1 if delta else 0, _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(a), _ptr(bias),
-                  _ptr(state), _ptr(out), chunks, heads, dim, vdim)
+    floats = size(1 if delta else 0, _address(q), _address(k), _address(v), ld, dtype_code(q.dtype), _address(a), _address(bias),
+                  _address(state), _address(out), chunks, heads, dim, vdim)
     return (q.new_empty(floats, dtype=torch.float32), chunks) if floats else None
 
 
@@ -1526,9 +1538,9 @@ def _chunked_scan(q, k, v, ld: int, decay, silu_inputs: bool, a, bias, tau: floa
     found = _chunk_scratch(ctx, False, q, k, v, ld, a, bias, state, out, heads, dim, vdim)
     if found is None:
         return False
-    _lib.core().call("mrun_chunked_scan", _ptr(q), _ptr(k), _ptr(v), ld, _ptr(decay), 1 if silu_inputs else 0,
-                     _ptr(a), _ptr(bias), tau, _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
-                     _ptr(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _stream())
+    _lib.core().call("mrun_chunked_scan", _address(q), _address(k), _address(v), ld, _address(decay), 1 if silu_inputs else 0,
+                     _address(a), _address(bias), tau, _address(state), _address(out), _address(found[0]), _address(ctx.seg_q_start),
+                     _address(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _queue())
     return True
 
 
@@ -1538,9 +1550,9 @@ def _chunked_delta_scan(q, k, v, ld: int, a, b, ldb: int, a_log, dt_bias, state,
     found = _chunk_scratch(ctx, True, q, k, v, ld, a, dt_bias, state, out, heads, dim, vdim)
     if found is None:
         return False
-    _lib.core().call("mrun_chunked_delta_scan", _ptr(q), _ptr(k), _ptr(v), ld, heads // kv_heads, _ptr(a), _ptr(b),
-                     ldb, _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(out), _ptr(found[0]), _ptr(ctx.seg_q_start),
-                     _ptr(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _stream())
+    _lib.core().call("mrun_chunked_delta_scan", _address(q), _address(k), _address(v), ld, heads // kv_heads, _address(a), _address(b),
+                     ldb, _address(a_log), _address(dt_bias), _address(state), _address(out), _address(found[0]), _address(ctx.seg_q_start),
+                     _address(ctx.seg_slot), ctx.num_segments, found[1], heads, dim, vdim, _queue())
     return True
 
 
@@ -1561,10 +1573,10 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if _chunked_scan(q, k, v, ld, decay, silu_inputs, None, None, 1.0, state, ctx, out, heads, dim, vdim):
         return out
     scratch = q.new_empty(tokens * (2 * heads * dim + heads * vdim), dtype=torch.float32)
-    _lib.core().call("mrun_decay_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(decay),
-                     _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
+    _lib.core().call("mrun_decay_scan", _address(q), _address(k), _address(v), ld, dtype_code(q.dtype), _address(decay),
+                     _address(state), _address(out), _address(scratch), _address(ctx.seg_q_start), _address(ctx.seg_slot),
                      ctx.num_segments, tokens, heads, dim, vdim,
-                     1 if silu_inputs else 0, _stream())
+                     1 if silu_inputs else 0, _queue())
     return out
 
 
@@ -1590,10 +1602,10 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
     if _chunked_delta_scan(q, k, v, ld, a, b, ldb, a_log, dt_bias, state, ctx, out, heads, kv_heads, dim, vdim):
         return out
     scratch = q.new_empty(tokens * (2 * kv_heads * dim + heads * (vdim + dim + 1)), dtype=torch.float32)
-    _lib.core().call("mrun_delta_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype),
-                     heads // kv_heads, _ptr(a), _ptr(b), ldb, _ptr(a_log), _ptr(dt_bias), _ptr(state),
-                     _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments,
-                     tokens, heads, dim, vdim, _stream())
+    _lib.core().call("mrun_delta_scan", _address(q), _address(k), _address(v), ld, dtype_code(q.dtype),
+                     heads // kv_heads, _address(a), _address(b), ldb, _address(a_log), _address(dt_bias), _address(state),
+                     _address(out), _address(scratch), _address(ctx.seg_q_start), _address(ctx.seg_slot), ctx.num_segments,
+                     tokens, heads, dim, vdim, _queue())
     return out
 
 
@@ -1616,9 +1628,9 @@ def gated_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
     if _chunked_scan(q, k, v, ld, None, False, a, bias, tau, state, ctx, out, heads, dim, vdim):
         return out
     scratch = q.new_empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32)
-    _lib.core().call("mrun_gated_scan", _ptr(q), _ptr(k), _ptr(v), ld, dtype_code(q.dtype), _ptr(a), _ptr(bias),
-                     tau, _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     ctx.num_segments, tokens, heads, dim, vdim, _stream())
+    _lib.core().call("mrun_gated_scan", _address(q), _address(k), _address(v), ld, dtype_code(q.dtype), _address(a), _address(bias),
+                     tau, _address(state), _address(out), _address(scratch), _address(ctx.seg_q_start), _address(ctx.seg_slot),
+                     ctx.num_segments, tokens, heads, dim, vdim, _queue())
     return out
 
 
@@ -1643,9 +1655,9 @@ def gated_norm(o: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, eps: f
     ldo = _strided_rows(out, "out")
     if out.shape != o.shape or out.dtype != out_dtype:
         raise KernelError(f"gated_norm: out is {tuple(out.shape)} {out.dtype}")
-    _lib.core().call("mrun_gated_norm", _ptr(o), _ptr(weight), weight.numel(), _ptr(gate), ldg,
-                     dtype_code(out_dtype), eps, _ptr(out), ldo, scale, tokens, groups, n,
-                     GATE_SHAPES[gate_function], _stream())
+    _lib.core().call("mrun_gated_norm", _address(o), _address(weight), weight.numel(), _address(gate), ldg,
+                     dtype_code(out_dtype), eps, _address(out), ldo, scale, tokens, groups, n,
+                     GATE_SHAPES[gate_function], _queue())
     return out
 
 
@@ -1662,9 +1674,9 @@ def skip_gate_norm(o: torch.Tensor, x: torch.Tensor, skip: torch.Tensor, z: torc
             or features % skip.numel():
         raise KernelError(f"skip_gate_norm: o {tuple(o.shape)}, x {tuple(x.shape)}, z {tuple(z.shape)}, {groups} groups")
     out = o.new_empty((tokens, features), dtype=x.dtype)
-    _lib.core().call("mrun_skip_gate_norm", _ptr(o), _ptr(x), ldx, _ptr(skip), features // skip.numel(),
-                     _ptr(z), ldz, _ptr(weight), dtype_code(x.dtype), eps, _ptr(out),
-                     tokens, groups, features // groups, _stream())
+    _lib.core().call("mrun_skip_gate_norm", _address(o), _address(x), ldx, _address(skip), features // skip.numel(),
+                     _address(z), ldz, _address(weight), dtype_code(x.dtype), eps, _address(out),
+                     tokens, groups, features // groups, _queue())
     return out
 
 
@@ -1678,9 +1690,9 @@ def token_blend(x: torch.Tensor, mu: torch.Tensor, state: torch.Tensor, ctx) -> 
     if mu.dim() != 2 or mu.shape[1] != channels or state.shape[1:] != (1, channels):
         raise KernelError(f"token_blend: x {tuple(x.shape)}, mu {tuple(mu.shape)}, state {tuple(state.shape)}")
     out = x.new_empty((tokens, mu.shape[0], channels))
-    _lib.core().call("mrun_token_blend", _ptr(x), ldx, _ptr(mu), _ptr(state), _ptr(out), dtype_code(x.dtype),
-                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
-                     channels, mu.shape[0], _stream())
+    _lib.core().call("mrun_token_blend", _address(x), ldx, _address(mu), _address(state), _address(out), dtype_code(x.dtype),
+                     _address(ctx.seg_q_start), _address(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
+                     channels, mu.shape[0], _queue())
     return out
 
 
@@ -1704,12 +1716,12 @@ def bonus_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tenso
         raise KernelError("bonus_scan: sizes do not match")
     out = r.new_empty((tokens, heads * vdim), dtype=torch.float32)
     scratch = None
-    if not _lib.core().function("mrun_scan_walks")(0, _ptr(r), _ptr(k), _ptr(v), ld, dtype_code(r.dtype), _ptr(a),
-                                                   _ptr(bias), _ptr(bonus), _ptr(state), dim, vdim):
+    if not _lib.core().function("mrun_scan_walks")(0, _address(r), _address(k), _address(v), ld, dtype_code(r.dtype), _address(a),
+                                                   _address(bias), _address(bonus), _address(state), dim, vdim):
         scratch = r.new_empty(tokens * heads * (3 * dim + vdim), dtype=torch.float32)
-    _lib.core().call("mrun_bonus_scan", _ptr(r), _ptr(k), _ptr(v), ld, dtype_code(r.dtype), _ptr(a), _ptr(bias),
-                     _ptr(bonus), _ptr(state), _ptr(out), _ptr(scratch), _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot),
-                     ctx.num_segments, ctx.max_q_len, tokens, heads, dim, vdim, _stream())
+    _lib.core().call("mrun_bonus_scan", _address(r), _address(k), _address(v), ld, dtype_code(r.dtype), _address(a), _address(bias),
+                     _address(bonus), _address(state), _address(out), _address(scratch), _address(ctx.seg_q_start), _address(ctx.seg_slot),
+                     ctx.num_segments, ctx.max_q_len, tokens, heads, dim, vdim, _queue())
     return out
 
 
@@ -1732,13 +1744,13 @@ def ssm_scan(c: torch.Tensor, b: torch.Tensor, x: torch.Tensor, dt: torch.Tensor
         raise KernelError("ssm_scan: sizes do not match")
     out = c.new_empty((tokens, heads * vdim), dtype=torch.float32)
     scratch = None
-    if not _lib.core().function("mrun_scan_walks")(1, _ptr(c), _ptr(b), _ptr(x), ld, dtype_code(c.dtype), _ptr(None),
-                                                   _ptr(dt_bias), _ptr(None), _ptr(state), size, vdim):
+    if not _lib.core().function("mrun_scan_walks")(1, _address(c), _address(b), _address(x), ld, dtype_code(c.dtype), _address(None),
+                                                   _address(dt_bias), _address(None), _address(state), size, vdim):
         scratch = c.new_empty(tokens * (2 * groups * size + heads * (vdim + 1)), dtype=torch.float32)
-    _lib.core().call("mrun_ssm_scan", _ptr(c), _ptr(b), _ptr(x), ld, dtype_code(c.dtype), heads // groups,
-                     _ptr(dt), lddt, _ptr(dt_bias), _ptr(a_log), _ptr(state), _ptr(out), _ptr(scratch),
-                     _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len, tokens, heads,
-                     size, vdim, _stream())
+    _lib.core().call("mrun_ssm_scan", _address(c), _address(b), _address(x), ld, dtype_code(c.dtype), heads // groups,
+                     _address(dt), lddt, _address(dt_bias), _address(a_log), _address(state), _address(out), _address(scratch),
+                     _address(ctx.seg_q_start), _address(ctx.seg_slot), ctx.num_segments, ctx.max_q_len, tokens, heads,
+                     size, vdim, _queue())
     return out
 
 
@@ -1760,10 +1772,10 @@ def selective_scan(x: torch.Tensor, z: torch.Tensor, dt: torch.Tensor, dt_bias: 
             or b.dtype != (x.dtype if ctx.max_q_len == 1 else torch.float32):
         raise KernelError("selective_scan: sizes or types do not match")
     out = x.new_empty((tokens, inner))
-    _lib.core().call("mrun_selective_scan", _ptr(x), ldx, _ptr(z), ldz, _ptr(b), _ptr(c), ldb,
-                     dtype_code(x.dtype), _ptr(dt), lddt, _ptr(dt_bias), _ptr(a), _ptr(skip), _ptr(state), _ptr(out),
-                     inner, _ptr(ctx.seg_q_start), _ptr(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
-                     tokens, inner, states, _stream())
+    _lib.core().call("mrun_selective_scan", _address(x), ldx, _address(z), ldz, _address(b), _address(c), ldb,
+                     dtype_code(x.dtype), _address(dt), lddt, _address(dt_bias), _address(a), _address(skip), _address(state), _address(out),
+                     inner, _address(ctx.seg_q_start), _address(ctx.seg_slot), ctx.num_segments, ctx.max_q_len,
+                     tokens, inner, states, _queue())
     return out
 
 
@@ -1775,8 +1787,8 @@ def head_gate(y: torch.Tensor, gate: torch.Tensor, heads: int) -> torch.Tensor:
     tokens, features = y.shape
     if gate.shape != (tokens, heads) or gate.dtype != y.dtype or features % heads:
         raise KernelError("head_gate: sizes do not match")
-    _lib.core().call("mrun_head_gate", _ptr(y), _ptr(gate), ldg, dtype_code(y.dtype), tokens, heads,
-                     features // heads, _stream())
+    _lib.core().call("mrun_head_gate", _address(y), _address(gate), ldg, dtype_code(y.dtype), tokens, heads,
+                     features // heads, _queue())
     return y
 
 
@@ -1800,10 +1812,10 @@ def diff_rope_cache(qkv: torch.Tensor, rot: Optional[torch.Tensor], rot_dims: in
             raise KernelError(f"diff_rope_cache: rot is {tuple(rot.shape)}")
     if slots is not None:
         _check(slots, "slots", torch.int32)
-    _lib.core().call("mrun_diff_rope_cache", _ptr(qkv), qkv.stride(0), dtype_code(qkv.dtype), _ptr(rot),
-                     rot_dims if rot is not None else 0, _ptr(slots), _ptr(k_cache), _ptr(v_cache), pages,
+    _lib.core().call("mrun_diff_rope_cache", _address(qkv), qkv.stride(0), dtype_code(qkv.dtype), _address(rot),
+                     rot_dims if rot is not None else 0, _address(slots), _address(k_cache), _address(v_cache), pages,
                      tokens, heads, kv_heads, dim, vdim, vdim // chunks,
-                     page_size, _stream())
+                     page_size, _queue())
 
 
 def diff_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor,
@@ -1822,11 +1834,11 @@ def diff_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
             or v_cache.shape[0] * v_cache.shape[4] != vdim:
         raise KernelError("diff_attention: sizes do not match")
     out = q.new_empty((tokens, heads * vdim))
-    _lib.core().call("mrun_diff_attention", _ptr(q), ld, _ptr(out), _ptr(k_cache), _ptr(v_cache),
-                     dtype_code(q.dtype), _ptr(block_tables), block_tables.shape[1], _ptr(token_slot),
-                     _ptr(positions), pages, tokens, heads, kv_heads, dim,
+    _lib.core().call("mrun_diff_attention", _address(q), ld, _address(out), _address(k_cache), _address(v_cache),
+                     dtype_code(q.dtype), _address(block_tables), block_tables.shape[1], _address(token_slot),
+                     _address(positions), pages, tokens, heads, kv_heads, dim,
                      vdim, v_cache.shape[4], page_size, scale, lam,
-                     eps, out_scale, window, _stream())
+                     eps, out_scale, window, _queue())
     return out
 
 
@@ -1838,8 +1850,8 @@ def diff_combine(maps: torch.Tensor, heads: int, vdim: int, lam: float, eps: flo
     if two != 2 or row * chunks != heads * vdim:
         raise KernelError("diff_combine: sizes do not match")
     out = maps.new_empty((tokens, heads * vdim))
-    _lib.core().call("mrun_diff_combine", _ptr(maps), _ptr(out), dtype_code(maps.dtype), tokens, heads,
-                     vdim, vdim // chunks, lam, eps, out_scale, _stream())
+    _lib.core().call("mrun_diff_combine", _address(maps), _address(out), dtype_code(maps.dtype), tokens, heads,
+                     vdim, vdim // chunks, lam, eps, out_scale, _queue())
     return out
 
 
@@ -1856,8 +1868,8 @@ def table_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, chos
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"table_route: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_table_route", _ptr(token_ids), _ptr(table), _ptr(weights), _ptr(chosen), tokens,
-                     vocab, experts, top, _stream())
+    _lib.core().call("mrun_table_route", _address(token_ids), _address(table), _address(weights), _address(chosen), tokens,
+                     vocab, experts, top, _queue())
     return weights
 
 
@@ -1894,9 +1906,9 @@ def clamped_glu(u: torch.Tensor, weights: Optional[torch.Tensor], blocks: int, f
     lda = _strided_rows(out, "out")
     if out.shape != (rows, blocks * ff) or out.dtype != u.dtype:
         raise KernelError(f"clamped_glu: out is {tuple(out.shape)} {out.dtype}")
-    _lib.core().call("mrun_clamped_glu", _ptr(u), ldu, _ptr(out), lda, dtype_code(u.dtype), _ptr(weights),
+    _lib.core().call("mrun_clamped_glu", _address(u), ldu, _address(out), lda, dtype_code(u.dtype), _address(weights),
                      ldw, per_block, rows, blocks, ff, limit,
-                     alpha, up_offset, _ptr(bias), _stream())
+                     alpha, up_offset, _address(bias), _queue())
     return out
 
 
@@ -1932,10 +1944,10 @@ def route_grouped(logits: torch.Tensor, experts: int, top: int, groups: int, kee
         _check(chosen, "chosen", torch.int32)
         if chosen.shape != (tokens, top):
             raise KernelError(f"route_grouped: chosen is {tuple(chosen.shape)}, expected {(tokens, top)}")
-    _lib.core().call("mrun_route_grouped", _ptr(logits), logits.stride(0), ROUTER_SCORES[score], _ptr(correction),
-                     _ptr(weights), _ptr(unchanged), _ptr(shared), _ptr(chosen), tokens, experts,
+    _lib.core().call("mrun_route_grouped", _address(logits), logits.stride(0), ROUTER_SCORES[score], _address(correction),
+                     _address(weights), _address(unchanged), _address(shared), _address(chosen), tokens, experts,
                      identity, top, groups, keep, group_top,
                      1 if renormalize else 0, scale,
-                     *((_ptr(handed_on.sums), handed_on.shape[1], handed_on.eps) if handed_on is not None
-                       else (_ptr(None), 0, 0.0)), _stream())
+                     *((_address(handed_on.sums), handed_on.shape[1], handed_on.eps) if handed_on is not None
+                       else (_address(None), 0, 0.0)), _queue())
     return weights, shared, unchanged
