@@ -47,6 +47,17 @@ def prototypes() -> Dict[str, list]:
     return _prototypes
 
 
+def _undeclared(path: str, name: str, fn):
+    """A function that the sources do not define: ctypes would cut a plain number to a 32-bit int, so it takes ctypes objects only."""
+    def call(*args):
+        for position, value in enumerate(args):
+            if isinstance(value, (int, float)):
+                raise KernelError(f"{name} of {path} has no declared parameters: argument {position} must say its type "
+                                  f"(a ctypes object), not {value!r}")
+        return fn(*args)
+    return call
+
+
 class Library:
     """A loaded ``.so``: ``lib.call("mrun_x", args...)`` raises on a non-zero return."""
 
@@ -68,7 +79,11 @@ class Library:
             except AttributeError:
                 raise KernelError(f"{self.path} exports no {name}") from None
             fn.restype = ctypes.c_int
-            fn.argtypes = prototypes().get(name)
+            types = prototypes().get(name)
+            if types is None:
+                fn = _undeclared(self.path, name, fn)
+            else:
+                fn.argtypes = types
             self._functions[name] = fn
         return fn
 
