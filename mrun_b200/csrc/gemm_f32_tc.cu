@@ -479,17 +479,18 @@ MRUN_API int mrun_gemm_f32_tc(const float* x, const float* w, float* y, void* pa
                  "gemm_f32_tc: a cluster of %d for %d ranges", cluster, ranges);
     const int pitch = (K + 7) / 8 * 8;
     const bool aligned = ((uintptr_t)x & 15) == 0 && (ldx % 4 == 0 || M == 1);
-    // Up to 32 rows: w's bytes count, and two blocks on a multiprocessor read it in all the ranges at once.
-    if (tile == 0 && M <= 32) {
+    // Up to 32 rows: w's bytes count, and two blocks on a multiprocessor read it in all the ranges at once.  (A block of the
+    // small tiles has one range: only the larger ones take several one after the other.)
+    if (tile == 0 && M <= 32 && (cluster == 0 || cluster == ranges)) {
         tile = M <= 16 ? 16 : 32;
-        if (cluster == 0) cluster = ranges;
+        cluster = ranges;
     } else if (tile == 0 || cluster == 0) {
         const int asked_tile = tile, asked_cluster = cluster;
         float least = 0.f;
         for (int t : TILES) {
             if (asked_tile ? t != asked_tile : t <= 32) continue;
             for (int c : {ranges, 1}) {
-                if (asked_cluster && c != asked_cluster) continue;
+                if ((asked_cluster && c != asked_cluster) || (t <= 32 && c != ranges)) continue;
                 const float cost = cost_of(t, c, M, N, a);
                 if (least == 0.f || cost < least) { least = cost; tile = t; cluster = c; }
             }
