@@ -59,10 +59,11 @@ template <int TOK> struct Shape {
     static constexpr unsigned COLUMNS = COLUMNS_USED <= 128 ? 128 : COLUMNS_USED <= 256 ? 256 : 512;
     static constexpr int SUM_WARPS = TOK <= 32 ? 4 : 8, EACH = TOK * 4 / SUM_WARPS;      // EACH: tokens of a summing thread
     static constexpr int W_WARP = CONVERT_WARPS + SUM_WARPS, MMA_WARP = W_WARP + 1, X_WARP = W_WARP + 3;
-    // The summing warps of the widest tiles take registers from the others (setmaxnreg works on four warps together).
+    // The summing warps of the widest tiles take registers from the others (setmaxnreg works on four warps together, and waits
+    // for good where the block was launched with fewer than are dealt out: launch() looks).
     static constexpr bool UNEVEN = TOK >= 112;
-    static constexpr int THREADS = 32 * (X_WARP + 1);
-    static_assert(!UNEVEN || CONVERT_WARPS * 72 + SUM_WARPS * 144 + 4 * 40 <= THREADS / 32 * 96, "more registers than the block has");
+    static constexpr int THREADS = 32 * (X_WARP + 1), LAUNCH_REGISTERS = 96;
+    static_assert(!UNEVEN || CONVERT_WARPS * 72 + SUM_WARPS * 144 + 4 * 40 <= THREADS / 32 * LAUNCH_REGISTERS, "more registers than the block has");
     static_assert(COLUMNS_USED <= 512 && W_STAGES >= 4 && TOK % 16 == 0, "the tile does not fit");
     static_assert(X_STAGES * X_BYTES >= TOK * ROWS * 4, "the ranges' sums take the place of x");
 };
@@ -419,6 +420,11 @@ void configure(cudaLaunchConfig_t* config, cudaLaunchAttribute* attributes, dim3
     config->numAttrs = 2;
 }
 
+int registers_of(const void* kernel) {
+    cudaFuncAttributes has;
+    return cudaFuncGetAttributes(&has, kernel) == cudaSuccess ? has.numRegs : -1;
+}
+
 template <int TOK>
 int launch(const CUtensorMap& map_w, const void* parts, int pitch, const ProductArgs& a, int cluster, cudaStream_t stream) {
     CUtensorMap map_x;
@@ -430,6 +436,11 @@ int launch(const CUtensorMap& map_w, const void* parts, int pitch, const Product
     MRUN_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "gemm_f32_tc: M=%d N=%d exceed the grid", a.M, a.N);
     MRUN_CHECK_CUDA(cudaFuncSetAttribute(gemm_f32_tc_kernel<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<TOK>::SMEM),
                     "gemm_f32_tc");
+    if constexpr (Shape<TOK>::UNEVEN) {
+        static const int registers = registers_of((const void*)gemm_f32_tc_kernel<TOK>);
+        MRUN_REQUIRE(registers == Shape<TOK>::LAUNCH_REGISTERS, "gemm_f32_tc: tiles of %d tokens were built with %d registers a thread, %d are dealt out",
+                     TOK, registers, Shape<TOK>::LAUNCH_REGISTERS);
+    }
     cudaLaunchConfig_t config;
     cudaLaunchAttribute attributes[2];
     configure<TOK>(&config, attributes, grid, stream);
