@@ -1,12 +1,13 @@
 // 32-bit linear layer on the bfloat16 tensor cores (tcgen05): y[M, N] = x[M, K] · w[N, K]^T where every 32-bit
-// operand is taken as the exact sum of three bfloat16 values, a = a1 + a2 + a3 (8 significant bits each, rounded to
+// operand is taken as the exact sum of three bfloat16 values, 2^24 a = a1 + a2 + a3 (8 significant bits each, rounded to
 // nearest, so |a2| <= 2^-8 |a1| and |a3| <= 2^-16 |a1|), and the six products
 //     a1 b1,  a1 b2 + a2 b1,  a1 b3 + a2 b2 + a3 b1
-// are added up; what is left out is below 2^-24 of |a b|, and of either sign.  Products of two bfloat16 values are
-// exact in 32 bits.  The tensor core adds up 64 values of k at a time from zero; these sums are added by 32-bit
+// are added up; what is left out is below 2^-24 of |a b|, and of either sign.  Without the factor, which a sum loses again, the third
+// part of an operand below 2^-109 would have fallen under bfloat16's least value; with it the split is exact down to the least 32-bit
+// value.  Products of two bfloat16 values are exact in 32 bits.  The tensor core adds up 64 values of k at a time from zero; these sums are added by 32-bit
 // additions in order, and where a row of w is cut into `split` ranges of k (chosen from N and K alone), the ranges' sums in order of
 // range.  So a row of x has the same bits whatever M is and wherever it sits in the batch.  A result that is not
-// finite (an operand that is not, or a sum out of range) is computed again as a chain of fused multiply-adds.
+// finite (an operand that is not or is beyond 2^103, or a sum beyond 2^79) is computed again as a chain of fused multiply-adds.
 //
 //   split   (a kernel in front) writes the three parts of x, [3][M][K], so that TMA brings them
 //   product a block a tile of 128 rows of w (the MMA's M) x TOK tokens (its N) and a range of k; a cluster's
@@ -40,6 +41,7 @@ constexpr int CONVERT_WARPS = 8;          // two groups, each every second box o
 constexpr int MAX_SPLIT = 8;              // the portable cluster size
 constexpr int W_BYTES = ROWS * HALF * 4;
 constexpr int A_COLUMNS = PARTS * HALF / 2;
+constexpr float SCALE = 16777216.f, UNSCALE = 1.f / SCALE / SCALE;      // 2^24 of either operand, 2^-48 of a sum
 constexpr long long WAIT_CYCLES = 3000000000LL;   // about 1.5 s at 2 GHz
 
 enum : int { STATUS_W = 1, STATUS_X = 2, STATUS_CONVERT = 3, STATUS_MMA = 4, STATUS_SUM = 5 };
@@ -87,8 +89,11 @@ __device__ __forceinline__ void tmem_load8(unsigned address, float (&v)[8]) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// The three parts of two values, packed as the tensor core wants them (the first in the low half).
+// The three parts of 2^24 times two values, packed as the tensor core wants them (the first in the low half).
 __device__ __forceinline__ void three_parts(float x, float y, unsigned (&part)[PARTS]) {
+    const float2 scaled = __fmul2_rn(make_float2(x, y), make_float2(SCALE, SCALE));
+    x = scaled.x;
+    y = scaled.y;
 #pragma unroll
     for (int p = 0; p < PARTS; ++p) {
         const __nv_bfloat162 both = __floats2bfloat162_rn(x, y);
@@ -331,7 +336,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     }
 #pragma unroll
                     for (int i = 0; i < RUN; ++i) {
-                        const float v = S::FOLDS && range > 0 ? before[i] + acc[c + i] : acc[c + i];
+                        const float sum = acc[c + i] * UNSCALE, v = S::FOLDS && range > 0 ? before[i] + sum : sum;
                         if (first + c + i < a.M && row < a.N) {
                             *dst = v;
                             if (j + 1 == n) out_of_range |= !finite(v);
@@ -351,7 +356,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             float* sums = reinterpret_cast<float*>(x_ring);
             if (!*(volatile int*)&aborted)
 #pragma unroll
-                for (int i = 0; i < S::EACH; ++i) sums[(part * S::EACH + i) * ROWS + in] = acc[i];
+                for (int i = 0; i < S::EACH; ++i) sums[(part * S::EACH + i) * ROWS + in] = acc[i] * UNSCALE;
         }
     }
 

@@ -28,3 +28,18 @@ def test_small_tiles_take_one_range_a_block(tile):
     from mrun_b200.kernels import ops
     with pytest.raises(ops.KernelError, match="cluster of 1 for 2 ranges"):
         ops.gemm_f32_tc(rows(5, 4096, 1), rows(256, 4096, 2), ranges=2, tile=tile, cluster=1)
+
+
+@pytest.mark.parametrize("m", [3, 150])
+@pytest.mark.parametrize("low,high", [(-112, 100), (-120, 100), (-126, 100), (-135, 100), (100, -120), (100, -135), (-70, -50)])
+def test_tiny_operands_keep_their_digits(m, low, high):
+    """Operands down to values with few significant bits of their own, beside large ones, so that the results are ordinary numbers;
+    and results near the least normal value, where a rounding is up to 2^-150 of each of the ranges' sums."""
+    from mrun_b200.kernels import ops
+    k = 2048
+    x, w = rows(m, k, 3) * 2.0 ** low, rows(200, k, 4) * 2.0 ** high
+    if m > 100:
+        x[:, ::7] *= 2.0 ** 20 if low < 0 else 2.0 ** -20             # beside each other in a row
+    got, want = ops.gemm_f32_nt(x, w).double(), x.double() @ w.double().T
+    ops.tc5_check()
+    assert (got - want).norm() <= 6e-7 * want.norm() + (m * 200) ** 0.5 * 9 * 2.0 ** -150
