@@ -382,7 +382,7 @@ def _sizing(memory: MemoryBudget, context: Optional[int], page_size: int, max_re
         element = 2 if precision.act == torch.bfloat16 else 4
         per_token, per_slot = token_bytes(model.cache_needs(), model.cache_shares(), element)
         scratch = budget.scratch_estimate(spec.hidden_size, model.activation_elements(), spec.vocab_size,
-                                          max_batch_tokens, max_requests, element)
+                                          max_batch_tokens, max_requests, element) + model.product_scratch(max_batch_tokens)
         weights = model.weight_bytes()
         most = spec.max_positions * max_requests
         if context is not None:

@@ -82,30 +82,33 @@ class Model:
         return (all(getattr(block.mixer, "graph_safe", False) for block in self.blocks)
                 and (self.embedder is None or getattr(self.embedder, "graph_safe", False)))
 
-    def weight_bytes(self) -> int:
-        seen, total = set(), 0
+    def _tensors(self):
+        """Every tensor that a part holds, views of one another included."""
         def walk(obj):
-            nonlocal total
             if isinstance(obj, torch.Tensor):
-                storage = obj.untyped_storage()         # views of one tensor share it and count once
-                if storage.data_ptr() not in seen:
-                    seen.add(storage.data_ptr())
-                    total += storage.nbytes()
+                yield obj
             elif hasattr(obj, "__dict__"):
                 for value in vars(obj).values():
                     if isinstance(value, (torch.Tensor,)) or hasattr(value, "__dict__"):
-                        walk(value)
+                        yield from walk(value)
                     elif isinstance(value, (list, tuple)):
                         for item in value:
-                            walk(item)
-        walk(self.final_norm)
+                            yield from walk(item)
+        yield from walk(self.final_norm)
         for block in self.blocks:
-            walk(block)
+            yield from walk(block)
         for t in (self.embedding, self.head):
-            walk(t)
+            yield from walk(t)
         if self.embedder is not None:
-            walk(self.embedder)
-        return total
+            yield from walk(self.embedder)
+
+    def weight_bytes(self) -> int:
+        storages = (t.untyped_storage() for t in self._tensors())      # views of one tensor share it and count once
+        return sum({storage.data_ptr(): storage.nbytes() for storage in storages}.values())
+
+    def product_scratch(self, tokens: int) -> int:
+        """Bytes that the largest product of a step of ``tokens`` takes beside its operands and its result."""
+        return max((ops.product_scratch(t, tokens) for t in self._tensors()), default=0)
 
     # ------------------------------------------------------------------ forward
     def hidden_states(self, ctx: StepContext, caches) -> tuple:

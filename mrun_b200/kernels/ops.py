@@ -718,6 +718,19 @@ def f32_tc_ok(w: torch.Tensor) -> bool:
     return k >= F32_TC_MIN_K and n >= F32_TC_MIN_N and k % 4 == 0 and w.data_ptr() % 16 == 0
 
 
+def _f32_tc_rows(m: int, k: int) -> int:
+    """Rows that a portion of such a product splits at once."""
+    return max(1, min(m, F32_TC_SCRATCH // (6 * (-(-k // 8) * 8))))
+
+
+def product_scratch(w: torch.Tensor, rows: int) -> int:
+    """Bytes that the product of up to ``rows`` rows with ``w`` takes beside its operands and its result."""
+    if w.dtype != torch.float32 or w.dim() != 2 or not f32_tc_ok(w):
+        return 0
+    k = w.shape[1]
+    return 6 * (-(-k // 8) * 8) * _f32_tc_rows(rows, k)
+
+
 def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, ranges: int = 0, tile: int = 0,
                 cluster: int = 0) -> torch.Tensor:
     """:func:`gemm_f32_nt` on the tensor cores, every operand as the sum of three bfloat16 values (``csrc/gemm_f32_tc.cu``).
@@ -733,7 +746,7 @@ def gemm_f32_tc(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
     if out.shape != (m, n):
         raise KernelError(f"gemm_f32_tc: out is {tuple(out.shape)}, expected {(m, n)}")
     pitch = -(-k // 8) * 8
-    rows = max(1, min(m, F32_TC_SCRATCH // (6 * pitch)))
+    rows = _f32_tc_rows(m, k)
     parts = x.new_empty(3 * rows * pitch, dtype=torch.bfloat16)
     status = status_word(x.device, "gemm_f32_tc", {1: "the copies of w", 2: "the copies of x", 3: "the conversion of w",
                                                    4: "the MMA issuer", 5: "the sums"})
