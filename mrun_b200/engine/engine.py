@@ -16,6 +16,7 @@ import torch
 
 from ..cache.manager import token_bytes
 from ..cache.pages import OutOfPages
+from ..kernels.ops import STATUS_WORDS, status_block
 from ..sampling.mask import TokenMask
 from ..sampling.params import REPETITION_CONTEXT, SamplingParams, draw_key
 from ..sampling.sampler import Sampler
@@ -52,6 +53,7 @@ class _Flying:
     rows: dict                     # id(request) -> row of the step
     bucket: int
     pinned: torch.Tensor           # where its tokens land on the host
+    status: torch.Tensor           # and the status words of its kernels
     event: torch.cuda.Event
 
 
@@ -78,7 +80,7 @@ class Engine:
         self.stats = EngineStats()
         self._next_id = 0
         rows = max(1, 2 * executor.cache.max_requests)
-        self._token_buffers = [torch.empty(rows, dtype=torch.int32, pin_memory=True) for _ in range(2)]
+        self._token_buffers = [torch.zeros(rows + STATUS_WORDS, dtype=torch.int32, pin_memory=True) for _ in range(2)]
         self._token_turn = 0
 
     # ------------------------------------------------------------------ construction
@@ -241,19 +243,25 @@ class Engine:
         pinned = self._token_buffers[self._token_turn]
         self._token_turn ^= 1
         pinned[:len(entries)].copy_(tokens, non_blocking=True)
+        status = pinned[-STATUS_WORDS:]
+        words = status_block(self.executor.device)
+        if words is not None:
+            status.copy_(words, non_blocking=True)
         event = torch.cuda.Event()
         event.record()
         scheduler.launched(plan)
         self.stats.steps += 1
         self.stats.tokens_in += plan.num_tokens
         return _Flying(plan, {id(e.request): row for row, e in enumerate(plan.entries)},
-                       self.executor.decode_bucket(len(entries)), pinned, event)
+                       self.executor.decode_bucket(len(entries)), pinned, status, event)
 
     def _deliver(self, scheduler: Scheduler, flying: "_Flying") -> None:
         flying.event.synchronize()
+        if flying.status.count_nonzero():       # a kernel of the step gave up on a wait: its tokens are void
+            self.executor.check()
         host = flying.pinned[:len(flying.plan.entries)].tolist()
         self.stats.tokens_out += len(host)
-        self.stats.d2h_bytes += 4 * len(host)
+        self.stats.d2h_bytes += 4 * (len(host) + STATUS_WORDS)
         scheduler.complete(flying.plan, host)
 
     def _run_plan(self, scheduler: Scheduler, plan: StepPlan) -> None:
@@ -287,8 +295,7 @@ class Engine:
         host = tokens.to("cpu").tolist()
         for row in refused:
             host[row] = None
-        if plan.num_tokens > len(plan.entries):          # a step with prompt portions: its kernels wait on one another
-            self.executor.check()
+        self.executor.check()               # before a token is handed out
         self.stats.tokens_out += len(host)
         self.stats.d2h_bytes += 4 * len(host)
         scheduler.complete(plan, host)

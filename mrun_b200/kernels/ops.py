@@ -813,28 +813,46 @@ def gemm_tc5(x, w: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16, swiglu
     return out
 
 
-_status_words = {}       # (device, kernel name) -> (int32[1] on the device, {code: role})
+STATUS_WORDS = 32
+_status_blocks = {}      # device -> (int32[STATUS_WORDS] on the device, {kernel name: (its word, {code: role})})
+
+
+def _status(device: torch.device):
+    return _status_blocks.get(device if device.index is not None else torch.device(device.type, torch.cuda.current_device()))
 
 
 def status_word(device: torch.device, kernel: str, roles: dict) -> torch.Tensor:
     """The word a kernel with bounded waits reports into (zero = fine), one per device and kernel,
     never reallocated, so that captured graphs may keep its address.  :func:`tc5_check` reads it."""
-    entry = _status_words.get((device, kernel))
+    found = _status(device)
+    if found is None:
+        found = _status_blocks[device] = (torch.zeros(STATUS_WORDS, dtype=torch.int32, device=device), {})
+    block, words = found
+    entry = words.get(kernel)
     if entry is None:
-        entry = _status_words[(device, kernel)] = (torch.zeros(1, dtype=torch.int32, device=device), dict(roles))
+        if len(words) == STATUS_WORDS:
+            raise KernelError(f"no status word is left for {kernel}")
+        entry = words[kernel] = (block[len(words):len(words) + 1], dict(roles))
     return entry[0]
 
 
+def status_block(device: torch.device) -> Optional[torch.Tensor]:
+    """All status words of a device in one tensor, to bring them to the host with a step's result; None before the first one."""
+    found = _status(device)
+    return None if found is None else found[0]
+
+
 def tc5_check(device: Optional[torch.device] = None) -> None:
-    """Raises if a tcgen05 kernel on the device gave up on a wait (and clears its status word)."""
-    for (dev, kernel), (status, roles) in list(_status_words.items()):
-        if device is not None and dev != device:
+    """Raises if a kernel with bounded waits on the device gave up on one (and clears its status word)."""
+    for dev, (block, words) in list(_status_blocks.items()):
+        if device is not None and _status(device) is not _status_blocks[dev]:
             continue
-        code = int(status.item())
-        if code:
-            status.zero_()
-            raise KernelError(f"{kernel}: {roles.get(code, 'a role')} waited longer than its budget on {dev}; "
-                              f"the results of that call are invalid")
+        codes = block.tolist()
+        for (kernel, (word, roles)), code in zip(list(words.items()), codes):
+            if code:
+                word.zero_()
+                raise KernelError(f"{kernel}: {roles.get(code, 'a role')} waited longer than its budget on {dev}; "
+                                  f"the results of that call are invalid")
 
 
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
