@@ -1,5 +1,5 @@
 """The host runtime library (``csrc/host/*.cpp``) loaded through ctypes: page pools, the cache
-manager's books and the scheduler's decisions in C++.  Built with the system's C++ compiler at
+manager's books, the scheduler's decisions and the dealing of prompt portions in C++.  Built with the system's C++ compiler at
 first use."""
 from __future__ import annotations
 
@@ -16,6 +16,7 @@ def library() -> ctypes.CDLL:
         dll = ctypes.CDLL(build_host())
         P, I = ctypes.c_void_p, ctypes.c_int
         IP = ctypes.POINTER(ctypes.c_int)
+        D = ctypes.c_double
         L, LP = ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)
         signatures = {
             "mrun_pool_create": (P, [I]), "mrun_pool_destroy": (None, [P]), "mrun_pool_free_count": (I, [P]),
@@ -39,6 +40,7 @@ def library() -> ctypes.CDLL:
             "mrun_sched_end_reason": (I, [I, I, L, L, IP, L]),
             "mrun_sched_preemption_victim": (I, [I, IP, LP]),
             "mrun_sched_next_turn": (I, [I, IP, IP, IP, I, I]),
+            "mrun_prompt_blocks": (I, [I, IP, I, I, I, I, D, D, D, D, P, I]),
             "mrun_sched_stop_match": (I, [IP, I, IP, IP, I]), "mrun_sched_stop_held": (I, [IP, I, IP, IP, I]),
         }
         for name, (restype, argtypes) in signatures.items():

@@ -22,7 +22,6 @@ the fused norm/rotary/cache kernel just before.
 from __future__ import annotations
 
 import ctypes
-import heapq
 import math
 from typing import Optional
 
@@ -31,6 +30,7 @@ import torch
 
 from . import lib as _lib
 from . import ops
+from ..cache import native
 from .ops import _address, _queue
 
 COUNTER_CAPACITY = 1 << 16     # (token, kv head) pairs of one decode launch that may be split
@@ -193,61 +193,25 @@ def prefill_tiles(ctx, tokens_per_tile: int, longer_than: int = 0, up_to: int = 
 TC5_BLOCK, TC5_PAIR_TILE, TC5_SINGLE_TILE = 5.0, 2.25, 1.32
 
 
-def _makespan(costs, machines: int) -> float:
-    """When the last of ``machines`` is done, each taking the next of ``costs`` as it gets free."""
-    if len(costs) <= machines:
-        return max(costs, default=0.0)
-    free = [0.0] * machines
-    for cost in costs:
-        heapq.heapreplace(free, free[0] + cost)
-    return max(free)
-
-
 def tc5_tiles(ctx, tokens: int, longer_than: int, streams: int, window: int, blocks_at_once: float):
     """(first token row, token count) of the blocks of the tcgen05 prompt kernel over the segments with more than
     ``longer_than`` tokens, the longest first, as device int32 arrays; made once per step and choice of sizes.
 
-    A stream of the kernel takes up to ``tokens`` tokens.  A block of two ``streams`` reads keys and values once for both and costs
-    less a row; a block of a single stream is done sooner and leaves fewer multiprocessors idle at the end.  So the longest
-    blocks are pairs and the rest are not; how many are is what ends first by the costs above, of none, all, and as many as
-    fill the device evenly (``blocks_at_once`` a kv head).  A row's result has the same bits in either.
+    A stream of the kernel takes up to ``tokens`` tokens; which blocks are pairs of ``streams`` and which single ones is decided in
+    ``csrc/host/prompt_blocks.cpp`` (``blocks_at_once``: a kv head's).  A row's result has the same bits in either.
     """
     key = ("attention_tc5_tiles", tokens, longer_than, streams, window, blocks_at_once)
     tiles = ctx.shared.get(key)
     if tiles is None:
-        def keys_of(end, count):              # tiles of 128 keys
-            low = end - count                 # the first token's position
-            low = 0 if window == 0 else max(0, low - window + 1) if window > 0 else low // -window * -window
-            return (end - 1) // 128 - low // 128 + 1
-        wide = []
-        for seg in ctx.segments:
-            if seg.q_len > longer_than:
-                for t0 in range(0, seg.q_len, streams * tokens):
-                    count = min(streams * tokens, seg.q_len - t0)
-                    end = seg.pos_start + t0 + count
-                    wide.append((keys_of(end, count), end, seg.q_start + t0, count))
-        wide.sort(key=lambda tile: (-tile[0], -tile[1]))        # a stable sort: the order depends on the segments only
-        found = [(TC5_SINGLE_TILE * keys + TC5_BLOCK, first, count) for keys, _, first, count in wide]
-        if streams == 2 and any(tile[3] > tokens for tile in wide):
-            machines = max(1, int(blocks_at_once))
-            best = None
-            for pairs in sorted({len(wide), int(len(wide) // blocks_at_once * blocks_at_once), 0}, reverse=True):
-                blocks = []
-                for i, (keys, end, first, count) in enumerate(wide):
-                    if count <= tokens:
-                        blocks.append((TC5_SINGLE_TILE * keys + TC5_BLOCK, first, count))
-                    elif i < pairs:
-                        blocks.append((TC5_PAIR_TILE * keys + TC5_BLOCK, first, count))
-                    else:
-                        rest = count - tokens
-                        blocks.append((TC5_SINGLE_TILE * keys_of(end, rest) + TC5_BLOCK, first + tokens, rest))
-                        blocks.append((TC5_SINGLE_TILE * keys_of(end - rest, tokens) + TC5_BLOCK, first, tokens))
-                blocks.sort(key=lambda block: -block[0])
-                ends = _makespan([block[0] for block in blocks], machines)
-                if best is None or ends < best:
-                    best, found = ends, blocks
-        n = len(found)
-        both = ctx.upload(np.asarray([b[1] for b in found] + [b[2] for b in found], dtype=np.int32)) if n else None
+        portions = [v for seg in ctx.segments if seg.q_len > longer_than for v in (seg.q_start, seg.q_len, seg.pos_start)]
+        n = len(portions) // 3
+        room = sum(portions[1::3]) // tokens + n
+        found = np.empty(2 * room, dtype=np.int32)
+        n = native.library().mrun_prompt_blocks(n, native.int_array(portions), tokens, longer_than, streams, window, blocks_at_once,
+                                                TC5_BLOCK, TC5_PAIR_TILE, TC5_SINGLE_TILE, found.ctypes.data, room)
+        if n < 0:
+            raise ops.KernelError(f"the blocks of {len(portions) // 3} prompt portions do not fit {room}")
+        both = ctx.upload(found[:2 * n]) if n else None
         tiles = ctx.shared[key] = (both[:n], both[n:], n) if n else (None, None, 0)
     return tiles
 
