@@ -4,7 +4,7 @@
 // Every output element is the sum over k = 0 .. K-1 in that order, in one chain of fused multiply-adds,
 // whatever M is, wherever the row sits in the batch and whichever of the kernels below runs, so a
 // token's result is bit-identical under every way of cutting the work.
-// Weights of 2,048 k and more that start on 16 bytes go to gemm_f32_tc.cu (kernels/ops.py, f32_tc_ok).
+// Weights of 64 rows and more with a multiple of 4 and at least 2,048 k that start on 16 bytes go to gemm_f32_tc.cu (kernels/ops.py, f32_tc_ok).
 // Reference call site: crates/mrun-engine/src/load.rs:294-306 (`x · Wᵀ`, weights [out, in]).
 //
 //   stream  up to 16 rows whose operands lie on 16-byte boundaries: bound by reading w once, and by the
