@@ -31,9 +31,9 @@
 // run side by side in a pair: a tile of 128 keys for 256 rows of 128 features takes 2.25 us (2,048 cycles of MMAs and as many of the
 // special-function units would be 1.1), for a single stream's 128 rows 1.32.  1,531 tokens behind 9,000, 32 heads over 8, B200:
 // 270 us, 0.91 PFLOP/s; single streams alone 299.
-// What the parts of a pair gave, us a tile: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
-// step); one elected lane, every wait but P's taken before, and both products issued in a row 2.1 -> 1.9; P in halves 2.3 ->
-// 2.25.  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 -> 1.96, a third stage of K or V nothing.
+// What the parts of a pair gave, us a tile, back to back (the figures above are after a pause: 2.05 for 1.9), before the next scores waited
+// for the product that reads P: a warp of products for both streams in place of one each 2.9 -> 2.1 (two fall into
+// step); one elected lane and every wait but P's taken before 2.1 -> 1.9; P in halves 2.3 -> 2.25.  A quarter of the exponentials as polynomials on the multiply-add pipe 1.92 -> 1.96, a third stage of K or V nothing.
 //
 // The roles hand tiles to one another through mbarriers; every wait is bounded by a cycle budget.
 // When a wait runs out the block records a code in the status word, every role stops, the block
