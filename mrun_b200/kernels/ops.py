@@ -710,8 +710,9 @@ F32_TC_MIN_N = 64
 
 def f32_tc_ok(w: torch.Tensor) -> bool:
     """Whether 32-bit products with ``w`` go to the tensor cores.  Decided by w alone, so that a row's bits do not depend on
-    the rows beside it.  From K = 2,048 on they are faster for any number of rows (B200, us, this / the chain of
-    multiply-adds: 1 row of 2,048 x 2,048 10.5 / 10.8, 17 rows 12.7 / 41; 1 row of 128 x 4,096 10.3 / 19; 517 rows of 24,576 x 4,096
+    the rows beside it.  From K = 2,048 on they are faster from a handful of rows on, and for one or two rows from K = 4,096 on (B200, us
+    after a pause, this / the chain of multiply-adds: 17 rows of 2,048 x 2,048 17 / 45, 8 of them 15.4 / 18.4, 1 of them 15.4 / 14.3, 1 row of
+    6,144 x 2,816 23.4 / 21.4, of 6,144 x 4,096 29.5 / 29.6, of 2,048 x 4,096 19 / 25; 517 rows of 24,576 x 4,096
     429 / 2,233) and closer to 64 bits (3.4e-7 / 1.1e-6 at K = 4,096); at K = 1,024 a few rows take longer (8.2 / 6.0), and at
     K = 256 both are equally close (2.9e-7)."""
     n, k = w.shape
